@@ -32,31 +32,20 @@ struct HbArgs {
     MaterialParams mp;
     double *scratch;  // [Ne][6][kScratchStride] block rows (NULL: residual only)
     double *rscr;     // [Ne][6][2K] residual entries (re | im)
+    double *nu_dc;    // [Ne] time-averaged reluctivity (NULL: not wanted; k_hbfem_std only)
 };
 
 // Index of (r, c), r <= c, in the upper triangle of a 6 x 6 block stored row by row.
 __host__ __device__ constexpr int kb_at(int r, int c) { return r * 6 - r * (r - 1) / 2 + (c - r); }
 
-// Resident CTAs per SM the element kernel is compiled for (registers <= 65536 / (128 x this)):
-// with the harmonic count a compile-time constant (MAG_HBFEM_MINB) and at run time
-// (MAG_HBFEM_MINB_RT). Measured at 40^3, K = 3, N = 32: run-time count 3.26 ms (3 CTAs/SM);
-// constant count 2.24 ms (3 CTAs/SM, 168 registers) and 1.66 ms (2 CTAs/SM, 255 registers).
-#ifndef MAG_HBFEM_MINB
-#define MAG_HBFEM_MINB 2
-#endif
-#ifndef MAG_HBFEM_MINB_RT
-#define MAG_HBFEM_MINB_RT 3
-#endif
-
-// KC: the harmonic count as a compile-time constant (0: A.K at run time, arrays sized for
-// kMaxHarm); with a constant count the harmonic loops unroll and the arrays are indexed
-// statically.
-template <bool CALCJ, int KC>
-__global__ void __launch_bounds__(128, KC > 0 ? MAG_HBFEM_MINB : MAG_HBFEM_MINB_RT) k_hbfem_elems(HbArgs A) {
-    constexpr int KA = KC > 0 ? KC : kMaxHarm;
+// General form, one thread per element: any curl table, any weights, any sample count
+// (harmonic arrays sized for kMaxHarm, in local memory).
+template <bool CALCJ>
+__global__ void __launch_bounds__(128, 3) k_hbfem_elems(HbArgs A) {
+    constexpr int KA = kMaxHarm;
     const int64_t e = blockIdx.x * (int64_t)blockDim.x + threadIdx.x;
     if (e >= A.m.ne) return;
-    const int K = KC > 0 ? KC : A.K, N = A.N;
+    const int K = A.K, N = A.N;
     const int4 tt = A.m.tet[e];
     int d[6];
     load_dofs(A.m.dofs, e, d);
@@ -151,6 +140,196 @@ __global__ void __launch_bounds__(128, KC > 0 ? MAG_HBFEM_MINB : MAG_HBFEM_MINB_
     }
 }
 
+// ---- constant curls, equal weights: six threads per element ------------------------
+//
+// With the standard curl table and equal weights every quadrature point repeats the same
+// curls C_i, flux density B(t), nu(t) and weight w, so the time loop runs once per element,
+// not once per point. What cannot be merged is the order of the residual's sum: the
+// reference adds (w C_i . H(t)) P(h,t) over points, then samples, and its rounding needs all
+// nq N additions one after another. The products repeat, though, so each thread forms the N
+// products of one (edge, harmonic, part) once, in registers, and adds them nq times.
+//
+// A CTA of six warps takes kHbElems = 32 elements, lane = element:
+//   1. warp i loads the harmonic values of local edge i; warp 0 the geometry (curls with the
+//      edge signs folded in: negation commutes with rounding);
+//   2. warp i evaluates samples i, i + 6, ...: A(t), B(t), nu(t), H(t) into shared memory
+//      (two samples per load of the harmonic values);
+//   3. warp i sums the 2K residual entries of edge i. NT > 0: N <= NT samples, w C_i . H(t) in
+//      registers (padded with zeros: adding +0 changes no sum, which starts from +0 and so is
+//      never -0). NT = 0: any N, kHbGroup sums at a time, w C_i . H(t) formed in the loop.
+// Bound by the FP64 pipe (no FMA: parity): 2 K N 6 (nq + 1) adds and products for the sums,
+// 24 K + 75 per sample for the fields.
+constexpr int kHbElems = 32;
+constexpr int kHbGroup = 8;
+constexpr size_t kHbMaxSmem = 200 * 1024;
+
+size_t hb_smem_bytes(int K, int N, int NT) {
+    const int np = NT > 0 ? NT : N;
+    return sizeof(double) * ((size_t)kHbElems * (19 + 6 * 2 * K + 4 * np) + (size_t)4 * K * np);
+}
+
+template <int NT>
+__global__ void __launch_bounds__(6 * kHbElems, NT > 0 ? 2 : 1) k_hbfem_std(HbArgs A) {
+    extern __shared__ __align__(16) double hb_smem[];
+    const int K = A.K, N = A.N, NP = NT > 0 ? NT : A.N, W = 2 * K;
+    double *sC = hb_smem;                    // [18][32] signed curls
+    double *sw = sC + 18 * kHbElems;         // [32] weight
+    double *sa = sw + kHbElems;              // [6][2K][32] harmonic values; the results at the end
+    double *sH = sa + 6 * W * kHbElems;      // [NP][3][32]
+    double *snu = sH + 3 * NP * kHbElems;    // [NP][32]
+    double *sd = snu + NP * kHbElems;        // [2K][NP] D re | im
+    double *sp = sd + W * NP;                // [2K][NP] P re | im
+    const int wi = threadIdx.x >> 5, lane = threadIdx.x & 31;
+    const int64_t e0 = (int64_t)blockIdx.x * kHbElems, e = e0 + lane;
+    const bool valid = e < A.m.ne;
+    const bool imag_a = A.si && A.di;
+    for (int i = threadIdx.x; i < W * NP; i += 6 * kHbElems) {
+        const int c = i / NP, t = i - c * NP, h = c < K ? c : c - K;
+        const bool in = t < N;
+        sd[i] = !in ? 0.0 : c < K ? __ldg(A.dr + h * N + t) : imag_a ? __ldg(A.di + h * N + t) : 0.0;
+        sp[i] = !in ? 0.0 : c < K ? __ldg(A.pr + t * K + h) : A.pi ? __ldg(A.pi + t * K + h) : 0.0;
+    }
+    {
+        const int d = valid ? __ldg(A.m.dofs + 6 * e + wi) : -1;
+        for (int h = 0; h < K; h++) {
+            sa[(wi * W + h) * kHbElems + lane] = d >= 0 ? __ldg(A.sr + h * A.ndof + d) : 0.0;
+            if (imag_a) sa[(wi * W + K + h) * kHbElems + lane] = d >= 0 ? __ldg(A.si + h * A.ndof + d) : 0.0;
+        }
+    }
+    const int tag = valid ? A.m.tags[e] : 0;
+    if (wi == 0 && valid) {
+        const int4 tt = A.m.tet[e];
+        const unsigned sb = A.m.signbits ? A.m.signbits[e] : derived_signs(tt);
+        Geo g;
+        geometry(A.m.xyz, tt, g);
+        double C[6][3];
+        curls_standard(g, C);
+#pragma unroll
+        for (int i = 0; i < 6; i++)
+#pragma unroll
+            for (int r = 0; r < 3; r++) sC[(3 * i + r) * kHbElems + lane] = flip(C[i][r], (sb >> i) & 1);
+        sw[lane] = A.qp.qw[0] * g.adet;
+    }
+    __syncthreads();
+    if (valid) {
+        double C[6][3];
+#pragma unroll
+        for (int i = 0; i < 6; i++)
+#pragma unroll
+            for (int r = 0; r < 3; r++) C[i][r] = sC[(3 * i + r) * kHbElems + lane];
+        for (int t = wi; t < N; t += 12) {
+            const int t2 = t + 6;
+            const bool two = t2 < N;
+            const int tb = two ? t2 : t;
+            double B[2][3] = {{0.0, 0.0, 0.0}, {0.0, 0.0, 0.0}};
+#pragma unroll
+            for (int k = 0; k < 6; k++) {
+                double a0 = 0.0, a1 = 0.0;
+                for (int h = 0; h < K; h++) {
+                    const double xr = sa[(k * W + h) * kHbElems + lane];
+                    double m0 = xr * sd[h * NP + t], m1 = xr * sd[h * NP + tb];
+                    if (imag_a) {
+                        const double xi = sa[(k * W + K + h) * kHbElems + lane];
+                        m0 = m0 - xi * sd[(K + h) * NP + t];
+                        m1 = m1 - xi * sd[(K + h) * NP + tb];
+                    }
+                    a0 = a0 + m0;
+                    a1 = a1 + m1;
+                }
+#pragma unroll
+                for (int c = 0; c < 3; c++) {
+                    B[0][c] = B[0][c] + C[k][c] * a0;
+                    B[1][c] = B[1][c] + C[k][c] * a1;
+                }
+            }
+#pragma unroll
+            for (int u = 0; u < 2; u++) {
+                if (u == 1 && !two) break;
+                const int ts = u ? t2 : t;
+                const double bsq = B[u][0] * B[u][0] + B[u][1] * B[u][1] + B[u][2] * B[u][2];
+                double nu, dnu;
+                material_eval(A.mp, tag, bsq, nu, dnu);
+                snu[ts * kHbElems + lane] = nu;
+#pragma unroll
+                for (int c = 0; c < 3; c++) sH[(3 * ts + c) * kHbElems + lane] = nu * B[u][c];
+            }
+        }
+    }
+    __syncthreads();
+    if (valid) {
+        const double c0 = sC[(3 * wi) * kHbElems + lane], c1 = sC[(3 * wi + 1) * kHbElems + lane],
+                     c2 = sC[(3 * wi + 2) * kHbElems + lane], w = sw[lane];
+        double *out = sa + (lane * 6 + wi) * W;  // the harmonic values are used up
+        const int nq = A.qp.nq;
+        if constexpr (NT > 0) {
+            double wd[NT];
+#pragma unroll
+            for (int t = 0; t < NT; t++) {
+                wd[t] = 0.0;
+                if (t < N) {
+                    const double *H = sH + 3 * t * kHbElems + lane;
+                    wd[t] = w * (c0 * H[0] + c1 * H[kHbElems] + c2 * H[2 * kHbElems]);
+                }
+            }
+#pragma unroll 1
+            for (int c = 0; c < W; c++) {
+                double u[NT], acc = 0.0;
+#pragma unroll
+                for (int t = 0; t < NT; t++) {
+                    u[t] = wd[t] * sp[c * NP + t];
+                    acc = acc + u[t];
+                }
+#pragma unroll 1
+                for (int q = 1; q < nq; q++)
+#pragma unroll
+                    for (int t = 0; t < NT; t++) acc = acc + u[t];
+                out[c] = acc;
+            }
+        } else {
+            for (int cb = 0; cb < W; cb += kHbGroup) {
+                double acc[kHbGroup];
+#pragma unroll
+                for (int j = 0; j < kHbGroup; j++) acc[j] = 0.0;
+                for (int q = 0; q < nq; q++)
+                    for (int t = 0; t < N; t++) {
+                        const double *H = sH + 3 * t * kHbElems + lane;
+                        const double v = w * (c0 * H[0] + c1 * H[kHbElems] + c2 * H[2 * kHbElems]);
+#pragma unroll
+                        for (int j = 0; j < kHbGroup; j++)
+                            if (cb + j < W) acc[j] = acc[j] + v * sp[(cb + j) * NP + t];
+                    }
+#pragma unroll
+                for (int j = 0; j < kHbGroup; j++)
+                    if (cb + j < W) out[cb + j] = acc[j];
+            }
+        }
+        if (A.scratch || (A.nu_dc && wi == 5)) {
+            double sum_nu = 0.0;
+            for (int t = 0; t < N; t++) sum_nu = sum_nu + snu[t * kHbElems + lane];
+            const double nu_dc = sum_nu / (double)N;
+            if (A.nu_dc && wi == 5) A.nu_dc[e] = nu_dc;
+            if (A.scratch) {  // row wi of the DC block, w nu_dc (C_r . C_c) summed over the points
+                double row[6];
+#pragma unroll
+                for (int j = 0; j < 6; j++) {
+                    const double dot = c0 * sC[(3 * j) * kHbElems + lane] + c1 * sC[(3 * j + 1) * kHbElems + lane] +
+                                       c2 * sC[(3 * j + 2) * kHbElems + lane];
+                    const double v = w * nu_dc * dot;
+                    double acc = v;
+                    for (int q = 1; q < nq; q++) acc = acc + v;
+                    row[j] = acc;
+                }
+                store_row(A.scratch + e * kScratchPerElem + wi * kScratchStride, row, 0.0);
+            }
+        }
+    }
+    __syncthreads();
+    const int64_t left = A.m.ne - e0;
+    const int count = (int)(left < kHbElems ? left : kHbElems) * 6 * W;
+    double *dst = A.rscr + e0 * 6 * W;
+    for (int i = threadIdx.x; i < count; i += 6 * kHbElems) dst[i] = sa[i];
+}
+
 // out_re[h][row], out_im[h][row]: per CSR row and residual component, the incidences'
 // entries summed from zero in ascending element order.
 __global__ void __launch_bounds__(128) k_rows_reduce_harm(RowPlan rp, const double *__restrict__ rscr, int K,
@@ -171,24 +350,47 @@ __global__ void __launch_bounds__(128) k_rows_reduce_harm(RowPlan rp, const doub
 
 }  // namespace
 
+namespace {
+
+template <int NT>
+int launch_hb_std(const HbArgs &A, size_t smem, cudaStream_t s) {
+    auto kern = k_hbfem_std<NT>;
+    if (cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem) != cudaSuccess)
+        return MAG_E_CUDA;
+    kern<<<(unsigned)((A.m.ne + kHbElems - 1) / kHbElems), 6 * kHbElems, smem, s>>>(A);
+    return cudaPeekAtLastError() == cudaSuccess ? MAG_OK : MAG_E_CUDA;
+}
+
+}  // namespace
+
+bool hbfem_constant_curls(const QuadParams &qp, int K, int N) {
+    const int nt = N <= 16 ? 16 : N <= 24 ? 24 : N <= 32 ? 32 : 0;
+    return qp.standard_curl && qp.uniform_w && hb_smem_bytes(K, N, nt) <= kHbMaxSmem;
+}
+
 int launch_hbfem(const ElemData &m, const RowPlan &rp, int max_row, const double *sr, const double *si, int K,
                  const double *dr, const double *di, const double *pr, const double *pi, int N,
-                 const QuadParams &qp, const MaterialParams &mp, double *scratch, double *rscr, double *vals,
-                 double *out_re, double *out_im, cudaStream_t s) {
-    HbArgs A{m, sr, si, dr, di, pr, pi, K, N, rp.ndof, qp, mp, vals ? scratch : nullptr, rscr};
-    const unsigned g = (unsigned)((m.ne + 127) / 128);
-    switch (K) {
-        case 1: vals ? k_hbfem_elems<true, 1><<<g, 128, 0, s>>>(A) : k_hbfem_elems<false, 1><<<g, 128, 0, s>>>(A); break;
-        case 2: vals ? k_hbfem_elems<true, 2><<<g, 128, 0, s>>>(A) : k_hbfem_elems<false, 2><<<g, 128, 0, s>>>(A); break;
-        case 3: vals ? k_hbfem_elems<true, 3><<<g, 128, 0, s>>>(A) : k_hbfem_elems<false, 3><<<g, 128, 0, s>>>(A); break;
-        case 4: vals ? k_hbfem_elems<true, 4><<<g, 128, 0, s>>>(A) : k_hbfem_elems<false, 4><<<g, 128, 0, s>>>(A); break;
-        default: vals ? k_hbfem_elems<true, 0><<<g, 128, 0, s>>>(A) : k_hbfem_elems<false, 0><<<g, 128, 0, s>>>(A);
+                 const QuadParams &qp, const MaterialParams &mp, double *scratch, double *rscr, double *nu_dc,
+                 double *vals, double *out_re, double *out_im, cudaStream_t s) {
+    const bool rows = vals && !nu_dc;  // DC block rows through the element scratch
+    HbArgs A{m, sr, si, dr, di, pr, pi, K, N, rp.ndof, qp, mp, rows ? scratch : nullptr, rscr, nu_dc};
+    if (hbfem_constant_curls(qp, K, N)) {
+        const int nt = N <= 16 ? 16 : N <= 24 ? 24 : N <= 32 ? 32 : 0;
+        const size_t smem = hb_smem_bytes(K, N, nt);
+        MAG_TRY(nt == 16   ? launch_hb_std<16>(A, smem, s)
+                : nt == 24 ? launch_hb_std<24>(A, smem, s)
+                : nt == 32 ? launch_hb_std<32>(A, smem, s)
+                           : launch_hb_std<0>(A, smem, s));
+    } else {
+        const unsigned g = (unsigned)((m.ne + 127) / 128);
+        if (rows) k_hbfem_elems<true><<<g, 128, 0, s>>>(A);
+        else k_hbfem_elems<false><<<g, 128, 0, s>>>(A);
+        if (cudaPeekAtLastError() != cudaSuccess) return MAG_E_CUDA;
     }
-    if (cudaPeekAtLastError() != cudaSuccess) return MAG_E_CUDA;
     const int64_t nt = rp.ndof * 2 * K;
     k_rows_reduce_harm<<<(unsigned)((nt + 127) / 128), 128, 0, s>>>(rp, rscr, K, out_re, out_im);
     if (cudaPeekAtLastError() != cudaSuccess) return MAG_E_CUDA;
-    if (vals) return launch_rows_reduce(rp, max_row, scratch, vals, nullptr, s);
+    if (rows) return launch_rows_reduce(rp, max_row, scratch, vals, nullptr, s);
     return MAG_OK;
 }
 

@@ -90,13 +90,24 @@ __device__ __forceinline__ double qsum4(double v, const QuadParams &qp, double w
     return acc;
 }
 
+// The sum of nq equal terms u from zero, in order (Q4: nq = 4, as above).
+template <bool Q4>
+__device__ __forceinline__ double qsum_equal(double u, int nq) {
+    if (Q4) return 3.0 * u + u;
+    double acc = u;
+    for (int q = 1; q < nq; q++) acc = acc + u;
+    return acc;
+}
+
 __device__ __forceinline__ void flag(int *err) { atomicOr(err, 1); }
 
-enum TileMode { kJacobian = 0, kStiffness = 1, kSeeded = 2 };
+enum TileMode { kJacobian = 0, kStiffness = 1, kSeeded = 2, kHarmonicDc = 3 };
 
 // One element of the block: record i.
 //   kJacobian: residual and tangent at the element's state (assemble_jacobian_kernel_mex.cpp:92-131);
 //   kStiffness: K(nu) with the element's given nu (assemble_curl_curl_kernel_mex.cpp:94-101), no residual;
+//   kHarmonicDc: the harmonic-balance DC block, K(nu_dc) in that kernel's operation order
+//            (w nu) (Ci.Cj) (assemble_hbfem_kernel_mex.cpp:211-226), no residual;
 //   kSeeded: residual at B, tangent at the seeded state beta B:
 //            nu(|beta B|^2) Ci.Cj + 2 nu'(|beta B|^2) (beta B.Ci)(beta B.Cj), the operation order of
 //            the two-pass seeded kernel.
@@ -130,7 +141,7 @@ __device__ __forceinline__ void tile_element(const TileArgs &A, int64_t i, doubl
             C[j][1] = -C[j][1];
             C[j][2] = -C[j][2];
         }
-    constexpr bool STIFF = MODE == kStiffness;
+    constexpr bool STIFF = MODE == kStiffness || MODE == kHarmonicDc;
     double nu, g2 = 0.0, b[6];
     double nut = 0.0, be = 1.0;  // seeded tangent: nu(|beta B|^2), beta
     if (STIFF) {
@@ -181,7 +192,11 @@ __device__ __forceinline__ void tile_element(const TileArgs &A, int64_t i, doubl
             // independent chains of arithmetic overlap; placing each entry as it is formed
             // measured slower)
             double v[6];
-            if (MODE == kSeeded) {
+            if (MODE == kHarmonicDc) {  // the weight times nu first, then the product with each dot
+                const double wn = w0 * nu;
+#pragma unroll
+                for (int j = 0; j < 6; j++) v[j] = qsum_equal<Q4>(wn * dot3(C[l], C[j]), A.qp.nq);
+            } else if (MODE == kSeeded) {
                 const double gl = g2 * (be * b[l]);
 #pragma unroll
                 for (int j = 0; j < 6; j++)
@@ -245,7 +260,7 @@ __device__ __forceinline__ void cp_async_wait_all() { asm volatile("cp.async.wai
 // elements run, so the row and store phases start without a global round trip.
 template <int BT, int MINB, bool CALCJ, bool Q4, int MODE>
 __global__ void __launch_bounds__(BT, MINB) k_tile(TileArgs A, int nblocks, int ahead) {
-    constexpr bool STIFF = MODE == kStiffness;
+    constexpr bool STIFF = MODE == kStiffness || MODE == kHarmonicDc;
     extern __shared__ __align__(16) double tile_smem[];
     double *slot = tile_smem;
     double2 *incv = reinterpret_cast<double2 *>(tile_smem + A.smem_nnz);
@@ -1113,6 +1128,17 @@ int launch_tile_stiffness(const TilePlan &tp, const ElemData &m, const double *n
     size_t smem = tile_smem_bytes(tp, &a);
     const bool q4 = qp.nq == 4 && qp.uniform_w;
     return q4 ? launch<true, true, kStiffness>(a, tp, smem, s) : launch<true, false, kStiffness>(a, tp, smem, s);
+}
+
+int launch_tile_harmonic_dc(const TilePlan &tp, const ElemData &m, const double *nu_dc, const QuadParams &qp,
+                            double *vals, int *err, cudaStream_t s) {
+    if (!tp.ok || !qp.standard_curl || !qp.uniform_w) return MAG_E_UNSUPPORTED;
+    TileArgs a = make_args(tp, m, qp, err);
+    a.nu_e = nu_dc;
+    a.vals = vals;
+    a.nnz_total = tp.nnz;
+    size_t smem = tile_smem_bytes(tp, &a);
+    return qp.nq == 4 ? launch<true, true, kHarmonicDc>(a, tp, smem, s) : launch<true, false, kHarmonicDc>(a, tp, smem, s);
 }
 
 int launch_tile_seeded(const TilePlan &tp, const ElemData &m, const double *sol, const double *bscale,

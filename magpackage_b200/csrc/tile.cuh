@@ -150,5 +150,9 @@ void free_tile_complex(TileComplexBatch *b);
 // K(nu) with per-element reluctivity nu [Ne].
 int launch_tile_stiffness(const TilePlan &tp, const ElemData &m, const double *nu, const QuadParams &qp,
                           double *vals, int *err, cudaStream_t s);
+// The DC block of a harmonic-balance assembly from the time-averaged reluctivity nu_dc [Ne]
+// (equal quadrature weights).
+int launch_tile_harmonic_dc(const TilePlan &tp, const ElemData &m, const double *nu_dc, const QuadParams &qp,
+                            double *vals, int *err, cudaStream_t s);
 
 }  // namespace mag

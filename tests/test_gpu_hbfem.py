@@ -80,3 +80,39 @@ def test_hbfem_device_resident_field_gives_the_same_bits(oracle_port):
         assert torch.equal(R, R0) and torch.equal(v, v0)
     with pytest.raises(ValueError):
         assemble_hbfem(plan, pair[0][:2], aft, False)
+
+
+@pytest.mark.parametrize("harmonics,samples,weights,schedule", [
+    ((0, 1), 5, "equal", None),            # fewer samples than warps
+    ((1, 3), 16, "equal", None),           # the 16-sample form filled
+    ((1, 3), 17, "equal", "two_pass"),     # 24-sample form, padded; DC block through the row reduction
+    ((0, 1, 2, 5), 24, "equal", None),
+    ((1, 15), 31, "equal", None),
+    ((1, 3, 5), 33, "equal", None),        # more samples than the register forms hold
+    (tuple(range(16)), 64, "equal", None),  # most harmonics
+    (tuple(range(16)), 128, "equal", "two_pass"),
+    ((1, 3), 32, "uneven", None),          # general kernel
+])
+def test_hbfem_sample_counts_and_weights(oracle_port, harmonics, samples, weights, schedule):
+    """Every form of the element kernel against the oracle, 354 elements (a ragged last CTA)."""
+    from magpackage_b200 import _lib
+
+    plan, m, pk, sol, E = _case(oracle_port, harmonics, n=(1, 1, 59), seed=3)
+    aft = AFT(harmonics, n_time_steps=samples)
+    assert aft.num_time_steps == samples
+    qw, val, curl = quadrature.reference_data(2)
+    if weights == "uneven":
+        qw = qw * np.array([1.0, 0.5, 1.25, 1.25])
+        plan.set_quadrature(qw, curl, val)
+    if schedule == "two_pass":
+        plan.set_schedule(_lib.SCHEDULE_TWO_PASS)
+    K = len(harmonics)
+    I, J, V, Rr, Rc, Rre, Rim = oracle_port.hbfem(m, sol, aft.D, aft.P, qw, curl, pk, True)
+    R, vals = assemble_hbfem(plan, sol, aft, True)
+    R = R.cpu().numpy()
+    lin = Rr + (Rc - 1) * E
+    assert bits_equal(np.real(R), oracle_port.sparse_vec(lin, Rre, E * K).reshape(K, E))
+    assert bits_equal(np.imag(R), oracle_port.sparse_vec(lin, Rim, E * K).reshape(K, E))
+    first = I <= E
+    _, _, rv = oracle_port.sparse_csr(I[first], J[first], V[first], E, drop_zeros=False)
+    assert bits_equal(vals.cpu().numpy(), rv)
