@@ -152,38 +152,120 @@ __global__ void __launch_bounds__(128, 3) k_hbfem_elems(HbArgs A) {
 // A CTA of six warps takes kHbElems = 32 elements, lane = element:
 //   1. warp i loads the harmonic values of local edge i; warp 0 the geometry (curls with the
 //      edge signs folded in: negation commutes with rounding);
-//   2. warp i evaluates samples i, i + 6, ...: A(t), B(t), nu(t), H(t) into shared memory
-//      (two samples per load of the harmonic values);
-//   3. warp i sums the 2K residual entries of edge i. NT > 0: N <= NT samples, w C_i . H(t) in
-//      registers (padded with zeros: adding +0 changes no sum, which starts from +0 and so is
-//      never -0). NT = 0: any N, kHbGroup sums at a time, w C_i . H(t) formed in the loop.
-// Bound by the FP64 pipe (no FMA: parity): 2 K N 6 (nq + 1) adds and products for the sums,
-// 24 K + 75 per sample for the fields.
+//   2. warp i evaluates samples i, i + 6, ...: A(t), B(t), nu(t), H(t) into shared memory,
+//      kHbSamples at a time (one load of a harmonic value serves them all, and their spline
+//      searches run side by side: the lookup is a chain of dependent loads);
+//   3. warp i sums the 2K residual entries of edge i. NT > 0: N <= NT samples, padded with
+//      zeros (adding +0 changes no sum, which starts from +0 and so is never -0); v(t) =
+//      w C_i . H(t) goes to the thread's own column of shared memory, over H and nu, so that
+//      only the products are held in registers and three CTAs fit an SM. NT = 0: any N,
+//      kHbGroup sums at a time, v(t) formed in the loop.
+// Work per element, without FMA (parity): 2 K 6 N (nq + 1) operations for the sums, N (24 K +
+// 75) for the fields; at 40^3 (384,000 elements), K = 3, N = 32 that is 0.24 ms of the FP64
+// pipe. Measured there, whole call: one thread per element with the time loop inside the point
+// loop 1687 us; this split with v in registers (160 of them, two CTAs per SM, one sample at a
+// time) 736 us; with v in shared memory and three CTAs 624 us (two CTAs: 721 us). Latency of
+// the sums' dependent additions and of the spline lookups bounds it now.
 constexpr int kHbElems = 32;
+constexpr int kHbThreads = 6 * kHbElems;
+constexpr int kHbSamples = 3;
 constexpr int kHbGroup = 8;
 constexpr size_t kHbMaxSmem = 200 * 1024;
 
+// Shared memory: curls and weight [19][32]; harmonic values [6][2K][32], reused for the
+// results; D and P [4K][np]; then H [np][3][32] and nu [np][32], which v [np][6][32] overlays
+// when NT > 0.
 size_t hb_smem_bytes(int K, int N, int NT) {
     const int np = NT > 0 ? NT : N;
-    return sizeof(double) * ((size_t)kHbElems * (19 + 6 * 2 * K + 4 * np) + (size_t)4 * K * np);
+    return sizeof(double) * ((size_t)kHbElems * (19 + 6 * 2 * K) + (size_t)4 * K * np +
+                             (size_t)kHbElems * np * (NT > 0 ? 6 : 4));
+}
+
+// nu of one material at M values of s = |B|^2: material_eval's arithmetic, the M searches in
+// step.
+template <int M>
+__device__ __forceinline__ void material_nu(const MaterialParams &mp, int tag, const double s[M], double nu[M]) {
+    const int m = tag - 1;
+    const double nu0 = __ldg(mp.lin + m);
+    if (__ldg(mp.is_non + m) == 0.0) {
+#pragma unroll
+        for (int j = 0; j < M; j++) nu[j] = nu0;
+        return;
+    }
+    const double smax = __ldg(mp.max_bsq + m);
+    const double *b = mp.breaks + __ldg(mp.start + m);
+    const double *coefs = mp.coefs + __ldg(mp.coef_start + m);
+    const int pieces = __ldg(mp.count + m);
+    const double scale = mp.bucket ? __ldg(mp.bucket_geom + 2 * m + 1) : 0.0;
+    double x[M];
+    int k[M], lo[M], hi[M];
+#pragma unroll
+    for (int j = 0; j < M; j++) {
+        x[j] = s[j] > smax ? smax : s[j];
+        k[j] = 0;
+        lo[j] = 0;
+        hi[j] = pieces - 1;
+    }
+    if (scale > 0.0) {
+        const double origin = __ldg(mp.bucket_geom + 2 * m);
+#pragma unroll
+        for (int j = 0; j < M; j++) {
+            const double f = (x[j] - origin) * scale;
+            const int i = !(f >= 0.0) ? 0 : (f >= (double)(kMatBuckets - 1) ? kMatBuckets - 1 : (int)f);
+            const int *w = mp.bucket + 2 * kMatBuckets * m + i;
+            lo[j] = __ldg(w);
+            hi[j] = __ldg(w + kMatBuckets);
+            k[j] = lo[j];
+        }
+    }
+    for (;;) {
+        bool more = false;
+#pragma unroll
+        for (int j = 0; j < M; j++)
+            if (lo[j] <= hi[j]) {
+                const int mid = lo[j] + (hi[j] - lo[j]) / 2;
+                if (x[j] >= __ldg(b + mid)) {
+                    k[j] = mid;
+                    lo[j] = mid + 1;
+                } else {
+                    hi[j] = mid - 1;
+                }
+                more = true;
+            }
+        if (!more) break;
+    }
+#pragma unroll
+    for (int j = 0; j < M; j++) {
+        int kk = k[j];
+        if (kk >= pieces) kk = pieces - 1;
+        if (kk < 0) kk = 0;
+        const double *c = coefs + 4 * kk;
+        const double q0 = __ldg(c), q1 = __ldg(c + 1), q2 = __ldg(c + 2), q3 = __ldg(c + 3);
+        const double t = x[j] - __ldg(b + kk);
+        double v = ((q0 * t + q1) * t + q2) * t + q3;
+        const double dv = (3.0 * q0 * t + 2.0 * q1) * t + q2;
+        if (s[j] > smax) v = v + dv * (s[j] - smax);
+        if (v > nu0 || v < 1e-7) v = nu0;
+        nu[j] = v;
+    }
 }
 
 template <int NT>
-__global__ void __launch_bounds__(6 * kHbElems, NT > 0 ? 2 : 1) k_hbfem_std(HbArgs A) {
+__global__ void __launch_bounds__(kHbThreads, NT > 0 ? 3 : 1) k_hbfem_std(HbArgs A) {
     extern __shared__ __align__(16) double hb_smem[];
     const int K = A.K, N = A.N, NP = NT > 0 ? NT : A.N, W = 2 * K;
     double *sC = hb_smem;                    // [18][32] signed curls
     double *sw = sC + 18 * kHbElems;         // [32] weight
     double *sa = sw + kHbElems;              // [6][2K][32] harmonic values; the results at the end
-    double *sH = sa + 6 * W * kHbElems;      // [NP][3][32]
-    double *snu = sH + 3 * NP * kHbElems;    // [NP][32]
-    double *sd = snu + NP * kHbElems;        // [2K][NP] D re | im
+    double *sd = sa + 6 * W * kHbElems;      // [2K][NP] D re | im
     double *sp = sd + W * NP;                // [2K][NP] P re | im
+    double *sH = sp + W * NP;                // [NP][3][32]
+    double *snu = sH + 3 * NP * kHbElems;    // [NP][32]
     const int wi = threadIdx.x >> 5, lane = threadIdx.x & 31;
     const int64_t e0 = (int64_t)blockIdx.x * kHbElems, e = e0 + lane;
     const bool valid = e < A.m.ne;
     const bool imag_a = A.si && A.di;
-    for (int i = threadIdx.x; i < W * NP; i += 6 * kHbElems) {
+    for (int i = threadIdx.x; i < W * NP; i += kHbThreads) {
         const int c = i / NP, t = i - c * NP, h = c < K ? c : c - K;
         const bool in = t < N;
         sd[i] = !in ? 0.0 : c < K ? __ldg(A.dr + h * N + t) : imag_a ? __ldg(A.di + h * N + t) : 0.0;
@@ -217,66 +299,100 @@ __global__ void __launch_bounds__(6 * kHbElems, NT > 0 ? 2 : 1) k_hbfem_std(HbAr
         for (int i = 0; i < 6; i++)
 #pragma unroll
             for (int r = 0; r < 3; r++) C[i][r] = sC[(3 * i + r) * kHbElems + lane];
-        for (int t = wi; t < N; t += 12) {
-            const int t2 = t + 6;
-            const bool two = t2 < N;
-            const int tb = two ? t2 : t;
-            double B[2][3] = {{0.0, 0.0, 0.0}, {0.0, 0.0, 0.0}};
+        for (int t = wi; t < N; t += 6 * kHbSamples) {
+            int ts[kHbSamples];
+            double at[kHbSamples][6], B[kHbSamples][3], s[kHbSamples], nu[kHbSamples];
 #pragma unroll
-            for (int k = 0; k < 6; k++) {
-                double a0 = 0.0, a1 = 0.0;
-                for (int h = 0; h < K; h++) {
-                    const double xr = sa[(k * W + h) * kHbElems + lane];
-                    double m0 = xr * sd[h * NP + t], m1 = xr * sd[h * NP + tb];
-                    if (imag_a) {
-                        const double xi = sa[(k * W + K + h) * kHbElems + lane];
-                        m0 = m0 - xi * sd[(K + h) * NP + t];
-                        m1 = m1 - xi * sd[(K + h) * NP + tb];
-                    }
-                    a0 = a0 + m0;
-                    a1 = a1 + m1;
+            for (int u = 0; u < kHbSamples; u++) {  // past the end: the first sample again
+                ts[u] = t + 6 * u < N ? t + 6 * u : t;
+#pragma unroll
+                for (int k = 0; k < 6; k++) at[u][k] = 0.0;
+            }
+            for (int h = 0; h < K; h++) {
+                double dr[kHbSamples], di[kHbSamples];
+#pragma unroll
+                for (int u = 0; u < kHbSamples; u++) {
+                    dr[u] = sd[h * NP + ts[u]];
+                    if (imag_a) di[u] = sd[(K + h) * NP + ts[u]];
                 }
 #pragma unroll
-                for (int c = 0; c < 3; c++) {
-                    B[0][c] = B[0][c] + C[k][c] * a0;
-                    B[1][c] = B[1][c] + C[k][c] * a1;
+                for (int k = 0; k < 6; k++) {
+                    const double xr = sa[(k * W + h) * kHbElems + lane];
+                    const double xi = imag_a ? sa[(k * W + K + h) * kHbElems + lane] : 0.0;
+#pragma unroll
+                    for (int u = 0; u < kHbSamples; u++) {
+                        double term = xr * dr[u];
+                        if (imag_a) term = term - xi * di[u];
+                        at[u][k] = at[u][k] + term;
+                    }
                 }
             }
 #pragma unroll
-            for (int u = 0; u < 2; u++) {
-                if (u == 1 && !two) break;
-                const int ts = u ? t2 : t;
-                const double bsq = B[u][0] * B[u][0] + B[u][1] * B[u][1] + B[u][2] * B[u][2];
-                double nu, dnu;
-                material_eval(A.mp, tag, bsq, nu, dnu);
-                snu[ts * kHbElems + lane] = nu;
+            for (int u = 0; u < kHbSamples; u++) {
 #pragma unroll
-                for (int c = 0; c < 3; c++) sH[(3 * ts + c) * kHbElems + lane] = nu * B[u][c];
+                for (int c = 0; c < 3; c++) {
+                    B[u][c] = 0.0;
+#pragma unroll
+                    for (int k = 0; k < 6; k++) B[u][c] = B[u][c] + C[k][c] * at[u][k];
+                }
+                s[u] = B[u][0] * B[u][0] + B[u][1] * B[u][1] + B[u][2] * B[u][2];
+            }
+            material_nu<kHbSamples>(A.mp, tag, s, nu);
+#pragma unroll
+            for (int u = 0; u < kHbSamples; u++) {
+                snu[ts[u] * kHbElems + lane] = nu[u];
+#pragma unroll
+                for (int c = 0; c < 3; c++) sH[(3 * ts[u] + c) * kHbElems + lane] = nu[u] * B[u][c];
             }
         }
     }
     __syncthreads();
-    if (valid) {
-        const double c0 = sC[(3 * wi) * kHbElems + lane], c1 = sC[(3 * wi + 1) * kHbElems + lane],
-                     c2 = sC[(3 * wi + 2) * kHbElems + lane], w = sw[lane];
-        double *out = sa + (lane * 6 + wi) * W;  // the harmonic values are used up
-        const int nq = A.qp.nq;
-        if constexpr (NT > 0) {
-            double wd[NT];
+    const double c0 = sC[(3 * wi) * kHbElems + lane], c1 = sC[(3 * wi + 1) * kHbElems + lane],
+                 c2 = sC[(3 * wi + 2) * kHbElems + lane], w = sw[lane];  // (not read for an invalid lane)
+    const int nq = A.qp.nq;
+    if (valid && (A.scratch || (A.nu_dc && wi == 5))) {
+        double sum_nu = 0.0;
+        for (int t = 0; t < N; t++) sum_nu = sum_nu + snu[t * kHbElems + lane];
+        const double nu_dc = sum_nu / (double)N;
+        if (A.nu_dc && wi == 5) A.nu_dc[e] = nu_dc;
+        if (A.scratch) {  // row wi of the DC block, w nu_dc (C_r . C_c) summed over the points
+            double row[6];
+#pragma unroll
+            for (int j = 0; j < 6; j++) {
+                const double dot = c0 * sC[(3 * j) * kHbElems + lane] + c1 * sC[(3 * j + 1) * kHbElems + lane] +
+                                   c2 * sC[(3 * j + 2) * kHbElems + lane];
+                const double v = w * nu_dc * dot;
+                double acc = v;
+                for (int q = 1; q < nq; q++) acc = acc + v;
+                row[j] = acc;
+            }
+            store_row(A.scratch + e * kScratchPerElem + wi * kScratchStride, row, 0.0);
+        }
+    }
+    double *out = sa + (lane * 6 + wi) * W;  // the harmonic values are used up
+    if constexpr (NT > 0) {
+        double *sv = sH + threadIdx.x;  // [NT][6][32], this thread's column
+        {
+            double v[NT];
 #pragma unroll
             for (int t = 0; t < NT; t++) {
-                wd[t] = 0.0;
-                if (t < N) {
+                v[t] = 0.0;
+                if (valid && t < N) {
                     const double *H = sH + 3 * t * kHbElems + lane;
-                    wd[t] = w * (c0 * H[0] + c1 * H[kHbElems] + c2 * H[2 * kHbElems]);
+                    v[t] = w * (c0 * H[0] + c1 * H[kHbElems] + c2 * H[2 * kHbElems]);
                 }
             }
+            __syncthreads();  // H and nu are used up
+#pragma unroll
+            for (int t = 0; t < NT; t++) sv[t * kHbThreads] = v[t];
+        }
+        if (valid)
 #pragma unroll 1
             for (int c = 0; c < W; c++) {
                 double u[NT], acc = 0.0;
 #pragma unroll
                 for (int t = 0; t < NT; t++) {
-                    u[t] = wd[t] * sp[c * NP + t];
+                    u[t] = sv[t * kHbThreads] * sp[c * NP + t];
                     acc = acc + u[t];
                 }
 #pragma unroll 1
@@ -285,49 +401,29 @@ __global__ void __launch_bounds__(6 * kHbElems, NT > 0 ? 2 : 1) k_hbfem_std(HbAr
                     for (int t = 0; t < NT; t++) acc = acc + u[t];
                 out[c] = acc;
             }
-        } else {
-            for (int cb = 0; cb < W; cb += kHbGroup) {
-                double acc[kHbGroup];
+    } else if (valid) {
+        for (int cb = 0; cb < W; cb += kHbGroup) {
+            double acc[kHbGroup];
 #pragma unroll
-                for (int j = 0; j < kHbGroup; j++) acc[j] = 0.0;
-                for (int q = 0; q < nq; q++)
-                    for (int t = 0; t < N; t++) {
-                        const double *H = sH + 3 * t * kHbElems + lane;
-                        const double v = w * (c0 * H[0] + c1 * H[kHbElems] + c2 * H[2 * kHbElems]);
+            for (int j = 0; j < kHbGroup; j++) acc[j] = 0.0;
+            for (int q = 0; q < nq; q++)
+                for (int t = 0; t < N; t++) {
+                    const double *H = sH + 3 * t * kHbElems + lane;
+                    const double v = w * (c0 * H[0] + c1 * H[kHbElems] + c2 * H[2 * kHbElems]);
 #pragma unroll
-                        for (int j = 0; j < kHbGroup; j++)
-                            if (cb + j < W) acc[j] = acc[j] + v * sp[(cb + j) * NP + t];
-                    }
-#pragma unroll
-                for (int j = 0; j < kHbGroup; j++)
-                    if (cb + j < W) out[cb + j] = acc[j];
-            }
-        }
-        if (A.scratch || (A.nu_dc && wi == 5)) {
-            double sum_nu = 0.0;
-            for (int t = 0; t < N; t++) sum_nu = sum_nu + snu[t * kHbElems + lane];
-            const double nu_dc = sum_nu / (double)N;
-            if (A.nu_dc && wi == 5) A.nu_dc[e] = nu_dc;
-            if (A.scratch) {  // row wi of the DC block, w nu_dc (C_r . C_c) summed over the points
-                double row[6];
-#pragma unroll
-                for (int j = 0; j < 6; j++) {
-                    const double dot = c0 * sC[(3 * j) * kHbElems + lane] + c1 * sC[(3 * j + 1) * kHbElems + lane] +
-                                       c2 * sC[(3 * j + 2) * kHbElems + lane];
-                    const double v = w * nu_dc * dot;
-                    double acc = v;
-                    for (int q = 1; q < nq; q++) acc = acc + v;
-                    row[j] = acc;
+                    for (int j = 0; j < kHbGroup; j++)
+                        if (cb + j < W) acc[j] = acc[j] + v * sp[(cb + j) * NP + t];
                 }
-                store_row(A.scratch + e * kScratchPerElem + wi * kScratchStride, row, 0.0);
-            }
+#pragma unroll
+            for (int j = 0; j < kHbGroup; j++)
+                if (cb + j < W) out[cb + j] = acc[j];
         }
     }
     __syncthreads();
     const int64_t left = A.m.ne - e0;
     const int count = (int)(left < kHbElems ? left : kHbElems) * 6 * W;
     double *dst = A.rscr + e0 * 6 * W;
-    for (int i = threadIdx.x; i < count; i += 6 * kHbElems) dst[i] = sa[i];
+    for (int i = threadIdx.x; i < count; i += kHbThreads) dst[i] = sa[i];
 }
 
 // out_re[h][row], out_im[h][row]: per CSR row and residual component, the incidences'
