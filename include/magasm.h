@@ -336,7 +336,7 @@ int mag_csr_apply_dirichlet(int64_t n, const int64_t *d_row_ptr, const int32_t *
  * iterations. Jacobi preconditioner, plus the auxiliary gradient space when set.
  * Deterministic (fixed-order reductions). Outputs: iterations, ||r||/||b||,
  * status 1 converged / 2 iteration limit / 3 breakdown (returns MAG_E_GEOMETRY).
- * Synchronises the host once per 32 iterations. */
+ * Synchronises the host once per 256 iterations. */
 typedef struct mag_pcg mag_pcg;
 int mag_pcg_create(int64_t n, mag_pcg **out);
 int mag_pcg_destroy(mag_pcg *pcg);
