@@ -19,8 +19,8 @@
 //              K + 1j*omega*M from the two assembled matrices
 //              (FrequencySolver.m:131), where 0*M adds nothing to the real part.
 // Variants 4 and 5 run the same assembly on the meshes' tile blocks instead
-// (k_tile_complex in tile.cu: one evaluation of each element per block it touches, K
-// pass then M pass). The launch is captured once in a CUDA graph and replayed. The
+// (k_tile_complex in tile.cu: one evaluation of each element per block it touches, a K
+// kernel, then an M kernel over the blocks that conduct). The launch is captured once in a CUDA graph and replayed. The
 // variant (schedule, block size, CTA residency) is chosen per batch by timing every
 // available one (mag_batch_create).
 #include <algorithm>

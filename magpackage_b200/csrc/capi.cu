@@ -414,9 +414,14 @@ int require_ready(const mag_mesh *m, bool need_mat) {
 // Stream-ordered workspace of one call, from the handle's pool: freed memory stays in the
 // pool for the next call (the default pool would return it at the next synchronisation and
 // map it again: 1.3 ms for 110 MB) and goes back when the handle is destroyed.
-int workspace(const mag_mesh *m, size_t bytes, cudaStream_t s, double **p) {
+// The pool is made by the first call outside a stream capture; a captured call's allocation
+// belongs to its graph.
+int workspace(mag_mesh *m, size_t bytes, cudaStream_t s, double **p) {
     void *v = nullptr;
-    if (m->pool) MAG_CUDA_TRY(cudaMallocFromPoolAsync(&v, bytes, m->pool, s));
+    cudaStreamCaptureStatus cap = cudaStreamCaptureStatusNone;
+    MAG_CUDA_TRY(cudaStreamIsCapturing(s, &cap));
+    if (!m->pool && cap == cudaStreamCaptureStatusNone) m->pool = make_pool();
+    if (m->pool && cap == cudaStreamCaptureStatusNone) MAG_CUDA_TRY(cudaMallocFromPoolAsync(&v, bytes, m->pool, s));
     else MAG_CUDA_TRY(cudaMallocAsync(&v, bytes, s));
     *p = static_cast<double *>(v);
     return MAG_OK;
@@ -551,7 +556,6 @@ int mag_mesh_create(const double *d_P, int64_t Nn, const int32_t *d_T, int64_t N
         cudaGetLastError();
     }
     if (cudaMalloc(&m->status, sizeof(int)) != cudaSuccess) return fail(MAG_E_NOMEM);
-    m->pool = make_pool();
     cudaMemsetAsync(m->status, 0, sizeof(int), s);
     {
         const TilePlanInput ti{m->xyz, m->tet, m->dofs, m->tags, m->signbits, m->pat.row_ptr, m->pat.inc_ptr,
@@ -773,6 +777,10 @@ int mag_assemble_mass(mag_mesh *m, const double *d_sigma, double *d_vals, void *
         return MAG_E_ARG;
     }
     cudaStream_t s = (cudaStream_t)stream;
+    if (m->schedule == MAG_SCHEDULE_TILE_BLOCKS && m->tile.ok) {
+        MAG_TRY(launch_tile_mass(m->tile, m->elems(), d_sigma, m->qp, d_vals, m->status, s));
+        return finish(s);
+    }
     MAG_TRY(launch_mass_elems(m->elems(), d_sigma, m->qp, m->scratch, s));
     MAG_TRY(launch_rows_reduce(m->rows(), m->pat.max_row, m->scratch, d_vals, nullptr, s));
     return finish(s);
@@ -785,8 +793,7 @@ int mag_assemble_source(mag_mesh *m, const double *d_js, double *d_out, void *st
         return MAG_E_ARG;
     }
     cudaStream_t s = (cudaStream_t)stream;
-    MAG_TRY(launch_source_elems(m->elems(), d_js, m->qp, m->scratch, s));
-    MAG_TRY(launch_rows_reduce(m->rows(), m->pat.max_row, m->scratch, nullptr, d_out, s));
+    MAG_TRY(launch_source(m->elems(), m->rows(), d_js, m->qp, m->scratch, d_out, s));
     return finish(s);
 }
 
@@ -799,9 +806,7 @@ int mag_assemble_winding(mag_mesh *m, int coil_id, const double *d_dir_field, co
     }
     cudaStream_t s = (cudaStream_t)stream;
     const double zero[3] = {0.0, 0.0, 0.0};
-    MAG_TRY(launch_winding_elems(m->elems(), coil_id, d_dir_field, dir ? dir : zero, scale, m->qp, m->scratch,
-                                 nullptr, nullptr, s));
-    MAG_TRY(launch_rows_reduce(m->rows(), m->pat.max_row, m->scratch, nullptr, d_out, s));
+    MAG_TRY(launch_winding(m->elems(), m->rows(), coil_id, d_dir_field, dir ? dir : zero, scale, m->qp, d_out, s));
     return finish(s);
 }
 
@@ -1881,7 +1886,7 @@ int mag_mex_winding(const double *P, int64_t Nn, const double *T, int64_t Ne, co
     double *dI = out.as<double>(), *dV = dI + 6 * Ne;
     if (rc == MAG_OK)
         rc = launch_winding_elems(mm.ed, coil, DirField ? field.as<double>() : nullptr, UniDir ? UniDir : zero,
-                                  Scale, qp, nullptr, dI, dV, s);
+                                  Scale, qp, dI, dV, s);
     if (rc == MAG_OK && (cudaMemcpyAsync(I, dI, Ne * 48, cudaMemcpyDeviceToHost, s) != cudaSuccess ||
                          cudaMemcpyAsync(V, dV, Ne * 48, cudaMemcpyDeviceToHost, s) != cudaSuccess ||
                          cudaStreamSynchronize(s) != cudaSuccess))

@@ -359,29 +359,54 @@ struct TileComplexInstance {
 };
 
 // The sigma-mass rows of one element of the block (assemble_mass_kernel_mex.cpp:186-230):
-// per local row l, m_j = sum_q ((N_l . N_j) sigma) w_q with N = J^{-T} N_ref at each point,
-// signed; off-diagonal entries into their nonzeros' slots, the diagonal into the
-// incidence slot's x. Elements with |sigma| <= 1e-12 add nothing (the reference skips
-// them; a skipped contribution and a +0 one give the same sums).
-__device__ __forceinline__ void tile_mass_element(const TileComplexInstance &I, int64_t i, double *__restrict__ slot,
-                                                  double2 *__restrict__ incv, int bnnz, int binc,
-                                                  const double *__restrict__ sval) {
-    const TileArgs &A = I.a;
+// m_lj = sum_q ((N_l . N_j) sigma) w_q with N = J^{-T} N_ref at each point. The element's
+// matrix is symmetric bit for bit (the same products in the same order), so its upper triangle
+// is accumulated once, point by point, and each of the block's rows picks its six entries,
+// signed: off-diagonal ones into their nonzeros' slots, the diagonal into the incidence slot's
+// x. Elements with |sigma| <= 1e-12 add nothing (the reference skips them; a skipped
+// contribution and a +0 one give the same sums).
+// FIRST: the block's first colour class, whose slots are all still +0: stored, not added.
+template <bool FIRST>
+__device__ __forceinline__ void tile_mass_element(const TileArgs &A, const double *__restrict__ sigma_e, int64_t i,
+                                                  double *__restrict__ slot, double2 *__restrict__ incv, int bnnz,
+                                                  int binc, const double *__restrict__ sval) {
     const int64_t n = A.nrec;
     const uint4 p2 = __ldg(A.recs + 2 * n + i);
-    const double sigma = I.sigma ? __ldg(I.sigma + p2.z) : 1.0;
+    const double sigma = sigma_e ? __ldg(sigma_e + p2.z) : 1.0;
     if (!(fabs(sigma) > 1e-12)) return;
-    const uint4 p0 = __ldg(A.recs + i), p3 = __ldg(A.recs + 3 * n + i), p4 = __ldg(A.recs + 4 * n + i),
-                p5 = __ldg(A.recs + 5 * n + i);
+    const uint4 p0 = __ldg(A.recs + i);
     const int4 tt = make_int4((int)p0.x, (int)p0.y, (int)p0.z, (int)p0.w);
     const unsigned sb = (p2.w >> 8) & 0x3Fu;
+    double M[21];  // row by row from the diagonal
+#pragma unroll
+    for (int k = 0; k < 21; k++) M[k] = 0.0;
+    {
+        Geo g;
+        geometry(A.xyz, tt, g);
+        double iv[3][3];
+        inverse3(g, iv);
+        const int nq = A.qp.nq;
+#pragma unroll 1
+        for (int q = 0; q < nq; q++) {
+            const double w = A.qp.qw[q] * g.adet;
+            const double *r = sval + 18 * q;
+            double N[6][3];
+#pragma unroll
+            for (int j = 0; j < 6; j++) {
+                const double r0 = r[j], r1 = r[j + 6], r2 = r[j + 12];
+#pragma unroll
+                for (int c = 0; c < 3; c++) N[j][c] = iv[0][c] * r0 + iv[1][c] * r1 + iv[2][c] * r2;
+            }
+            int k = 0;
+#pragma unroll
+            for (int l = 0; l < 6; l++)
+#pragma unroll
+                for (int j = l; j < 6; j++, k++) M[k] = M[k] + dot3(N[l], N[j]) * sigma * w;
+        }
+    }
+    const uint4 p3 = __ldg(A.recs + 3 * n + i), p4 = __ldg(A.recs + 4 * n + i), p5 = __ldg(A.recs + 5 * n + i);
     const unsigned pos[6] = {p3.x, p3.y, p3.z, p3.w, p4.x, p4.y};
     const unsigned sl[6] = {p4.z, p4.w, p5.x, p5.y, p5.z, p5.w};
-    Geo g;
-    geometry(A.xyz, tt, g);
-    double iv[3][3];
-    inverse3(g, iv);
-    const int nq = A.qp.nq;
 #pragma unroll
     for (int l = 0; l < 6; l++) {
         const unsigned s = sl[l];
@@ -392,29 +417,16 @@ __device__ __forceinline__ void tile_mass_element(const TileComplexInstance &I, 
             continue;
         }
         const unsigned si = (sb >> l) & 1u;
-        double m[6] = {0.0, 0.0, 0.0, 0.0, 0.0, 0.0};
-#pragma unroll 1
-        for (int q = 0; q < nq; q++) {
-            const double w = A.qp.qw[q] * g.adet;
-            const double *r = sval + 18 * q;
-            double Nl[3];
-#pragma unroll
-            for (int c = 0; c < 3; c++) Nl[c] = iv[0][c] * r[l] + iv[1][c] * r[l + 6] + iv[2][c] * r[l + 12];
-#pragma unroll
-            for (int j = 0; j < 6; j++) {
-                double Nj[3];
-#pragma unroll
-                for (int c = 0; c < 3; c++) Nj[c] = iv[0][c] * r[j] + iv[1][c] * r[j + 6] + iv[2][c] * r[j + 12];
-                m[j] = m[j] + dot3(Nl, Nj) * sigma * w;
-            }
-        }
 #pragma unroll
         for (int j = 0; j < 6; j++) {
             if (j == l) continue;
+            const int a = l < j ? l : j, b = l < j ? j : l;
             const int k = nzb + (int)((pos[l] >> (5 * j)) & 31u);  // absent column: the diagonal
-            slot[k] = slot[k] + flip(m[j], si ^ ((sb >> j) & 1u));
+            const double v = flip(M[a * 6 - a * (a - 1) / 2 + (b - a)], si ^ ((sb >> j) & 1u));
+            if (FIRST) slot[k] = v;
+            else slot[k] = slot[k] + v;
         }
-        if (is < binc) incv[is].x = m[l];  // the diagonal: si ^ si = 0, no flip
+        if (is < binc) incv[is].x = M[l * 6 - l * (l - 1) / 2];  // the diagonal: si ^ si = 0, no flip
         else flag(A.err);
     }
 }
@@ -439,21 +451,20 @@ __device__ __forceinline__ void tile_rows_diag(const uint2 *srows, int nrows, co
     }
 }
 
-// One CTA per (mesh, block) item. K pass: the tile kernel's K(nu) elements (incidence
-// slots get (0, K diagonal)), row sums, real parts stored. M pass, only when some element
-// of the block conducts: slots zeroed again, the conducting elements' M rows, row sums,
-// imaginary parts stored as omega * M; otherwise the imaginary parts are omega * 0.
+// One CTA per (mesh, block) item: the tile kernel's K(nu) elements (incidence slots get (0, K
+// diagonal)), row sums, (K, omega * 0) pairs stored in one coalesced pass. A block that holds a
+// conducting element goes onto the list of k_tile_complex_mass, which then stores its imaginary
+// parts. (Both passes in one kernel needed the registers of the M pass everywhere.)
 // Values equal (K_ab, omega * M_ab) of MATLAB's K + 1j*omega*M (FrequencySolver.m:131).
 template <int BT, int MINB, bool Q4>
 __global__ void __launch_bounds__(BT, MINB)
     k_tile_complex(const TileComplexInstance *__restrict__ inst, const int2 *__restrict__ items, int nitems,
-                   int ahead, int smem_nnz, int smem_inc, int smem_rows, int smem_chunks) {
+                   int ahead, int smem_nnz, int smem_inc, int smem_rows, int smem_chunks, int *__restrict__ list) {
     extern __shared__ __align__(16) double tile_smem[];
     double *slot = tile_smem;
     double2 *incv = reinterpret_cast<double2 *>(tile_smem + smem_nnz);
     uint2 *srows = reinterpret_cast<uint2 *>(incv + smem_inc);
     uint2 *schunks = srows + smem_rows;
-    double *sval = reinterpret_cast<double *>(schunks + smem_chunks);
     const int tid = threadIdx.x;
     const int it = blockIdx.x;
     if (tid == 0 && it + ahead < nitems) {
@@ -467,21 +478,17 @@ __global__ void __launch_bounds__(BT, MINB)
     const int nrows = Bp->nrows, row0 = Bp->row0, rec0 = Bp->rec0;
     const int nnz = Bp->nnz, ninc = Bp->ninc, ncolors = Bp->ncolors;
     const int chunk0 = Bp->chunk0, nchunks = Bp->nchunks;
-    const int nq = A.qp.nq;
-    if (nrows > smem_rows || nchunks > smem_chunks || nnz > smem_nnz - kTileSlotPad || ninc > smem_inc ||
-        nq > kMaxQuad) {
+    if (nrows > smem_rows || nchunks > smem_chunks || nnz > smem_nnz - kTileSlotPad || ninc > smem_inc) {
         if (tid == 0) flag(A.err);  // the whole CTA leaves before its first barrier
         return;
     }
     for (int i = tid; i < nrows; i += BT) cp_async8(srows + i, A.rows + row0 + i);
     for (int i = tid; i < nchunks; i += BT) cp_async8(schunks + i, A.chunks + chunk0 + i);
     cp_async_commit();
-    for (int i = tid; i < 18 * nq; i += BT) sval[i] = __ldg(I.val_ref + i);
     for (int i = tid; i < (nnz + 1) / 2; i += BT)  // 16-byte stores; an odd tail's pair ends in the pad
         reinterpret_cast<double2 *>(slot)[i] = make_double2(0.0, 0.0);
     __syncthreads();
-    // K pass; the barrier after its last colour also tells every thread whether any element
-    // of the block conducts
+    // the barrier after the last colour also tells whether any element of the block conducts
     int conducting = 0;
     int c0 = 0;
     bool any_m = false;
@@ -508,11 +515,12 @@ __global__ void __launch_bounds__(BT, MINB)
         cp_async_wait_all();
         __syncthreads();
     }
+    if (tid == 0 && any_m) list[1 + atomicAdd(list, 1)] = it;
     tile_rows_diag<BT, true>(srows, nrows, incv, ninc, slot, nnz, A.err);
     __syncthreads();
-    // real parts; a block without a conductor stores (K, omega * 0) pairs in this one pass
     const int warp = tid >> 5, lane = tid & 31;
     double2 *cv2 = reinterpret_cast<double2 *>(I.cvals);
+    const double im = I.omega * 0.0;
     for (int c = warp; c < nchunks; c += BT / 32) {
         const uint2 ch = schunks[c];
         const int sb0 = (int)(ch.x & 0xFFFFu), len = (int)(ch.x >> 16);
@@ -521,32 +529,120 @@ __global__ void __launch_bounds__(BT, MINB)
             if (lane == 0) flag(A.err);
             continue;
         }
-        if (any_m)  // (+ 0.0: -0 -> +0, the first colour stores its entries)
-            for (int i = lane; i < len; i += 32) I.cvals[2 * (g + i)] = slot[sb0 + i] + 0.0;
-        else
-            for (int i = lane; i < len; i += 32) cv2[g + i] = make_double2(slot[sb0 + i] + 0.0, I.omega * 0.0);
+        // (+ 0.0: -0 -> +0, the first colour stores its entries)
+        for (int i = lane; i < len; i += 32) cv2[g + i] = make_double2(slot[sb0 + i] + 0.0, im);
     }
-    if (!any_m) return;
-    // M pass over the same slots
-    __syncthreads();  // the real parts are read out of the slots
+}
+
+// The sigma-mass values of one block: slots and incidence slots zeroed, the conducting elements'
+// rows colour by colour, diagonals in element order, then each stored value through `store(nonzero,
+// value)`. Uniform over the CTA; ends without a barrier.
+struct TileSmem {
+    double *slot;
+    double2 *incv;
+    uint2 *rows, *chunks;
+    double *val;  // [18 nq] reference basis values
+    int nnz, inc, nrows, nchunks;
+};
+
+__device__ __forceinline__ TileSmem tile_smem_layout(double *base, int nnz, int inc, int rows, int chunks) {
+    TileSmem S;
+    S.slot = base;
+    S.incv = reinterpret_cast<double2 *>(base + nnz);
+    S.rows = reinterpret_cast<uint2 *>(S.incv + inc);
+    S.chunks = S.rows + rows;
+    S.val = reinterpret_cast<double *>(S.chunks + chunks);
+    S.nnz = nnz;
+    S.inc = inc;
+    S.nrows = rows;
+    S.nchunks = chunks;
+    return S;
+}
+
+template <int BT, typename Store>
+__device__ __forceinline__ void tile_mass_block(const TileArgs &A, const TileSmem &S, const TileBlock *Bp,
+                                                const double *__restrict__ sigma, const double *__restrict__ val_ref,
+                                                Store store) {
+    const int tid = threadIdx.x;
+    const int nrows = Bp->nrows, row0 = Bp->row0, rec0 = Bp->rec0;
+    const int nnz = Bp->nnz, ninc = Bp->ninc, ncolors = Bp->ncolors;
+    const int chunk0 = Bp->chunk0, nchunks = Bp->nchunks;
+    const int nq = A.qp.nq;
+    if (nrows > S.nrows || nchunks > S.nchunks || nnz > S.nnz - kTileSlotPad || ninc > S.inc || nq > kMaxQuad) {
+        if (tid == 0) flag(A.err);  // the whole CTA skips the block
+        return;
+    }
+    for (int i = tid; i < nrows; i += BT) cp_async8(S.rows + i, A.rows + row0 + i);
+    for (int i = tid; i < nchunks; i += BT) cp_async8(S.chunks + i, A.chunks + chunk0 + i);
+    cp_async_commit();
+    for (int i = tid; i < 18 * nq; i += BT) S.val[i] = __ldg(val_ref + i);
     for (int i = tid; i < (nnz + 1) / 2; i += BT)  // 16-byte stores; an odd tail's pair ends in the pad
-        reinterpret_cast<double2 *>(slot)[i] = make_double2(0.0, 0.0);
+        reinterpret_cast<double2 *>(S.slot)[i] = make_double2(0.0, 0.0);
+    for (int i = tid; i < ninc; i += BT) S.incv[i] = make_double2(0.0, 0.0);  // no sigma: nothing written
     __syncthreads();
-    c0 = 0;
+    int c0 = 0;
     for (int c = 0; c < ncolors; c++) {
         const int c1 = Bp->col_end[c];
-        for (int i = c0 + tid; i < c1; i += BT) tile_mass_element(I, (int64_t)rec0 + i, slot, incv, nnz, ninc, sval);
+        if (c == 0)
+            for (int i = c0 + tid; i < c1; i += BT)
+                tile_mass_element<true>(A, sigma, (int64_t)rec0 + i, S.slot, S.incv, nnz, ninc, S.val);
+        else
+            for (int i = c0 + tid; i < c1; i += BT)
+                tile_mass_element<false>(A, sigma, (int64_t)rec0 + i, S.slot, S.incv, nnz, ninc, S.val);
         c0 = c1;
+        if (c + 1 == ncolors) cp_async_wait_all();
         __syncthreads();
     }
-    tile_rows_diag<BT, false>(srows, nrows, incv, ninc, slot, nnz, A.err);
+    if (ncolors == 0) {
+        cp_async_wait_all();
+        __syncthreads();
+    }
+    tile_rows_diag<BT, false>(S.rows, nrows, S.incv, ninc, S.slot, nnz, A.err);
     __syncthreads();
+    const int warp = tid >> 5, lane = tid & 31;
     for (int c = warp; c < nchunks; c += BT / 32) {
-        const uint2 ch = schunks[c];
+        const uint2 ch = S.chunks[c];
         const int sb0 = (int)(ch.x & 0xFFFFu), len = (int)(ch.x >> 16);
         const int64_t g = (int64_t)ch.y;
-        if (sb0 + len > nnz || g + len > A.nnz_total) continue;  // flagged in the K pass
-        for (int i = lane; i < len; i += 32) I.cvals[2 * (g + i) + 1] = I.omega * slot[sb0 + i];
+        if (sb0 + len > nnz || g + len > A.nnz_total) {
+            if (lane == 0) flag(A.err);
+            continue;
+        }
+        for (int i = lane; i < len; i += 32) store(g + i, S.slot[sb0 + i] + 0.0);  // -0 -> +0
+    }
+}
+
+// 256 threads x 2 CTAs per SM: 128 registers hold the element's upper triangle and six basis
+// vectors (at 320 x 2, 96 registers, they spill).
+constexpr int kMassBT = 256;
+
+// M(sigma) of one mesh, one CTA per block. 613,000 elements, a tenth of them conducting: 295 us
+// with element blocks through HBM scratch and row sums, 60 us here.
+__global__ void __launch_bounds__(kMassBT, 2)
+    k_tile_mass(TileArgs A, const double *__restrict__ sigma, const double *__restrict__ val_ref, int nblocks, int ahead) {
+    extern __shared__ __align__(16) double tile_smem[];
+    const TileSmem S = tile_smem_layout(tile_smem, A.smem_nnz, A.smem_inc, A.smem_rows, A.smem_chunks);
+    const int blk = blockIdx.x;
+    if (threadIdx.x == 0 && blk + ahead < nblocks) prefetch_block(A, blk + ahead);
+    double *vals = A.vals;
+    tile_mass_block<kMassBT>(A, S, A.blocks + blk, sigma, val_ref, [&](int64_t k, double v) { vals[k] = v; });
+}
+
+// The imaginary parts omega * M of the listed items (list[0] of them), resident CTAs striding.
+__global__ void __launch_bounds__(kMassBT, 2)
+    k_tile_complex_mass(const TileComplexInstance *__restrict__ inst, const int2 *__restrict__ items, int smem_nnz,
+                        int smem_inc, int smem_rows, int smem_chunks, const int *__restrict__ list) {
+    extern __shared__ __align__(16) double tile_smem[];
+    const TileSmem S = tile_smem_layout(tile_smem, smem_nnz, smem_inc, smem_rows, smem_chunks);
+    const int count = list[0];
+    for (int k = blockIdx.x; k < count; k += gridDim.x) {
+        const int2 w = items[list[1 + k]];
+        const TileComplexInstance &I = inst[w.x];
+        double *im = I.cvals + 1;
+        const double omega = I.omega;
+        tile_mass_block<kMassBT>(I.a, S, I.a.blocks + w.y, I.sigma, I.val_ref,
+                                 [&](int64_t k, double v) { im[2 * k] = omega * v; });
+        __syncthreads();  // the block's values are read out of shared memory
     }
 }
 
@@ -1055,19 +1151,26 @@ size_t tile_smem_bytes(const TilePlan &tp, TileArgs *a) {
            (size_t)(a->smem_rows + a->smem_chunks) * sizeof(uint2);
 }
 
+// Allows the kernel its shared memory and gives the CTAs resident at once on the device (how
+// far ahead a CTA prefetches).
+int resident_ctas(const void *kern, int threads, size_t smem, int *out) {
+    int dev = 0, nsm = 0, per = 0;
+    if (cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem) != cudaSuccess ||
+        cudaGetDevice(&dev) != cudaSuccess ||
+        cudaDeviceGetAttribute(&nsm, cudaDevAttrMultiProcessorCount, dev) != cudaSuccess ||
+        cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per, kern, threads, smem) != cudaSuccess || per < 1)
+        return MAG_E_CUDA;
+    *out = per * nsm;
+    return MAG_OK;
+}
+
 template <bool CALCJ, bool Q4, int MODE, int BT = kTileBT, int MINB = kTileMinB>
 int launch(const TileArgs &a, const TilePlan &tp, size_t smem, cudaStream_t s) {
     auto kern = k_tile<BT, MINB, CALCJ, Q4, MODE>;
-    if (cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem) != cudaSuccess)
-        return MAG_E_CUDA;
-    // CTAs resident at once: how far ahead a CTA prefetches
-    int dev = 0, nsm = 0, per = 0;
-    if (cudaGetDevice(&dev) != cudaSuccess ||
-        cudaDeviceGetAttribute(&nsm, cudaDevAttrMultiProcessorCount, dev) != cudaSuccess ||
-        cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per, kern, BT, smem) != cudaSuccess || per < 1)
-        return MAG_E_CUDA;
+    int resident = 0;
+    MAG_TRY(resident_ctas((const void *)kern, BT, smem, &resident));
     // (ahead >= nblocks: no CTA prefetches)
-    const int ahead = tp.prefetch_waves > 0 ? per * nsm * tp.prefetch_waves : tp.nblocks;
+    const int ahead = tp.prefetch_waves > 0 ? resident * tp.prefetch_waves : tp.nblocks;
     kern<<<tp.nblocks, BT, smem, s>>>(a, tp.nblocks, ahead);
     return cudaPeekAtLastError() == cudaSuccess ? MAG_OK : MAG_E_CUDA;
 }
@@ -1130,6 +1233,20 @@ int launch_tile_stiffness(const TilePlan &tp, const ElemData &m, const double *n
     return q4 ? launch<true, true, kStiffness>(a, tp, smem, s) : launch<true, false, kStiffness>(a, tp, smem, s);
 }
 
+int launch_tile_mass(const TilePlan &tp, const ElemData &m, const double *sigma, const QuadParams &qp, double *vals,
+                     int *err, cudaStream_t s) {
+    if (!tp.ok || qp.nq > kMaxQuad) return MAG_E_UNSUPPORTED;
+    TileArgs a = make_args(tp, m, qp, err);
+    a.vals = vals;
+    a.nnz_total = tp.nnz;
+    const size_t smem = tile_smem_bytes(tp, &a) + (size_t)18 * qp.nq * sizeof(double);
+    int resident = 0;
+    MAG_TRY(resident_ctas((const void *)k_tile_mass, kMassBT, smem, &resident));
+    const int ahead = tp.prefetch_waves > 0 ? resident * tp.prefetch_waves : tp.nblocks;
+    k_tile_mass<<<tp.nblocks, kMassBT, smem, s>>>(a, sigma, qp.val_ref, tp.nblocks, ahead);
+    return cudaPeekAtLastError() == cudaSuccess ? MAG_OK : MAG_E_CUDA;
+}
+
 int launch_tile_harmonic_dc(const TilePlan &tp, const ElemData &m, const double *nu_dc, const QuadParams &qp,
                             double *vals, int *err, cudaStream_t s) {
     if (!tp.ok || !qp.standard_curl || !qp.uniform_w) return MAG_E_UNSUPPORTED;
@@ -1159,7 +1276,7 @@ int launch_tile_seeded(const TilePlan &tp, const ElemData &m, const double *sol,
 
 namespace {
 
-using ComplexKernel = void (*)(const TileComplexInstance *, const int2 *, int, int, int, int, int, int);
+using ComplexKernel = void (*)(const TileComplexInstance *, const int2 *, int, int, int, int, int, int, int *);
 
 ComplexKernel complex_kernel(int variant, bool q4) {
     if (q4) return variant == 1 ? k_tile_complex<288, 2, true> : k_tile_complex<320, 2, true>;
@@ -1202,25 +1319,22 @@ int build_tile_complex(const std::vector<TileComplexInput> &in, TileComplexBatch
     if (items.empty() || items.size() >= (size_t)INT32_MAX) return MAG_OK;
     b->q4 = q4;
     b->smem = (size_t)b->smem_nnz * sizeof(double) + (size_t)b->smem_inc * sizeof(double2) +
-              (size_t)(b->smem_rows + b->smem_chunks) * sizeof(uint2) + (size_t)18 * kMaxQuad * sizeof(double);
-    int dev = 0, nsm = 0;
-    MAG_CUDA_TRY(cudaGetDevice(&dev));
-    MAG_CUDA_TRY(cudaDeviceGetAttribute(&nsm, cudaDevAttrMultiProcessorCount, dev));
-    for (int v = 0; v < kTileComplexVariants; v++) {
-        const ComplexKernel kern = complex_kernel(v, q4 != 0);
-        int per = 0;
-        if (cudaFuncSetAttribute((const void *)kern, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)b->smem) !=
-                cudaSuccess ||
-            cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per, (const void *)kern, kComplexThreads[v], b->smem) !=
-                cudaSuccess || per < 1) {
+              (size_t)(b->smem_rows + b->smem_chunks) * sizeof(uint2);
+    b->smem_mass = b->smem + (size_t)18 * kMaxQuad * sizeof(double);
+    for (int v = 0; v <= kTileComplexVariants; v++) {  // the last one: the mass kernel
+        const bool mass = v == kTileComplexVariants;
+        const void *kern = mass ? (const void *)k_tile_complex_mass : (const void *)complex_kernel(v, q4 != 0);
+        if (resident_ctas(kern, mass ? kMassBT : kComplexThreads[v], mass ? b->smem_mass : b->smem,
+                          mass ? &b->mass_ctas : &b->ahead[v]) != MAG_OK) {
             cudaGetLastError();
             *b = TileComplexBatch{};
             return MAG_OK;  // the blocks do not fit: the other batch variants remain
         }
-        b->ahead[v] = per * nsm;
     }
+    if (b->mass_ctas > (int)items.size()) b->mass_ctas = (int)items.size();
     if (cudaMalloc(&b->inst, hi.size() * sizeof(TileComplexInstance)) != cudaSuccess ||
-        cudaMalloc(&b->items, items.size() * sizeof(int2)) != cudaSuccess) {
+        cudaMalloc(&b->items, items.size() * sizeof(int2)) != cudaSuccess ||
+        cudaMalloc(&b->list, (items.size() + 1) * sizeof(int)) != cudaSuccess) {
         cudaGetLastError();
         free_tile_complex(b);
         return MAG_OK;
@@ -1236,9 +1350,12 @@ int build_tile_complex(const std::vector<TileComplexInput> &in, TileComplexBatch
 int launch_tile_complex(const TileComplexBatch &b, int variant, cudaStream_t s) {
     if (!b.ok || variant < 0 || variant >= kTileComplexVariants) return MAG_E_UNSUPPORTED;
     const ComplexKernel kern = complex_kernel(variant, b.q4 != 0);
-    kern<<<b.nitems, kComplexThreads[variant], b.smem, s>>>(static_cast<const TileComplexInstance *>(b.inst), b.items,
-                                                           b.nitems, b.ahead[variant], b.smem_nnz, b.smem_inc,
-                                                           b.smem_rows, b.smem_chunks);
+    const TileComplexInstance *inst = static_cast<const TileComplexInstance *>(b.inst);
+    if (cudaMemsetAsync(b.list, 0, sizeof(int), s) != cudaSuccess) return MAG_E_CUDA;
+    kern<<<b.nitems, kComplexThreads[variant], b.smem, s>>>(inst, b.items, b.nitems, b.ahead[variant], b.smem_nnz,
+                                                           b.smem_inc, b.smem_rows, b.smem_chunks, b.list);
+    k_tile_complex_mass<<<b.mass_ctas, kMassBT, b.smem_mass, s>>>(inst, b.items, b.smem_nnz, b.smem_inc, b.smem_rows,
+                                                                 b.smem_chunks, b.list);
     return cudaPeekAtLastError() == cudaSuccess ? MAG_OK : MAG_E_CUDA;
 }
 
@@ -1251,6 +1368,7 @@ const char *tile_complex_variant_name(int v) {
 void free_tile_complex(TileComplexBatch *b) {
     if (b->inst) cudaFree(b->inst);
     if (b->items) cudaFree(b->items);
+    if (b->list) cudaFree(b->list);
     *b = TileComplexBatch{};
 }
 

@@ -116,8 +116,8 @@ int launch_tile_seeded(const TilePlan &tp, const ElemData &m, const double *sol,
 const char *tile_variant_name(int v);
 
 // Batched complex assembly A_i = K_i(nu_i) + j omega_i M_i(sigma_i) over the tile blocks of
-// many meshes: one CTA per (mesh, block) item; K pass then, where the block holds a
-// conducting element, M pass over the same shared-memory slots.
+// many meshes: one CTA per (mesh, block) item for K, then resident CTAs over the items that
+// hold a conducting element for M.
 struct TileComplexInput {
     const TilePlan *tp;
     ElemData m;
@@ -136,8 +136,10 @@ struct TileComplexBatch {
     int2 *items = nullptr;  // device (mesh, block), larger meshes first
     int nitems = 0, q4 = 0;
     int smem_nnz = 0, smem_inc = 0, smem_rows = 0, smem_chunks = 0;
-    size_t smem = 0;
+    int *list = nullptr;    // device: count and items with a conducting element, of the running launch
+    size_t smem = 0, smem_mass = 0;
     int ahead[kTileComplexVariants] = {0, 0};  // CTAs resident at once per launch shape
+    int mass_ctas = 0;                         // of the mass kernel
     int ok = 0;
 };
 
@@ -150,6 +152,9 @@ void free_tile_complex(TileComplexBatch *b);
 // K(nu) with per-element reluctivity nu [Ne].
 int launch_tile_stiffness(const TilePlan &tp, const ElemData &m, const double *nu, const QuadParams &qp,
                           double *vals, int *err, cudaStream_t s);
+// M(sigma), sigma [Ne] or NULL (1 everywhere); any curl table and weights.
+int launch_tile_mass(const TilePlan &tp, const ElemData &m, const double *sigma, const QuadParams &qp, double *vals,
+                     int *err, cudaStream_t s);
 // The DC block of a harmonic-balance assembly from the time-averaged reluctivity nu_dc [Ne]
 // (equal quadrature weights).
 int launch_tile_harmonic_dc(const TilePlan &tp, const ElemData &m, const double *nu_dc, const QuadParams &qp,

@@ -122,3 +122,34 @@ def test_element_b_matches_postprocessor(oracle_port, flip):
         assert np.all(np.abs(b - B) <= 1e-12 * scale + 1e-300)
         assert bits_equal(bsq, (b[:, 0] * b[:, 0] + b[:, 1] * b[:, 1]) + b[:, 2] * b[:, 2])
     plan.close()
+
+
+@pytest.mark.parametrize("order", [1, 2])
+@pytest.mark.parametrize("sigma", ["one", "none", "slab", "all"])
+@pytest.mark.parametrize("n,absent", [((1, 1, 1), 0.0), ((9, 4, 5), 0.0), ((9, 8, 9), 0.05)])
+def test_mass_and_source_match_oracle(oracle_port, n, absent, sigma, order):
+    """M(sigma) through the tile blocks and the source vector: one element to several tiles, no,
+    few or all conducting elements, dofs missing, one and four quadrature points."""
+    mesh = synth.kuhn_box(*n, seed=5)
+    tags = synth.cube_layout(mesh)
+    edges, t2e, sign = oracle_port.generate_edges(mesh.T)
+    E = edges.shape[0]
+    rng = np.random.default_rng(n[0])
+    dofs = t2e.copy()
+    dofs[rng.random(dofs.shape) < absent] = -1
+    m = mex_inputs(mesh.P, mesh.T, dofs, sign, tags)
+    qw, val, curl = quadrature.reference_data(order)
+    plan = AssemblyPlan(mesh.P, mesh.T, dofs, E, tags, sign)
+    plan.set_quadrature(qw, curl, val)
+    assert plan.info.schedule == _lib.SCHEDULE_TILE_BLOCKS
+    s = rng.uniform(0.5, 2.0, mesh.num_elements) * synth.SIGMA_AL
+    s = {"one": None, "none": 0.0 * s, "slab": np.where(tags == synth.ALUMINIUM, s, 1e-13), "all": s}[sigma]
+    I, J, V = oracle_port.mass(m, np.ones(mesh.num_elements) if s is None else s, qw, val)
+    keep = (I > 0) & (J > 0)
+    _, _, ref = oracle_port.sparse_csr(I[keep], J[keep], V[keep], E, drop_zeros=False)
+    got = plan.mass(None if s is None else torch.as_tensor(s, device="cuda"))
+    assert bits_equal(got.cpu().numpy(), ref)
+    js = rng.normal(size=(mesh.num_elements, 3)) * (rng.random(mesh.num_elements) < 0.7)[:, None]
+    I, V = oracle_port.source(m, js, qw, val)
+    assert bits_equal(plan.source(torch.as_tensor(js, device="cuda")).cpu().numpy(), _vector(oracle_port, I, V, E))
+    plan.check()
