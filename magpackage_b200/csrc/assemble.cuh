@@ -9,6 +9,9 @@ namespace mag {
 
 int launch_jacobian_elems(const ElemData &m, const double *sol, const QuadParams &qp,
                           const MaterialParams &mp, int calcj, double *scratch, cudaStream_t s);
+// The residual alone (standard curl table); f: [Ne][6].
+int launch_residual(const ElemData &m, const RowPlan &rp, const double *sol, const QuadParams &qp,
+                    const MaterialParams &mp, double *f, double *res, cudaStream_t s);
 int launch_jacobian_seeded_elems(const ElemData &m, const double *sol, const double *bscale, const QuadParams &qp,
                                  const MaterialParams &mp, double *scratch, cudaStream_t s);
 int launch_seed_midpoint(const ElemData &m, const double *sol, const double *nu_hat, const MaterialParams &mp,

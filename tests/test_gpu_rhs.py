@@ -153,3 +153,37 @@ def test_mass_and_source_match_oracle(oracle_port, n, absent, sigma, order):
     I, V = oracle_port.source(m, js, qw, val)
     assert bits_equal(plan.source(torch.as_tensor(js, device="cuda")).cpu().numpy(), _vector(oracle_port, I, V, E))
     plan.check()
+
+
+@pytest.mark.parametrize("n,absent,weights", [((33, 32, 32), 0.0, "equal"), ((34, 33, 31), 0.03, "uneven"),
+                                              ((33, 32, 32), 0.0, "captured")])
+def test_residual_alone_equals_jacobian_call(n, absent, weights):
+    """The residual-only path of larger meshes gives the Jacobian call's residual (which the other
+    tests pin to the oracle) bit for bit, also with dofs missing, with uneven weights, and replayed
+    from a graph."""
+    from magpackage_b200.material import pack_material_data
+    from magpackage_b200.plan import generate_edges
+
+    mesh = synth.kuhn_box(*n, seed=2)
+    assert mesh.num_elements >= 200000
+    edges, t2e, sign = generate_edges(mesh.T)
+    g = torch.Generator(device="cuda").manual_seed(1)
+    dofs = torch.where(torch.rand(t2e.shape, generator=g, device="cuda") < absent, -1, t2e.long()).int()
+    plan = AssemblyPlan(mesh.P, mesh.T, dofs, int(edges.shape[0]), synth.cube_layout(mesh), sign)
+    plan.set_materials(pack_material_data(synth.standard_materials()))
+    if weights == "uneven":
+        qw, val, curl = quadrature.reference_data(2)
+        plan.set_quadrature(qw * np.array([1.0, 0.5, 1.25, 1.25]), curl, val)
+    sol = 3e-4 * torch.randn(plan.num_dofs, dtype=torch.float64, device="cuda", generator=g)
+    _, want = plan.jacobian(sol)
+    if weights == "captured":
+        got = plan.new_vector()
+        graph = torch.cuda.CUDAGraph()
+        with torch.cuda.graph(graph):
+            plan.jacobian(sol, None, got, calc_j=False)
+        got.zero_()
+        graph.replay()
+    else:
+        _, got = plan.jacobian(sol, calc_j=False)
+    assert torch.equal(got, want) and float(want.abs().max()) > 0
+    plan.check()
