@@ -1220,7 +1220,7 @@ int mag_mlp_create(const float *init_params, mag_mlp **out) {
     size_t pb = (size_t)kMlpParams * sizeof(float);
     if (cudaMalloc(&n->params, pb) != cudaSuccess || cudaMalloc(&n->grad, pb) != cudaSuccess ||
         cudaMalloc(&n->m, pb) != cudaSuccess || cudaMalloc(&n->v, pb) != cudaSuccess ||
-        cudaMalloc(&n->partial, pb * n->grid) != cudaSuccess ||
+        cudaMalloc(&n->partial, (size_t)kMlpPartial * sizeof(float) * n->grid) != cudaSuccess ||
         cudaMalloc(&n->ops, (size_t)kMlpOperandElems * sizeof(__nv_bfloat16)) != cudaSuccess ||
         cudaMalloc(&n->err, sizeof(int)) != cudaSuccess) {
         destroy_mlp(n);

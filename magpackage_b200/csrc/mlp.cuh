@@ -11,6 +11,7 @@
 namespace mag {
 
 constexpr int kMlpParams = 64 * 4 + 64 + 64 * 64 + 64 + 64 * 64 + 64 + 64 + 1;  // 8705
+constexpr int kMlpPartial = (kMlpParams + 3) & ~3;  // stride of the per-CTA partial gradients (16-byte rows)
 constexpr int kMlpOperandElems = 64 * 16 + 4 * 64 * 64;                       // BF16 images
 
 struct MlpForwardArgs {
@@ -33,7 +34,7 @@ struct MlpBackwardArgs {
     float loss_scale;       // dL/dy = (y - target) * loss_scale
     const float *params;
     const __nv_bfloat16 *ops;
-    float *grad_partial;    // [grid][kMlpParams]
+    float *grad_partial;    // [grid][kMlpPartial]
     float *grad;            // [kMlpParams]
     int *err;
     long long spin_limit;
