@@ -453,7 +453,8 @@ __global__ void __launch_bounds__(kRows, 6) k_mlp_forward(MlpForwardArgs a) {
 // read), columns 32 (w >> 2) .. + 31. The weight gradients dW = dZ^T H (FP32 dZ, BF16-valued H)
 // are register-tiled outer products over the rows, 4 x 4 outputs a thread, summed in row order;
 // they run while the tensor core forms the next layer's dZ W. Measured at 32,768 rows: 130 us
-// with one thread per row and 32 outputs a thread read from shared memory one by one, MEASURED
+// with one thread per row and 32 outputs a thread read from shared memory one by one, 43 us here,
+// most of it the shared-memory reads of the outer products (8 words for 16 products).
 constexpr int kBwd = 256;
 constexpr int kLd = kH + 4;  // row stride of the FP32 tiles: a column's rows fall into different banks
 
@@ -675,21 +676,31 @@ __global__ void __launch_bounds__(kBwd, 2) k_mlp_backward(MlpBackwardArgs a) {
     tmem_free(S);
 }
 
-// grad[p] = sum over CTAs (fixed order) of the partials; 16 loads in flight per thread.
-__global__ void __launch_bounds__(64) k_mlp_reduce(const float *__restrict__ partial, int nparts, float *__restrict__ grad) {
-    int p = blockIdx.x * blockDim.x + threadIdx.x;
-    if (p >= kMlpParams) return;
+// grad[p] = sum over CTAs (fixed order) of the partials. A CTA of eight warps takes 32
+// parameters: the warps load kRedChunk partials side by side into shared memory, the first one
+// adds them in order. (One thread per parameter loading as it adds: 13 us at 256 partials, a
+// chain of loads; 6.8 us so.)
+constexpr int kRedChunk = 256;
+__global__ void __launch_bounds__(256) k_mlp_reduce(const float *__restrict__ partial, int nparts, float *__restrict__ grad) {
+    __shared__ float sh[kRedChunk][32];
+    const int lane = threadIdx.x & 31, w = threadIdx.x >> 5, p = blockIdx.x * 32 + lane;
     float s = 0.0f;
-    int c = 0;
-    for (; c + 16 <= nparts; c += 16) {
-        float v[16];
+    for (int c0 = 0; c0 < nparts; c0 += kRedChunk) {
+        const int m = nparts - c0 < kRedChunk ? nparts - c0 : kRedChunk;
+        float v[kRedChunk / 8];
 #pragma unroll
-        for (int j = 0; j < 16; j++) v[j] = __ldg(partial + (size_t)(c + j) * kMlpPartial + p);
+        for (int j = 0; j < kRedChunk / 8; j++)
+            v[j] = w + 8 * j < m && p < kMlpParams ? __ldg(partial + (size_t)(c0 + w + 8 * j) * kMlpPartial + p) : 0.0f;
+        __syncthreads();
 #pragma unroll
-        for (int j = 0; j < 16; j++) s += v[j];
+        for (int j = 0; j < kRedChunk / 8; j++) sh[w + 8 * j][lane] = v[j];
+        __syncthreads();
+        if (w == 0) {
+#pragma unroll 16
+            for (int c = 0; c < m; c++) s += sh[c][lane];
+        }
     }
-    for (; c < nparts; c++) s += __ldg(partial + (size_t)c * kMlpPartial + p);
-    grad[p] = s;
+    if (w == 0 && p < kMlpParams) grad[p] = s;
 }
 
 // Adam step on the FP32 master weights.
@@ -796,7 +807,7 @@ int mlp_backward(const MlpBackwardArgs &a, int grid, cudaStream_t s) {
     cudaFuncSetAttribute(k_mlp_backward, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)sm);
     k_mlp_backward<<<grid, kBwd, sm, s>>>(a);
     if (cudaPeekAtLastError() != cudaSuccess) return MAG_E_CUDA;
-    k_mlp_reduce<<<(kMlpParams + 63) / 64, 64, 0, s>>>(a.grad_partial, grid, a.grad);
+    k_mlp_reduce<<<(kMlpParams + 31) / 32, 256, 0, s>>>(a.grad_partial, grid, a.grad);
     return cudaPeekAtLastError() == cudaSuccess ? MAG_OK : MAG_E_CUDA;
 }
 
