@@ -59,7 +59,7 @@ typedef struct {
     int32_t reserved0;      /* 0 */
     int32_t nz_pass;        /* 1 if MAG_SCHEDULE_NZ_ROW_BLOCKS is available for this mesh */
     double tile_evals_per_elem; /* element evaluations per element and assembly of the tile schedule */
-    double tile_plan_ms;    /* host time to build its plan */
+    double tile_plan_ms;    /* time to build its plan */
 } mag_mesh_info;
 
 /* Jacobian assembly schedules; all give identical bits. */

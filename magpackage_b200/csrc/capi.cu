@@ -594,7 +594,7 @@ int mag_mesh_create(const double *d_P, int64_t Nn, const int32_t *d_T, int64_t N
         const TilePlanInput ti{m->xyz, m->tet, m->dofs, m->tags, m->signbits, m->pat.row_ptr, m->pat.inc_ptr,
                                m->pat.inc_elem, m->pat.inc_pos, Nn, Ne, num_dofs, m->pat.nnz, m->pat.ninc,
                                m->pat.wide};
-        rc = build_tile_plan(ti, &m->tile, s);
+        rc = build_tile_plan(ti, m->scratch, (size_t)Ne * kScratchPerElem * sizeof(double), &m->tile, s);
         if (rc != MAG_OK) return fail(rc);
         if (m->tile.ok) m->bytes += m->tile.bytes;
         make_residual_buffer(m);

@@ -22,28 +22,12 @@
 //   store phase -- the block's rows form runs of consecutive rows, contiguous in the
 //              CSR; warps store them in chunks, coalesced.
 // No floating-point atomics; results equal the reference's MEX + sparse() bit for bit.
-#include <omp.h>
-
 #include <algorithm>
-#include <atomic>
-#include <chrono>
-#include <cmath>
-#include <cstdlib>
-#include <cstring>
 #include <vector>
 
 #include "common.cuh"
 #include "element.cuh"
 #include "tile.cuh"
-
-// Node layers per tile along z (x and y: 4); a build option (-DMAG_TILE_LAYERS_Z=n).
-#ifndef MAG_TILE_LAYERS_Z
-#define MAG_TILE_LAYERS_Z 4
-#endif
-// Order a colour's records by the rows they hold in the block (build option).
-#ifndef MAG_TILE_SORT_ROWS
-#define MAG_TILE_SORT_ROWS 0
-#endif
 
 namespace mag {
 
@@ -651,492 +635,7 @@ __global__ void __launch_bounds__(kMassBT, 2)
 constexpr int kTileBT = 320;
 constexpr int kTileMinB = 2;
 
-// ---- host plan builder --------------------------------------------------------------
-
-struct HostRec {
-    uint32_t w[24];  // the six 16-byte planes of one record, plane-major
-};
-
-// Layer index of every node along one axis: sorted coordinates split where
-// consecutive values are more than 0.3 h apart or a layer would span more than h.
-void axis_layers(const std::vector<double4> &xyz, int axis, double h, std::vector<int32_t> &layer) {
-    const int64_t n = (int64_t)xyz.size();
-    std::vector<std::pair<double, int32_t>> v((size_t)n);
-    for (int64_t i = 0; i < n; i++) {
-        const double c = axis == 0 ? xyz[i].x : axis == 1 ? xyz[i].y : xyz[i].z;
-        v[i] = {c, (int32_t)i};
-    }
-    std::sort(v.begin(), v.end());
-    layer.assign((size_t)n, 0);
-    int32_t L = 0;
-    double start = n ? v[0].first : 0.0;
-    for (int64_t i = 1; i < n; i++) {
-        const double x = v[i].first;
-        if (x - v[i - 1].first > 0.3 * h || x - start > h) {
-            L++;
-            start = x;
-        }
-        layer[v[i].second] = L;
-    }
-}
-
-template <typename T>
-int download(std::vector<T> &dst, const T *src, int64_t count, cudaStream_t s) {
-    dst.resize((size_t)count);
-    if (count == 0) return MAG_OK;
-    MAG_CUDA_TRY(cudaMemcpyAsync(dst.data(), src, (size_t)count * sizeof(T), cudaMemcpyDeviceToHost, s));
-    return MAG_OK;
-}
-
 }  // namespace
-
-void free_tile_plan(TilePlan *p) {
-    void *q[] = {p->blocks, p->rows, p->chunks, p->recs};
-    for (void *x : q)
-        if (x) cudaFree(x);
-    *p = TilePlan{};
-}
-
-bool plan_tiles_host(const TileHostMesh &hm, TileHostPlan *out) {
-    *out = TileHostPlan{};
-    const std::vector<double4> &xyz = hm.xyz;
-    const std::vector<int4> &tet = hm.tet;
-    const std::vector<int32_t> &dofs = hm.dofs, &row_ptr = hm.row_ptr, &inc_ptr = hm.inc_ptr;
-    const std::vector<uint8_t> &tags = hm.tags, &sbits = hm.sbits;
-    const std::vector<uint32_t> &inc_elem = hm.inc_elem, &inc_pos = hm.inc_pos;
-    const int64_t ndof = (int64_t)row_ptr.size() - 1, ne = (int64_t)tet.size();
-    const int64_t ninc_total = (int64_t)inc_elem.size();
-    const bool have_signs = !sbits.empty();
-    if (ne <= 0 || ndof <= 0 || hm.nnz >= (int64_t(1) << 32)) return false;
-
-    // an element with a repeated dof would update a diagonal slot or one slot twice
-    for (int64_t e = 0; e < ne; e++)
-        for (int a = 0; a < 6; a++)
-            for (int b = a + 1; b < 6; b++)
-                if (dofs[6 * e + a] >= 0 && dofs[6 * e + a] == dofs[6 * e + b]) return false;
-
-    // ---- spatial layers and tiles ----
-    double lo[3] = {1e300, 1e300, 1e300}, hi[3] = {-1e300, -1e300, -1e300};
-    for (const double4 &p : xyz) {
-        const double c[3] = {p.x, p.y, p.z};
-        for (int a = 0; a < 3; a++) {
-            lo[a] = std::min(lo[a], c[a]);
-            hi[a] = std::max(hi[a], c[a]);
-        }
-    }
-    double vol = 1.0, ext_max = 0.0;
-    for (int a = 0; a < 3; a++) {
-        vol *= hi[a] - lo[a];
-        ext_max = std::max(ext_max, hi[a] - lo[a]);
-    }
-    const double nn = (double)xyz.size();
-    double h = vol > 0.0 ? std::cbrt(vol / nn) : ext_max / std::max(1.0, std::cbrt(nn));
-    if (!(h > 0.0)) h = 1.0;
-    std::vector<int32_t> layer[3];
-    for (int a = 0; a < 3; a++) axis_layers(xyz, a, h, layer[a]);
-    constexpr int kTileLayers[3] = {4, 4, MAG_TILE_LAYERS_Z};
-    int32_t ntile[3] = {1, 1, 1};
-    for (int a = 0; a < 3; a++) {
-        int32_t m = 0;
-        for (int32_t v : layer[a]) m = std::max(m, v);
-        ntile[a] = m / kTileLayers[a] + 1;
-    }
-    const int64_t tiles = (int64_t)ntile[0] * ntile[1] * ntile[2];
-    if (tiles >= (int64_t(1) << 31)) return false;
-    // tile of every row: that of its edge's lower node; a row without incidences
-    // (an unused dof) joins the tile of the row before it
-    std::vector<int32_t> row_tile((size_t)ndof, 0);
-    {
-        int32_t prev = 0;
-        for (int64_t r = 0; r < ndof; r++) {
-            if (inc_ptr[r + 1] > inc_ptr[r]) {
-                const uint32_t ew = inc_elem[inc_ptr[r]];
-                const int64_t e = ew & 0x1FFFFFFFu;
-                const int l = (int)(ew >> 29);
-                const int *t = &tet[e].x;
-                const int32_t na = t[edge_a(l)], nb = t[edge_b(l)];
-                const int32_t node = na < nb ? na : nb;
-                prev = (layer[0][node] / kTileLayers[0]) +
-                       ntile[0] * ((layer[1][node] / kTileLayers[1]) + ntile[1] * (layer[2][node] / kTileLayers[2]));
-            }
-            row_tile[r] = prev;
-        }
-    }
-    // rows grouped by tile (stable: ascending ids within a tile)
-    std::vector<int64_t> tstart((size_t)tiles + 1, 0);
-    for (int64_t r = 0; r < ndof; r++) tstart[row_tile[r] + 1]++;
-    for (int64_t t = 0; t < tiles; t++) tstart[t + 1] += tstart[t];
-    std::vector<int32_t> order((size_t)ndof);
-    {
-        std::vector<int64_t> fill(tstart.begin(), tstart.end() - 1);
-        for (int64_t r = 0; r < ndof; r++) order[fill[row_tile[r]]++] = (int32_t)r;
-    }
-    // blocks: each tile's rows, cut where a block would exceed its capacity
-    std::vector<int64_t> bstart;  // index into order
-    for (int64_t t = 0; t < tiles; t++) {
-        int64_t k = tstart[t];
-        const int64_t k1 = tstart[t + 1];
-        while (k < k1) {
-            bstart.push_back(k);
-            int64_t bn = 0, bi = 0;
-            while (k < k1) {
-                const int32_t r = order[k];
-                const int64_t rn = row_ptr[r + 1] - row_ptr[r], ri = inc_ptr[r + 1] - inc_ptr[r];
-                if (rn > kCompactMaxRow || ri > kCompactMaxRow) return false;
-                if (bn + rn > kTileMaxNnz || bi + ri > kTileMaxInc) break;
-                bn += rn;
-                bi += ri;
-                k++;
-            }
-        }
-    }
-    bstart.push_back(ndof);
-    const int64_t nb = (int64_t)bstart.size() - 1;
-    if (nb >= (int64_t(1) << 31)) return false;
-
-    std::vector<TileBlock> blocks((size_t)nb);
-    std::vector<uint2> rows((size_t)ndof);
-    std::vector<std::vector<HostRec>> brec((size_t)nb);
-    std::vector<std::vector<uint2>> bchunk((size_t)nb);
-    std::atomic<int> fail{0};
-
-#pragma omp parallel
-    {
-        struct Inc {
-            int64_t e;
-            int l;
-            int lr;     // block-local row
-            int32_t k;  // incidence index
-        };
-        std::vector<Inc> incs;
-        std::vector<int32_t> own_a, own_b, color, adj_ptr, adj, queue;
-        std::vector<uint8_t> cnt;
-#pragma omp for schedule(dynamic, 16)
-        for (int64_t b = 0; b < nb; b++) {
-            if (fail) continue;
-            const int64_t k0 = bstart[b], k1 = bstart[b + 1];
-            TileBlock &B = blocks[b];
-            std::memset(&B, 0, sizeof B);
-            B.row0 = (int32_t)k0;
-            B.nrows = (int32_t)(k1 - k0);
-            // row table and incidences
-            int32_t bn = 0, bi = 0;
-            incs.clear();
-            for (int64_t k = k0; k < k1; k++) {
-                const int32_t r = order[k];
-                const int32_t rn = row_ptr[r + 1] - row_ptr[r];
-                const int32_t i0 = inc_ptr[r], i1 = inc_ptr[r + 1];
-                uint32_t diag = 0;
-                for (int32_t t = i0; t < i1; t++) {
-                    const uint32_t ew = inc_elem[t];
-                    const int l = (int)(ew >> 29);
-                    if (t == i0) diag = (inc_pos[t] >> (5 * l)) & 31u;
-                    incs.push_back(Inc{(int64_t)(ew & 0x1FFFFFFFu), l, (int)(k - k0), t});
-                }
-                rows[k] = make_uint2((uint32_t)r, (uint32_t)bn | ((uint32_t)bi << 13) | (diag << 25));
-                bn += rn;
-                bi += i1 - i0;
-            }
-            B.nnz = bn;
-            B.ninc = bi;
-            // store chunks: runs of consecutive rows, cut at kTileChunk nonzeros
-            std::vector<uint2> &ch = bchunk[b];
-            ch.clear();
-            {
-                int32_t off = 0;
-                int64_t k = k0;
-                while (k < k1) {
-                    int64_t k2 = k + 1;
-                    while (k2 < k1 && order[k2] == order[k2 - 1] + 1) k2++;
-                    const int64_t g0 = row_ptr[order[k]], g1 = row_ptr[order[k2 - 1] + 1];
-                    for (int64_t g = g0; g < g1; g += kTileChunk) {
-                        const int32_t len = (int32_t)std::min<int64_t>(kTileChunk, g1 - g);
-                        ch.push_back(make_uint2((uint32_t)(off + (g - g0)) | ((uint32_t)len << 16), (uint32_t)g));
-                    }
-                    off += (int32_t)(g1 - g0);
-                    k = k2;
-                }
-            }
-            B.nchunks = (int32_t)ch.size();
-            // distinct elements (ascending) and their records
-            std::sort(incs.begin(), incs.end(), [](const Inc &x, const Inc &y) {
-                return x.e != y.e ? x.e < y.e : x.l < y.l;
-            });
-            std::vector<HostRec> &rec = brec[b];
-            rec.clear();
-            for (size_t q = 0; q < incs.size(); q++) {
-                const Inc &c = incs[q];
-                if (q == 0 || incs[q - 1].e != c.e) {
-                    HostRec h;
-                    const int64_t e = c.e;
-                    const int4 tt = tet[e];
-                    h.w[0] = (uint32_t)tt.x;
-                    h.w[1] = (uint32_t)tt.y;
-                    h.w[2] = (uint32_t)tt.z;
-                    h.w[3] = (uint32_t)tt.w;
-                    for (int j = 0; j < 4; j++) h.w[4 + j] = (uint32_t)dofs[6 * e + j];
-                    h.w[8] = (uint32_t)dofs[6 * e + 4];
-                    h.w[9] = (uint32_t)dofs[6 * e + 5];
-                    h.w[10] = (uint32_t)e;
-                    unsigned sb = 0;
-                    if (have_signs) {
-                        sb = sbits[e];
-                    } else {
-                        const int n4[4] = {tt.x, tt.y, tt.z, tt.w};
-                        for (int j = 0; j < 6; j++) sb |= (n4[edge_a(j)] < n4[edge_b(j)] ? 0u : 1u) << j;
-                    }
-                    h.w[11] = (uint32_t)tags[e] | (sb << 8);
-                    for (int j = 12; j < 18; j++) h.w[j] = 0;
-                    for (int j = 18; j < 24; j++) h.w[j] = kTileAbsent;
-                    rec.push_back(h);
-                } else if (incs[q - 1].l == c.l) {
-                    fail = 1;  // one element twice in a row's incidences at the same local row
-                }
-                HostRec &h = rec.back();
-                const uint2 rw = rows[k0 + c.lr];
-                const int32_t r = order[k0 + c.lr];
-                const uint32_t nzb = rw.y & 0x1FFFu, incb = (rw.y >> 13) & 0xFFFu;
-                h.w[12 + c.l] = inc_pos[c.k];
-                h.w[18 + c.l] = nzb | ((incb + (uint32_t)(c.k - inc_ptr[r])) << 16);
-            }
-            const int32_t nr = (int32_t)rec.size();
-            // colour classes: conflict = two elements updating the same off-diagonal slot
-            own_a.assign((size_t)bn, -1);
-            own_b.assign((size_t)bn, -1);
-            cnt.assign((size_t)bn, 0);
-            for (int32_t i = 0; i < nr && !fail; i++) {
-                const HostRec &h = rec[i];
-                for (int l = 0; l < 6; l++) {
-                    if (h.w[18 + l] == kTileAbsent) continue;
-                    const uint32_t nzb = h.w[18 + l] & 0xFFFFu;
-                    for (int j = 0; j < 6; j++) {
-                        if (j == l) continue;
-                        const uint32_t p = (h.w[12 + l] >> (5 * j)) & 31u;
-                        if (p == (uint32_t)kCompactMaxRow) continue;
-                        const uint32_t sl = nzb + p;
-                        if (sl >= (uint32_t)bn || cnt[sl] >= 2) {
-                            fail = 1;
-                            break;
-                        }
-                        if (cnt[sl] == 0) own_a[sl] = i;
-                        else own_b[sl] = i;
-                        cnt[sl]++;
-                    }
-                }
-            }
-            if (fail) continue;
-            // An absent column (a dof of -1) of a row points at the row's own diagonal
-            // nonzero: the kernels add its discarded value there without a test, and the row
-            // phase overwrites that slot with the diagonal's element-ordered sum afterwards.
-            for (int32_t i = 0; i < nr; i++) {
-                HostRec &h = rec[i];
-                for (int l = 0; l < 6; l++) {
-                    if (h.w[18 + l] == kTileAbsent) continue;
-                    const uint32_t diagp = (h.w[12 + l] >> (5 * l)) & 31u;
-                    for (int j = 0; j < 6; j++)
-                        if (((h.w[12 + l] >> (5 * j)) & 31u) == (uint32_t)kCompactMaxRow)
-                            h.w[12 + l] = (h.w[12 + l] & ~(31u << (5 * j))) | (diagp << (5 * j));
-                }
-            }
-            // adjacency (CSR over records)
-            adj_ptr.assign((size_t)nr + 1, 0);
-            for (int32_t sl = 0; sl < bn; sl++)
-                if (cnt[sl] == 2) {
-                    adj_ptr[own_a[sl] + 1]++;
-                    adj_ptr[own_b[sl] + 1]++;
-                }
-            for (int32_t i = 0; i < nr; i++) adj_ptr[i + 1] += adj_ptr[i];
-            adj.assign((size_t)adj_ptr[nr], 0);
-            {
-                std::vector<int32_t> f(adj_ptr.begin(), adj_ptr.end() - 1);
-                for (int32_t sl = 0; sl < bn; sl++)
-                    if (cnt[sl] == 2) {
-                        adj[f[own_a[sl]]++] = own_b[sl];
-                        adj[f[own_b[sl]]++] = own_a[sl];
-                    }
-            }
-            // two colours by breadth-first search where the graph is bipartite (components
-            // flipped to balance the classes), else greedy in element order
-            color.assign((size_t)nr, -1);
-            bool two = true;
-            int64_t size0 = 0, size1 = 0;
-            for (int32_t s0 = 0; s0 < nr && two; s0++) {
-                if (color[s0] >= 0) continue;
-                queue.clear();
-                queue.push_back(s0);
-                color[s0] = 0;
-                int64_t c0 = 1, c1 = 0;
-                for (size_t qh = 0; qh < queue.size() && two; qh++) {
-                    const int32_t u = queue[qh];
-                    for (int32_t t = adj_ptr[u]; t < adj_ptr[u + 1]; t++) {
-                        const int32_t w = adj[t];
-                        if (color[w] < 0) {
-                            color[w] = 1 - color[u];
-                            (color[w] ? c1 : c0)++;
-                            queue.push_back(w);
-                        } else if (color[w] == color[u]) {
-                            two = false;
-                            break;
-                        }
-                    }
-                }
-                if (two && std::llabs((size0 + c1) - (size1 + c0)) < std::llabs((size0 + c0) - (size1 + c1))) {
-                    for (int32_t u : queue) color[u] = 1 - color[u];
-                    std::swap(c0, c1);
-                }
-                size0 += c0;
-                size1 += c1;
-            }
-            int ncol = 2;
-            if (!two) {
-                color.assign((size_t)nr, -1);
-                ncol = 0;
-                for (int32_t u = 0; u < nr; u++) {
-                    unsigned used = 0;
-                    for (int32_t t = adj_ptr[u]; t < adj_ptr[u + 1]; t++)
-                        if (color[adj[t]] >= 0) used |= 1u << color[adj[t]];
-                    int c = 0;
-                    while (c < 32 && (used >> c) & 1u) c++;
-                    color[u] = c;
-                    ncol = std::max(ncol, c + 1);
-                }
-                if (ncol > kTileMaxColors) {
-                    fail = 1;
-                    continue;
-                }
-            }
-            // records by colour; within a colour in ascending element order, or (build option)
-            // by the set of the element's rows in the block, most rows first, so that the
-            // threads of a warp run the same rows
-            std::vector<int32_t> idx((size_t)nr);
-            std::vector<uint32_t> rkey((size_t)nr, 0u);
-            for (int32_t i = 0; i < nr; i++) {
-                idx[i] = i;
-                if (MAG_TILE_SORT_ROWS) {
-                    uint32_t m = 0;
-                    for (int l = 0; l < 6; l++) m |= (rec[i].w[18 + l] != kTileAbsent ? 1u : 0u) << l;
-                    rkey[i] = ((6u - (uint32_t)__builtin_popcount(m)) << 6) | m;
-                }
-            }
-            std::stable_sort(idx.begin(), idx.end(), [&](int32_t x, int32_t y) {
-                return color[x] != color[y] ? color[x] < color[y] : rkey[x] < rkey[y];
-            });
-            std::vector<HostRec> sorted((size_t)nr);
-            for (int32_t i = 0; i < nr; i++) sorted[i] = rec[idx[i]];
-            rec.swap(sorted);
-            B.nrec = nr;
-            B.ncolors = ncol;
-            for (int c = 0; c < kTileMaxColors; c++) B.col_end[c] = 0;
-            for (int32_t i = 0; i < nr; i++) B.col_end[color[idx[i]]] = i + 1;
-            for (int c = 1; c < ncol; c++) B.col_end[c] = std::max(B.col_end[c], B.col_end[c - 1]);
-        }
-    }
-    if (fail) return false;
-
-    // concatenate: record and chunk offsets, planes
-    int64_t nrec = 0, nch = 0;
-    int32_t max_nnz = 0, max_inc = 0, max_col = 0, max_rows = 0, max_ch = 0;
-    for (int64_t b = 0; b < nb; b++) {
-        blocks[b].rec0 = (int32_t)nrec;
-        blocks[b].chunk0 = (int32_t)nch;
-        nrec += blocks[b].nrec;
-        nch += blocks[b].nchunks;
-        max_nnz = std::max(max_nnz, blocks[b].nnz);
-        max_inc = std::max(max_inc, blocks[b].ninc);
-        max_col = std::max(max_col, blocks[b].ncolors);
-        max_rows = std::max(max_rows, blocks[b].nrows);
-        max_ch = std::max(max_ch, blocks[b].nchunks);
-        if (nrec >= (int64_t(1) << 31) || nch >= (int64_t(1) << 31)) return false;
-    }
-    std::vector<uint4> planes((size_t)(6 * nrec));
-    std::vector<uint2> chunks((size_t)nch);
-#pragma omp parallel for schedule(dynamic, 64)
-    for (int64_t b = 0; b < nb; b++) {
-        const std::vector<HostRec> &rec = brec[b];
-        const int64_t o = blocks[b].rec0;
-        for (size_t i = 0; i < rec.size(); i++)
-            for (int k = 0; k < 6; k++) {
-                const uint32_t *w = rec[i].w + 4 * k;
-                planes[(size_t)k * nrec + o + i] = make_uint4(w[0], w[1], w[2], w[3]);
-            }
-        std::copy(bchunk[b].begin(), bchunk[b].end(), chunks.begin() + blocks[b].chunk0);
-    }
-    // coverage check: every incidence is one record slot
-    {
-        int64_t present = 0;
-        for (int64_t i = 0; i < nrec; i++) {
-            const uint4 a = planes[4 * nrec + i], c = planes[5 * nrec + i];
-            const uint32_t sl[6] = {a.z, a.w, c.x, c.y, c.z, c.w};
-            for (int l = 0; l < 6; l++) present += sl[l] != kTileAbsent;
-        }
-        if (present != ninc_total) return false;
-    }
-    out->blocks.swap(blocks);
-    out->rows.swap(rows);
-    out->chunks.swap(chunks);
-    out->planes.swap(planes);
-    out->nrec = nrec;
-    out->max_nnz = max_nnz;
-    out->max_inc = max_inc;
-    out->max_colors = max_col;
-    out->max_rows = max_rows;
-    out->max_chunks = max_ch;
-    return true;
-}
-
-int build_tile_plan(const TilePlanInput &in, TilePlan *plan, cudaStream_t s) {
-    *plan = TilePlan{};
-    if (in.wide || in.ne <= 0 || in.ndof <= 0 || in.nnz >= (int64_t(1) << 32)) return MAG_OK;
-    const auto t_start = std::chrono::steady_clock::now();
-    TileHostMesh hm;
-    MAG_TRY(download(hm.xyz, in.xyz, in.nn, s));
-    MAG_TRY(download(hm.tet, in.tet, in.ne, s));
-    MAG_TRY(download(hm.dofs, in.dofs, 6 * in.ne, s));
-    MAG_TRY(download(hm.tags, in.tags, in.ne, s));
-    if (in.signbits) MAG_TRY(download(hm.sbits, in.signbits, in.ne, s));
-    MAG_TRY(download(hm.row_ptr, in.row_ptr, in.ndof + 1, s));
-    MAG_TRY(download(hm.inc_ptr, in.inc_ptr, in.ndof + 1, s));
-    MAG_TRY(download(hm.inc_elem, in.inc_elem, in.ninc, s));
-    MAG_TRY(download(hm.inc_pos, in.inc_pos, in.ninc, s));
-    MAG_CUDA_TRY(cudaStreamSynchronize(s));
-    hm.nnz = in.nnz;
-    TileHostPlan hp;
-    if (!plan_tiles_host(hm, &hp)) return MAG_OK;
-    TilePlan p;
-    const int64_t nb = (int64_t)hp.blocks.size(), nch = (int64_t)hp.chunks.size(), nrec = hp.nrec;
-    p.nblocks = (int32_t)nb;
-    p.nrows = in.ndof;
-    p.nchunks = nch;
-    p.nrec = nrec;
-    p.nnz = in.nnz;
-    p.max_nnz = hp.max_nnz;
-    p.max_inc = hp.max_inc;
-    p.max_colors = hp.max_colors;
-    p.max_rows = hp.max_rows;
-    p.max_chunks = hp.max_chunks;
-    p.evals_per_elem = (double)nrec / (double)in.ne;
-    // rows and chunks padded by 16 bytes: the kernel's L2 prefetches round to 16 bytes
-    const size_t b_blk = (size_t)nb * sizeof(TileBlock), b_rows = hp.rows.size() * sizeof(uint2) + 16,
-                 b_ch = (size_t)std::max<int64_t>(nch, 1) * sizeof(uint2) + 16,
-                 b_rec = (size_t)std::max<int64_t>(6 * nrec, 1) * sizeof(uint4);
-    if (cudaMalloc(&p.blocks, b_blk) != cudaSuccess || cudaMalloc(&p.rows, b_rows) != cudaSuccess ||
-        cudaMalloc(&p.chunks, b_ch) != cudaSuccess || cudaMalloc(&p.recs, b_rec) != cudaSuccess) {
-        free_tile_plan(&p);
-        cudaGetLastError();
-        return MAG_OK;  // no room: the other schedules remain
-    }
-    MAG_CUDA_TRY(cudaMemcpyAsync(p.blocks, hp.blocks.data(), b_blk, cudaMemcpyHostToDevice, s));
-    MAG_CUDA_TRY(cudaMemcpyAsync(p.rows, hp.rows.data(), hp.rows.size() * sizeof(uint2), cudaMemcpyHostToDevice, s));
-    if (nch) MAG_CUDA_TRY(cudaMemcpyAsync(p.chunks, hp.chunks.data(), nch * sizeof(uint2), cudaMemcpyHostToDevice, s));
-    if (nrec)
-        MAG_CUDA_TRY(cudaMemcpyAsync(p.recs, hp.planes.data(), 6 * nrec * sizeof(uint4), cudaMemcpyHostToDevice, s));
-    MAG_CUDA_TRY(cudaStreamSynchronize(s));
-    p.bytes = (int64_t)(b_blk + b_rows + b_ch + b_rec);
-    p.build_ms = std::chrono::duration<double, std::milli>(std::chrono::steady_clock::now() - t_start).count();
-    p.ok = 1;
-    *plan = p;
-    return MAG_OK;
-}
 
 namespace {
 

@@ -75,33 +75,12 @@ struct TilePlanInput {
     int wide;
 };
 
-// Host copies of what the planner reads (the device mesh and incidence plan).
-struct TileHostMesh {
-    std::vector<double4> xyz;
-    std::vector<int4> tet;
-    std::vector<int32_t> dofs, row_ptr, inc_ptr;
-    std::vector<uint8_t> tags, sbits;  // sbits empty: signs derived from tet
-    std::vector<uint32_t> inc_elem, inc_pos;
-    int64_t nnz = 0;
-};
-
-// The plan's arrays on the host, in the device layout.
-struct TileHostPlan {
-    std::vector<TileBlock> blocks;
-    std::vector<uint2> rows, chunks;
-    std::vector<uint4> planes;  // 6 * nrec
-    int64_t nrec = 0;
-    int32_t max_nnz = 0, max_inc = 0, max_colors = 0, max_rows = 0, max_chunks = 0;
-};
-
-// The planner itself (host only): false when the mesh does not suit the schedule.
-bool plan_tiles_host(const TileHostMesh &hm, TileHostPlan *out);
-
-// Builds the plan on the host from the mesh's incidence plan (copied down once).
+// Builds the plan on the GPU (tileplan.cu); work: device workspace, 384 bytes an element hold it
+// (beyond it, stream-ordered allocations).
 // Leaves plan->ok = 0 (and returns MAG_OK) when the mesh does not suit the schedule:
 // wide rows (> 31 entries), an off-diagonal entry with more than two contributions
 // (repeated dofs), or a block needing more than kTileMaxColors colours.
-int build_tile_plan(const TilePlanInput &in, TilePlan *plan, cudaStream_t s);
+int build_tile_plan(const TilePlanInput &in, void *work, size_t work_bytes, TilePlan *plan, cudaStream_t s);
 void free_tile_plan(TilePlan *plan);
 
 // Jacobian (calc_j) and residual; vals may be NULL when !calc_j.

@@ -770,3 +770,57 @@ def test_tile_schedule_shuffled_numbering_and_unused_dofs(oracle_port):
     assert_csr_equal(plan.row_ptr, plan.col_idx, plan.stiffness(dev(nu)), oracle_matrix(oracle_port, Ik, Jk, Vk, n, False))
     plan.check()
     plan.close()
+
+
+def _stars(count):
+    """`count` separate rings of five tetrahedra around an edge: face-adjacency cycles of odd length."""
+    ang = 2 * np.pi * np.arange(5) / 5
+    P1 = np.vstack([[0, 0, 0], [0.1, 0.2, 1.0], np.stack([np.cos(ang), np.sin(ang), 0.5 + 0.1 * ang], 1)])
+    T1 = np.array([[0, 1, 2 + k, 2 + (k + 1) % 5] for k in range(5)])
+    rng = np.random.default_rng(count)
+    P = np.vstack([P1 + 0.05 * rng.normal(size=P1.shape) + [3.0 * (c % 4), 3.0 * (c // 4), 0.0] for c in range(count)])
+    T = np.vstack([T1 + 7 * c for c in range(count)])
+    return P, T.astype(np.int32), np.where(np.arange(len(T)) % 3 == 0, 2, 1).astype(np.int32)
+
+
+@pytest.mark.parametrize("form", ["one_tet", "stars", "far_element", "flat", "gaps"])
+def test_tile_plan_forms(oracle_port, form):
+    """Meshes that reach each branch of the plan builder: a single element, blocks that two colours
+    do not serve, a tile that exceeds a block's capacity and is cut, a box of one layer, layers far
+    apart; the Jacobian, residual and K(nu) equal the oracle's."""
+    if form == "one_tet":
+        P, T, tags = np.array([[0, 0, 0], [1, 0, 0], [0, 1, 0], [0, 0, 1.0]]), np.array([[0, 1, 2, 3]], np.int32), np.array([2])
+    elif form == "stars":
+        P, T, tags = _stars(23)
+    else:
+        mesh = synth.kuhn_box(*{"far_element": (11, 10, 9), "flat": (17, 13, 1), "gaps": (9, 9, 9)}[form], seed=7)
+        P, T, tags = mesh.P.copy(), mesh.T, synth.cube_layout(mesh)
+        if form == "far_element":  # the spacing estimate grows: all other nodes fall into one tile
+            far = np.array([[0, 0, 0], [50.0, 0, 0], [0, 60.0, 0], [0, 0, 70.0]]) + [2000.0, 1500.0, 1800.0]
+            P, T = np.vstack([P, far]), np.vstack([T, len(P) + np.array([[0, 1, 2, 3]], np.int32)]).astype(np.int32)
+            tags = np.r_[tags, 1].astype(np.int32)
+        if form == "gaps":
+            P[:, 0] = np.where(P[:, 0] > 0.5, P[:, 0] + 3.0, P[:, 0])
+            P[:, 2] = P[:, 2] ** 3
+    edges, t2e, sign, m = make_case(oracle_port, P, T, tags)
+    E = edges.shape[0]
+    pk = material.pack_material_data(synth.standard_materials())
+    plan = AssemblyPlan(P, T, t2e, E, tags, sign)
+    plan.set_materials(pk)
+    assert plan.info.schedule == _lib.SCHEDULE_TILE_BLOCKS
+    assert (plan.info.tile_colors > 2) == (form == "stars")
+    if form == "one_tet":
+        assert plan.info.tile_blocks == 1
+    if form == "far_element":  # filled to the capacity of 8,191 nonzeros (rows have at most 31), plus the far tile
+        assert plan.nnz / 8191 <= plan.info.tile_blocks <= plan.nnz / (8191 - 31) + 2
+    rng = np.random.default_rng(3)
+    sol = rng.normal(0, 0.05, E)
+    qw, val, curl = quadrature.reference_data(2)
+    I, J, V, Ri, Rv = oracle_port.jacobian(m, sol, qw, curl, pk, True)
+    vals, res = plan.jacobian(dev(sol))
+    assert_csr_equal(plan.row_ptr, plan.col_idx, vals, oracle_matrix(oracle_port, I, J, V, E, False))
+    assert bits_equal(host(res), oracle_port.sparse_vec(Ri, Rv, E))
+    nu = rng.uniform(0.5, 2.0, len(T))
+    _, _, Vk = oracle_port.curl_curl(m, nu, qw, curl)
+    assert_csr_equal(plan.row_ptr, plan.col_idx, plan.stiffness(dev(nu)), oracle_matrix(oracle_port, I, J, Vk, E, False))
+    plan.check()
