@@ -4,6 +4,7 @@
 #include <cuda_runtime.h>
 
 #include <cstdint>
+#include <memory>
 #include <vector>
 
 #include "common.cuh"
@@ -41,6 +42,7 @@ struct BatchState {
     std::vector<int32_t *> owned;  // block_row128 arrays built for the batch
     BatchVariantData var[4];
     std::vector<TileComplexInput> tile_in;  // the meshes' tile plans (variants 4, 5)
+    std::vector<std::unique_ptr<TilePlan>> own_tiles;  // large-tile plans of small meshes, made for the batch
     TileComplexBatch tile;
 };
 

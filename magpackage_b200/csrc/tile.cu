@@ -85,9 +85,16 @@ __device__ __forceinline__ double qsum_equal(double u, int nq) {
 
 __device__ __forceinline__ void flag(int *err) { atomicOr(err, 1); }
 
+// A record plane is read once: it does not displace the coordinates, solution and tables in L1.
+__device__ __forceinline__ uint4 ld_record(const uint4 *p) {
+    uint4 v;
+    asm("ld.global.nc.L1::no_allocate.v4.u32 {%0, %1, %2, %3}, [%4];" : "=r"(v.x), "=r"(v.y), "=r"(v.z), "=r"(v.w) : "l"(p));
+    return v;
+}
+
 enum TileMode { kJacobian = 0, kStiffness = 1, kSeeded = 2, kHarmonicDc = 3 };
 
-// One element of the block: record i.
+// One element of the block: record i. Returns the element's id.
 //   kJacobian: residual and tangent at the element's state (assemble_jacobian_kernel_mex.cpp:92-131);
 //   kStiffness: K(nu) with the element's given nu (assemble_curl_curl_kernel_mex.cpp:94-101), no residual;
 //   kHarmonicDc: the harmonic-balance DC block, K(nu_dc) in that kernel's operation order
@@ -100,11 +107,11 @@ enum TileMode { kJacobian = 0, kStiffness = 1, kSeeded = 2, kHarmonicDc = 3 };
 // slot = 0 + v, the same value up to the sign of an exact zero, which the store phase
 // normalises (x + 0 turns -0 into +0 and leaves every other value unchanged).
 template <bool CALCJ, bool Q4, int MODE, bool FIRST = false>
-__device__ __forceinline__ void tile_element(const TileArgs &A, int64_t i, double *__restrict__ slot,
+__device__ __forceinline__ uint32_t tile_element(const TileArgs &A, int64_t i, double *__restrict__ slot,
                                              double2 *__restrict__ incv, int bnnz, int binc) {
     const int64_t n = A.nrec;
-    const uint4 p0 = __ldg(A.recs + i), p1 = __ldg(A.recs + n + i), p2 = __ldg(A.recs + 2 * n + i);
-    const uint4 p3 = __ldg(A.recs + 3 * n + i), p4 = __ldg(A.recs + 4 * n + i), p5 = __ldg(A.recs + 5 * n + i);
+    const uint4 p0 = ld_record(A.recs + i), p1 = ld_record(A.recs + n + i), p2 = ld_record(A.recs + 2 * n + i);
+    const uint4 p3 = ld_record(A.recs + 3 * n + i), p4 = ld_record(A.recs + 4 * n + i), p5 = ld_record(A.recs + 5 * n + i);
     const int4 tt = make_int4((int)p0.x, (int)p0.y, (int)p0.z, (int)p0.w);
     const unsigned sb = (p2.w >> 8) & 0x3Fu;
     const unsigned pos[6] = {p3.x, p3.y, p3.z, p3.w, p4.x, p4.y};
@@ -158,6 +165,9 @@ __device__ __forceinline__ void tile_element(const TileArgs &A, int64_t i, doubl
         }
     }
     const double adet = g.adet, w0 = A.qp.qw[0] * adet;
+    // A warp that holds both kinds of element takes one path, not one after the other.
+    const bool linear = g2 == 0.0;
+    const bool linear_warp = MODE == kJacobian && CALCJ ? __all_sync(__activemask(), linear) != 0 : true;
 #pragma unroll
     for (int l = 0; l < 6; l++) {
         const unsigned s = sl[l];
@@ -185,13 +195,16 @@ __device__ __forceinline__ void tile_element(const TileArgs &A, int64_t i, doubl
 #pragma unroll
                 for (int j = 0; j < 6; j++)
                     v[j] = qsum4<Q4>(nut * dot3(C[l], C[j]) + gl * (be * b[j]), A.qp, w0, adet);
-            } else if (g2 == 0.0) {
+            } else if (linear_warp) {
 #pragma unroll
                 for (int j = 0; j < 6; j++) v[j] = qsum4<Q4>(nu * dot3(C[l], C[j]), A.qp, w0, adet);
-            } else {
+            } else {  // a linear element's second term is +0 (adding it changes at most the sign of a zero)
                 const double gl = g2 * b[l];
 #pragma unroll
-                for (int j = 0; j < 6; j++) v[j] = qsum4<Q4>(nu * dot3(C[l], C[j]) + gl * b[j], A.qp, w0, adet);
+                for (int j = 0; j < 6; j++) {
+                    const double t = linear ? 0.0 : gl * b[j];
+                    v[j] = qsum4<Q4>(nu * dot3(C[l], C[j]) + t, A.qp, w0, adet);
+                }
             }
             dv = v[l];
 #pragma unroll
@@ -208,6 +221,7 @@ __device__ __forceinline__ void tile_element(const TileArgs &A, int64_t i, doubl
             flag(A.err);
         }
     }
+    return p2.z;
 }
 
 // L2 prefetch of [p, p + bytes) (16-byte aligned start and length; the plan's arrays are
@@ -355,10 +369,10 @@ __device__ __forceinline__ void tile_mass_element(const TileArgs &A, const doubl
                                                   double *__restrict__ slot, double2 *__restrict__ incv, int bnnz,
                                                   int binc, const double *__restrict__ sval) {
     const int64_t n = A.nrec;
-    const uint4 p2 = __ldg(A.recs + 2 * n + i);
+    const uint4 p2 = ld_record(A.recs + 2 * n + i);
     const double sigma = sigma_e ? __ldg(sigma_e + p2.z) : 1.0;
     if (!(fabs(sigma) > 1e-12)) return;
-    const uint4 p0 = __ldg(A.recs + i);
+    const uint4 p0 = ld_record(A.recs + i);
     const int4 tt = make_int4((int)p0.x, (int)p0.y, (int)p0.z, (int)p0.w);
     const unsigned sb = (p2.w >> 8) & 0x3Fu;
     double M[21];  // row by row from the diagonal
@@ -388,7 +402,7 @@ __device__ __forceinline__ void tile_mass_element(const TileArgs &A, const doubl
                 for (int j = l; j < 6; j++, k++) M[k] = M[k] + dot3(N[l], N[j]) * sigma * w;
         }
     }
-    const uint4 p3 = __ldg(A.recs + 3 * n + i), p4 = __ldg(A.recs + 4 * n + i), p5 = __ldg(A.recs + 5 * n + i);
+    const uint4 p3 = ld_record(A.recs + 3 * n + i), p4 = ld_record(A.recs + 4 * n + i), p5 = ld_record(A.recs + 5 * n + i);
     const unsigned pos[6] = {p3.x, p3.y, p3.z, p3.w, p4.x, p4.y};
     const unsigned sl[6] = {p4.z, p4.w, p5.x, p5.y, p5.z, p5.w};
 #pragma unroll
@@ -480,12 +494,9 @@ __global__ void __launch_bounds__(BT, MINB)
         const int c1 = Bp->col_end[c];
         for (int i = c0 + tid; i < c1; i += BT) {
             const int64_t r = (int64_t)rec0 + i;
-            if (c == 0) tile_element<true, Q4, kStiffness, true>(A, r, slot, incv, nnz, ninc);
-            else tile_element<true, Q4, kStiffness>(A, r, slot, incv, nnz, ninc);
-            if (!conducting) {
-                const double sg = I.sigma ? __ldg(I.sigma + __ldg(A.recs + 2 * A.nrec + r).z) : 1.0;
-                conducting = fabs(sg) > 1e-12;
-            }
+            const uint32_t e = c == 0 ? tile_element<true, Q4, kStiffness, true>(A, r, slot, incv, nnz, ninc)
+                                      : tile_element<true, Q4, kStiffness>(A, r, slot, incv, nnz, ninc);
+            if (!conducting) conducting = fabs(I.sigma ? __ldg(I.sigma + e) : 1.0) > 1e-12;
         }
         c0 = c1;
         if (c + 1 == ncolors) {
@@ -602,14 +613,15 @@ constexpr int kMassBT = 256;
 
 // M(sigma) of one mesh, one CTA per block. 613,000 elements, a tenth of them conducting: 295 us
 // with element blocks through HBM scratch and row sums, 60 us here.
-__global__ void __launch_bounds__(kMassBT, 2)
+template <int BT, int MINB>
+__global__ void __launch_bounds__(BT, MINB)
     k_tile_mass(TileArgs A, const double *__restrict__ sigma, const double *__restrict__ val_ref, int nblocks, int ahead) {
     extern __shared__ __align__(16) double tile_smem[];
     const TileSmem S = tile_smem_layout(tile_smem, A.smem_nnz, A.smem_inc, A.smem_rows, A.smem_chunks);
     const int blk = blockIdx.x;
     if (threadIdx.x == 0 && blk + ahead < nblocks) prefetch_block(A, blk + ahead);
     double *vals = A.vals;
-    tile_mass_block<kMassBT>(A, S, A.blocks + blk, sigma, val_ref, [&](int64_t k, double v) { vals[k] = v; });
+    tile_mass_block<BT>(A, S, A.blocks + blk, sigma, val_ref, [&](int64_t k, double v) { vals[k] = v; });
 }
 
 // The imaginary parts omega * M of the listed items (list[0] of them), resident CTAs striding.
@@ -634,6 +646,9 @@ __global__ void __launch_bounds__(kMassBT, 2)
 // colour phase runs in one pass (256 threads left a second pass with one warp busy).
 constexpr int kTileBT = 320;
 constexpr int kTileMinB = 2;
+// Small tiles (4x2x2 or 3x3x3 layers): a colour class holds 90 to 135 elements.
+constexpr int kSmallBT = 160;
+constexpr int kSmallMinB = 3;
 
 }  // namespace
 
@@ -663,8 +678,8 @@ int resident_ctas(const void *kern, int threads, size_t smem, int *out) {
     return MAG_OK;
 }
 
-template <bool CALCJ, bool Q4, int MODE, int BT = kTileBT, int MINB = kTileMinB>
-int launch(const TileArgs &a, const TilePlan &tp, size_t smem, cudaStream_t s) {
+template <bool CALCJ, bool Q4, int MODE, int BT, int MINB>
+int launch_shape(const TileArgs &a, const TilePlan &tp, size_t smem, cudaStream_t s) {
     auto kern = k_tile<BT, MINB, CALCJ, Q4, MODE>;
     int resident = 0;
     MAG_TRY(resident_ctas((const void *)kern, BT, smem, &resident));
@@ -672,6 +687,13 @@ int launch(const TileArgs &a, const TilePlan &tp, size_t smem, cudaStream_t s) {
     const int ahead = tp.prefetch_waves > 0 ? resident * tp.prefetch_waves : tp.nblocks;
     kern<<<tp.nblocks, BT, smem, s>>>(a, tp.nblocks, ahead);
     return cudaPeekAtLastError() == cudaSuccess ? MAG_OK : MAG_E_CUDA;
+}
+
+// The shape of the plan's tiles.
+template <bool CALCJ, bool Q4, int MODE>
+int launch(const TileArgs &a, const TilePlan &tp, size_t smem, cudaStream_t s) {
+    return tp.small_tiles ? launch_shape<CALCJ, Q4, MODE, kSmallBT, kSmallMinB>(a, tp, smem, s)
+                          : launch_shape<CALCJ, Q4, MODE, kTileBT, kTileMinB>(a, tp, smem, s);
 }
 
 TileArgs make_args(const TilePlan &tp, const ElemData &m, const QuadParams &qp, int *err) {
@@ -704,9 +726,9 @@ int launch_tile_jacobian(const TilePlan &tp, const ElemData &m, const double *so
     const bool q4 = qp.nq == 4 && qp.uniform_w;
     if (calc_j && q4) {  // the launch shape of the Newton Jacobian (threads per CTA x CTAs per SM)
         switch (tp.variant) {
-            case 1: return launch<true, true, kJacobian, 288, 2>(a, tp, smem, s);
-            case 2: return launch<true, true, kJacobian, 256, 2>(a, tp, smem, s);
-            case 3: return launch<true, true, kJacobian, 512, 1>(a, tp, smem, s);
+            case 1: return launch_shape<true, true, kJacobian, 288, 2>(a, tp, smem, s);
+            case 2: return launch_shape<true, true, kJacobian, 256, 2>(a, tp, smem, s);
+            case 3: return launch_shape<true, true, kJacobian, 512, 1>(a, tp, smem, s);
             default: return launch<true, true, kJacobian>(a, tp, smem, s);
         }
     }
@@ -715,7 +737,7 @@ int launch_tile_jacobian(const TilePlan &tp, const ElemData &m, const double *so
 }
 
 const char *tile_variant_name(int v) {
-    static const char *names[kTileVariants] = {"320 threads x 2 CTAs/SM", "288 threads x 2 CTAs/SM",
+    static const char *names[kTileVariants] = {"320 threads x 2 CTAs/SM (small tiles: 160 x 3)", "288 threads x 2 CTAs/SM",
                                                "256 threads x 2 CTAs/SM", "512 threads x 1 CTA/SM"};
     return v >= 0 && v < kTileVariants ? names[v] : "";
 }
@@ -739,10 +761,12 @@ int launch_tile_mass(const TilePlan &tp, const ElemData &m, const double *sigma,
     a.vals = vals;
     a.nnz_total = tp.nnz;
     const size_t smem = tile_smem_bytes(tp, &a) + (size_t)18 * qp.nq * sizeof(double);
+    const auto kern = tp.small_tiles ? k_tile_mass<kSmallBT, kSmallMinB> : k_tile_mass<kMassBT, 2>;
+    const int threads = tp.small_tiles ? kSmallBT : kMassBT;
     int resident = 0;
-    MAG_TRY(resident_ctas((const void *)k_tile_mass, kMassBT, smem, &resident));
+    MAG_TRY(resident_ctas((const void *)kern, threads, smem, &resident));
     const int ahead = tp.prefetch_waves > 0 ? resident * tp.prefetch_waves : tp.nblocks;
-    k_tile_mass<<<tp.nblocks, kMassBT, smem, s>>>(a, sigma, qp.val_ref, tp.nblocks, ahead);
+    kern<<<tp.nblocks, threads, smem, s>>>(a, sigma, qp.val_ref, tp.nblocks, ahead);
     return cudaPeekAtLastError() == cudaSuccess ? MAG_OK : MAG_E_CUDA;
 }
 
@@ -820,24 +844,18 @@ int build_tile_complex(const std::vector<TileComplexInput> &in, TileComplexBatch
     b->smem = (size_t)b->smem_nnz * sizeof(double) + (size_t)b->smem_inc * sizeof(double2) +
               (size_t)(b->smem_rows + b->smem_chunks) * sizeof(uint2);
     b->smem_mass = b->smem + (size_t)18 * kMaxQuad * sizeof(double);
-    for (int v = 0; v <= kTileComplexVariants; v++) {  // the last one: the mass kernel
-        const bool mass = v == kTileComplexVariants;
-        const void *kern = mass ? (const void *)k_tile_complex_mass : (const void *)complex_kernel(v, q4 != 0);
-        if (resident_ctas(kern, mass ? kMassBT : kComplexThreads[v], mass ? b->smem_mass : b->smem,
-                          mass ? &b->mass_ctas : &b->ahead[v]) != MAG_OK) {
-            cudaGetLastError();
-            *b = TileComplexBatch{};
-            return MAG_OK;  // the blocks do not fit: the other batch variants remain
-        }
-    }
-    if (b->mass_ctas > (int)items.size()) b->mass_ctas = (int)items.size();
-    if (cudaMalloc(&b->inst, hi.size() * sizeof(TileComplexInstance)) != cudaSuccess ||
+    bool fits = resident_ctas((const void *)k_tile_complex_mass, kMassBT, b->smem_mass, &b->mass_ctas) == MAG_OK;
+    for (int v = 0; v < kTileComplexVariants; v++)
+        fits = fits && resident_ctas((const void *)complex_kernel(v, q4 != 0), kComplexThreads[v], b->smem,
+                                     &b->ahead[v]) == MAG_OK;
+    if (!fits || cudaMalloc(&b->inst, hi.size() * sizeof(TileComplexInstance)) != cudaSuccess ||
         cudaMalloc(&b->items, items.size() * sizeof(int2)) != cudaSuccess ||
         cudaMalloc(&b->list, (items.size() + 1) * sizeof(int)) != cudaSuccess) {
         cudaGetLastError();
         free_tile_complex(b);
-        return MAG_OK;
+        return MAG_OK;  // the blocks do not fit: the other batch variants remain
     }
+    b->mass_ctas = std::min(b->mass_ctas, (int)items.size());
     MAG_CUDA_TRY(cudaMemcpyAsync(b->inst, hi.data(), hi.size() * sizeof(TileComplexInstance), cudaMemcpyHostToDevice, s));
     MAG_CUDA_TRY(cudaMemcpyAsync(b->items, items.data(), items.size() * sizeof(int2), cudaMemcpyHostToDevice, s));
     MAG_CUDA_TRY(cudaStreamSynchronize(s));
@@ -848,13 +866,12 @@ int build_tile_complex(const std::vector<TileComplexInput> &in, TileComplexBatch
 
 int launch_tile_complex(const TileComplexBatch &b, int variant, cudaStream_t s) {
     if (!b.ok || variant < 0 || variant >= kTileComplexVariants) return MAG_E_UNSUPPORTED;
-    const ComplexKernel kern = complex_kernel(variant, b.q4 != 0);
     const TileComplexInstance *inst = static_cast<const TileComplexInstance *>(b.inst);
     if (cudaMemsetAsync(b.list, 0, sizeof(int), s) != cudaSuccess) return MAG_E_CUDA;
-    kern<<<b.nitems, kComplexThreads[variant], b.smem, s>>>(inst, b.items, b.nitems, b.ahead[variant], b.smem_nnz,
-                                                           b.smem_inc, b.smem_rows, b.smem_chunks, b.list);
-    k_tile_complex_mass<<<b.mass_ctas, kMassBT, b.smem_mass, s>>>(inst, b.items, b.smem_nnz, b.smem_inc, b.smem_rows,
-                                                                 b.smem_chunks, b.list);
+    complex_kernel(variant, b.q4 != 0)<<<b.nitems, kComplexThreads[variant], b.smem, s>>>(
+        inst, b.items, b.nitems, b.ahead[variant], b.smem_nnz, b.smem_inc, b.smem_rows, b.smem_chunks, b.list);
+    k_tile_complex_mass<<<b.mass_ctas, kMassBT, b.smem_mass, s>>>(
+        inst, b.items, b.smem_nnz, b.smem_inc, b.smem_rows, b.smem_chunks, b.list);
     return cudaPeekAtLastError() == cudaSuccess ? MAG_OK : MAG_E_CUDA;
 }
 

@@ -59,6 +59,7 @@ struct TilePlan {
     double build_ms = 0.0;
     int64_t bytes = 0;
     int ok = 0;
+    int small_tiles = 0;  // tiles of fewer than 4 x 4 x 4 node layers: launched with 160 threads x 3 CTAs/SM
     int variant = 0;  // launch shape of the Newton Jacobian (0 .. kTileVariants-1)
     int prefetch_waves = 1;  // staging depth: a CTA prefetches the block this many waves ahead (0: none)
 };
@@ -80,7 +81,9 @@ struct TilePlanInput {
 // Leaves plan->ok = 0 (and returns MAG_OK) when the mesh does not suit the schedule:
 // wide rows (> 31 entries), an off-diagonal entry with more than two contributions
 // (repeated dofs), or a block needing more than kTileMaxColors colours.
-int build_tile_plan(const TilePlanInput &in, void *work, size_t work_bytes, TilePlan *plan, cudaStream_t s);
+// large: 4 x 4 x 4 tiles whatever the mesh's size.
+int build_tile_plan(const TilePlanInput &in, void *work, size_t work_bytes, TilePlan *plan, cudaStream_t s,
+                    bool large = false);
 void free_tile_plan(TilePlan *plan);
 
 // Jacobian (calc_j) and residual; vals may be NULL when !calc_j.
@@ -113,12 +116,12 @@ constexpr int kTileComplexVariants = 2;
 struct TileComplexBatch {
     void *inst = nullptr;   // device array of the per-mesh launch arguments
     int2 *items = nullptr;  // device (mesh, block), larger meshes first
+    int *list = nullptr;    // device: count and items with a conducting element, of the running launch
     int nitems = 0, q4 = 0;
     int smem_nnz = 0, smem_inc = 0, smem_rows = 0, smem_chunks = 0;
-    int *list = nullptr;    // device: count and items with a conducting element, of the running launch
     size_t smem = 0, smem_mass = 0;
-    int ahead[kTileComplexVariants] = {0, 0};  // CTAs resident at once per launch shape
-    int mass_ctas = 0;                         // of the mass kernel
+    int ahead[kTileComplexVariants] = {};  // CTAs resident at once per launch shape
+    int mass_ctas = 0;                     // of the mass kernel
     int ok = 0;
 };
 

@@ -20,6 +20,7 @@
 #include <algorithm>
 #include <chrono>
 #include <cmath>
+#include <cstdint>
 #include <cstring>
 #include <vector>
 
@@ -32,7 +33,18 @@ namespace {
 
 constexpr int kPB = 256;         // threads of the per-block kernels
 constexpr int kLayerB = 1024;    // threads of the layer walk
-constexpr int kTileLayers = 4;   // node layers per tile and axis
+// Node layers per tile: the first of these forms whose tiles are few enough, the last one
+// otherwise. A block's time is latency: where blocks would leave SMs idle (148 on the GPU),
+// smaller ones finish sooner although they evaluate more elements twice (4x2x2 up to 1.9 times an
+// element, 3x3x3 1.67, 4x4x4 1.5). Measured on the device alone, us, with 4x4x4 / as chosen here:
+// Jacobian at 8^3 hexahedra (4x2x2) 14.9 / 10.3, 14^3 (3x3x3) 15.5 / 11.4, 16^3 15.7 / 12.5; M(1)
+// 18.6 / 10.5, 18.8 / 13.0, 19.0 / 14.9; at 20^3, where 4x4x4 stays, 3x3x3 has Jacobian 14.5
+// against 16.3 but at 24^3 23.3 against 20.0.
+struct TileForm {
+    int l[3];
+    int64_t most;
+};
+constexpr TileForm kTileForms[] = {{{4, 2, 2}, 148}, {{3, 3, 3}, 2 * 148}, {{4, 4, 4}, INT64_MAX}};
 constexpr uint32_t kNone16 = 0xFFFFu;
 
 unsigned grid1(int64_t n, int b = 256) { return (unsigned)((n + b - 1) / b); }
@@ -157,6 +169,7 @@ __global__ void __launch_bounds__(kLayerB) k_layers(const double *__restrict__ s
 
 struct TileGrid {
     int n[3];  // tiles per axis
+    int l[3];  // node layers per tile
 };
 
 __device__ __forceinline__ int layer_of(const double *__restrict__ thr, int n, double x) {
@@ -177,7 +190,7 @@ __global__ void k_node_tiles(const double4 *__restrict__ xyz, int64_t nn, const 
     const double v[3] = {p.x, p.y, p.z};
     int t[3];
 #pragma unroll
-    for (int a = 0; a < 3; a++) t[a] = layer_of(thr + a * nn, info->last_layer[a], v[a]) / kTileLayers;
+    for (int a = 0; a < 3; a++) t[a] = layer_of(thr + a * nn, info->last_layer[a], v[a]) / g.l[a];
     tile[i] = (uint32_t)(t[0] + g.n[0] * (t[1] + g.n[1] * t[2]));
 }
 
@@ -650,7 +663,7 @@ struct CubTemp {
         if (!arena.get(&ptr, n)) return MAG_E_NOMEM; \
     } while (0)
 
-int build(const TilePlanInput &in, void *work, size_t work_bytes, TilePlan *p, cudaStream_t s) {
+int build(const TilePlanInput &in, void *work, size_t work_bytes, bool large, TilePlan *p, cudaStream_t s) {
     Arena arena(work, work_bytes, s);
     CubTemp temp;
     const int64_t nn = in.nn, ne = in.ne, ndof = in.ndof, ninc = in.ninc;
@@ -680,10 +693,17 @@ int build(const TilePlanInput &in, void *work, size_t work_bytes, TilePlan *p, c
     if (hi.fail) return MAG_OK;
     TileGrid g;
     int64_t tiles = 1;
-    for (int a = 0; a < 3; a++) {
-        g.n[a] = hi.last_layer[a] / kTileLayers + 1;
-        tiles *= g.n[a];
-        if (tiles >= (int64_t(1) << 31)) return MAG_OK;
+    for (const TileForm &f : kTileForms) {
+        if (large && f.most < INT64_MAX) continue;
+        tiles = 1;
+        for (int a = 0; a < 3; a++) {
+            g.l[a] = f.l[a];
+            g.n[a] = hi.last_layer[a] / f.l[a] + 1;
+            tiles *= g.n[a];
+            if (tiles >= (int64_t(1) << 31)) return MAG_OK;
+        }
+        p->small_tiles = f.most < INT64_MAX ? 1 : 0;
+        if (tiles <= f.most) break;
     }
     uint32_t *node_tile = nullptr, *tile = nullptr, *tile_s = nullptr, *row = nullptr, *order = nullptr;
     int *last = nullptr, *pn = nullptr, *pi = nullptr;
@@ -789,12 +809,12 @@ void free_tile_plan(TilePlan *p) {
     *p = TilePlan{};
 }
 
-int build_tile_plan(const TilePlanInput &in, void *work, size_t work_bytes, TilePlan *plan, cudaStream_t s) {
+int build_tile_plan(const TilePlanInput &in, void *work, size_t work_bytes, TilePlan *plan, cudaStream_t s, bool large) {
     *plan = TilePlan{};
     if (in.wide || in.ne <= 0 || in.ndof <= 0 || in.nn <= 0 || in.nnz >= (int64_t(1) << 32)) return MAG_OK;
     const auto t0 = std::chrono::steady_clock::now();
     TilePlan p;
-    const int rc = build(in, work, work_bytes, &p, s);
+    const int rc = build(in, work, work_bytes, large, &p, s);
     if (rc != MAG_OK || !p.ok) {
         free_tile_plan(&p);
         if (rc != MAG_E_NOMEM) return rc;
