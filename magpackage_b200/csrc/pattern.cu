@@ -5,6 +5,7 @@
 // Sorting uses CUB's stable radix sort (header library shipped with the CUDA
 // toolkit). Stability is what makes every row's incidence list come out in
 // ascending element order, which fixes the summation order of the assembly.
+#include <cub/block/block_scan.cuh>
 #include <cub/device/device_radix_sort.cuh>
 #include <cub/device/device_reduce.cuh>
 #include <cub/device/device_scan.cuh>
@@ -168,30 +169,94 @@ __global__ void k_rows(const int32_t *__restrict__ dofs, const int32_t *__restri
 }
 
 // ---- zero dropping --------------------------------------------------------
+//
+// Three launches: the rows' counts and their sums within a CTA, the sums of the CTAs, the entries
+// to their places. A warp takes kDropAhead rows at a time, a lane per entry (rows of a Nedelec
+// matrix have 13 to 19, so a row is one coalesced load and its rank one vote), steps such groups
+// one after another. One thread per row walking its entries took 6.3 us to count and 10.4 us to
+// copy at 28,000 rows (460,000 entries), with a device-wide scan of 7.7 us between them: 6.2, 7.6
+// and 5.6 us here. The call, with its copy back, at 60^3 hexahedra (25 M entries): 565 to 350 us.
+constexpr int kDropThreads = 256;
+constexpr int kDropAhead = 4;
+constexpr int kDropStep = kDropThreads / 32 * kDropAhead;  // rows of a CTA's step
+constexpr int kDropMaxSteps = kDropThreads / kDropStep;    // at most a row per thread
+// Many rows: more of them per CTA, so that the sums of the CTAs (one CTA adds them) stay few.
+inline int drop_steps(int64_t nrows) { return nrows < 200000 ? 1 : kDropMaxSteps; }
 
-__global__ void k_count_nonzero(const int64_t *__restrict__ rp, const double *__restrict__ v,
-                                int64_t nrows, int64_t *__restrict__ cnt) {
-    int64_t r = blockIdx.x * (int64_t)blockDim.x + threadIdx.x;
-    if (r >= nrows) return;
-    int64_t c = 0;
-    for (int64_t t = rp[r]; t < rp[r + 1]; t++) c += (v[t] != 0.0);
-    cnt[r] = c;
+// COPY false: rp_out[r + 1] = nonzeros of the CTA's rows up to r. (The last of them is the CTA's
+// total, at the place of the next CTA's start: k_drop_scan turns these into the starts.)
+// COPY true: the start of the CTA's first row is final; the others' are added up, and the rows'
+// nonzeros go to their places.
+template <bool COPY>
+__global__ void __launch_bounds__(kDropThreads) k_drop(const int64_t *__restrict__ rp, const int32_t *__restrict__ ci,
+                                                       const double *__restrict__ v, int64_t nrows, int steps,
+                                                       int64_t *__restrict__ rp_out, int32_t *__restrict__ ci_out,
+                                                       double *__restrict__ v_out) {
+    using Scan = cub::BlockScan<int, kDropThreads>;
+    __shared__ typename Scan::TempStorage tmp;
+    __shared__ int cnt[kDropThreads];
+    const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
+    const int64_t r0 = blockIdx.x * (int64_t)steps * kDropStep;
+    const int64_t off = COPY ? rp_out[r0] : 0;
+    for (int st = 0; st < steps; st++) {
+        const int i0 = st * kDropStep + warp * kDropAhead;  // row of the CTA
+        int64_t a[kDropAhead], b[kDropAhead], o[kDropAhead];
+        double x[kDropAhead];
+        int c[kDropAhead];
+#pragma unroll
+        for (int u = 0; u < kDropAhead; u++) {
+            const int64_t r = r0 + i0 + u;
+            a[u] = r < nrows ? rp[r] : 0;
+            b[u] = r < nrows ? rp[r + 1] : 0;
+            o[u] = COPY && r < nrows ? (r == r0 ? 0 : rp_out[r]) + off : 0;
+        }
+#pragma unroll
+        for (int u = 0; u < kDropAhead; u++) {
+            x[u] = a[u] + lane < b[u] ? v[a[u] + lane] : 0.0;
+            c[u] = COPY && a[u] + lane < b[u] ? ci[a[u] + lane] : 0;
+        }
+#pragma unroll
+        for (int u = 0; u < kDropAhead; u++) {
+            int n = 0;
+            for (int64_t k = a[u];;) {  // one pass unless the row has more than 32 entries
+                const unsigned m = __ballot_sync(0xffffffffu, x[u] != 0.0);
+                if (COPY && x[u] != 0.0) {
+                    const int64_t d = o[u] + n + __popc(m & ((1u << lane) - 1u));
+                    ci_out[d] = c[u];
+                    v_out[d] = x[u];
+                }
+                n += __popc(m);
+                k += 32;
+                if (k >= b[u]) break;
+                x[u] = k + lane < b[u] ? v[k + lane] : 0.0;
+                if (COPY) c[u] = k + lane < b[u] ? ci[k + lane] : 0;
+            }
+            if (!COPY && lane == 0) cnt[i0 + u] = n;
+            if (COPY && lane == 0 && i0 + u > 0 && r0 + i0 + u < nrows) rp_out[r0 + i0 + u] = o[u];
+        }
+    }
+    if (!COPY) {
+        __syncthreads();
+        const bool mine = (int)threadIdx.x < steps * kDropStep;
+        int upto;
+        Scan(tmp).InclusiveSum(mine ? cnt[threadIdx.x] : 0, upto);
+        if (mine && r0 + threadIdx.x < nrows) rp_out[r0 + threadIdx.x + 1] = upto;
+        if (blockIdx.x == 0 && threadIdx.x == 0) rp_out[0] = 0;
+    }
 }
 
-__global__ void k_compact(const int64_t *__restrict__ rp, const int32_t *__restrict__ ci,
-                          const double *__restrict__ v, int64_t nrows,
-                          const int64_t *__restrict__ rp_out, int32_t *__restrict__ ci_out,
-                          double *__restrict__ v_out) {
-    int64_t r = blockIdx.x * (int64_t)blockDim.x + threadIdx.x;
-    if (r >= nrows) return;
-    int64_t o = rp_out[r];
-    for (int64_t t = rp[r]; t < rp[r + 1]; t++) {
-        double x = v[t];
-        if (x != 0.0) {
-            ci_out[o] = ci[t];
-            v_out[o] = x;
-            o++;
-        }
+// The totals of the nb CTAs of `rows` rows, at the starts of their successors, summed in place.
+__global__ void __launch_bounds__(1024) k_drop_scan(int64_t *__restrict__ rp_out, int64_t nb, int64_t rows, int64_t nrows) {
+    using Scan = cub::BlockScan<int64_t, 1024>;
+    __shared__ typename Scan::TempStorage tmp;
+    int64_t carry = 0;
+    for (int64_t i0 = 0; i0 < nb; i0 += 1024) {
+        const int64_t i = i0 + threadIdx.x, at = (i + 1) * rows < nrows ? (i + 1) * rows : nrows;
+        int64_t x = i < nb ? rp_out[at] : 0, sum;
+        Scan(tmp).InclusiveSum(x, x, sum);
+        if (i < nb) rp_out[at] = carry + x;
+        carry += sum;
+        __syncthreads();
     }
 }
 
@@ -373,16 +438,11 @@ int csr_drop_zeros(const int64_t *rp, const int32_t *ci, const double *v, int64_
         set_error("csr_drop_zeros: bad arguments");
         return MAG_E_ARG;
     }
-    DevBuf cnt(s), tmp(s);
-    MAG_CUDA_TRY(cnt.alloc((nrows + 1) * 8));
-    MAG_CUDA_TRY(cudaMemsetAsync(cnt.p, 0, (nrows + 1) * 8, s));
-    k_count_nonzero<<<grid_for(nrows), kBlock, 0, s>>>(rp, v, nrows, cnt.as<int64_t>());
-    size_t tb = 0;
-    cub::DeviceScan::ExclusiveSum(nullptr, tb, cnt.as<int64_t>(), rp_out, (int64_t)nrows + 1, s);
-    MAG_CUDA_TRY(tmp.alloc(tb));
-    MAG_CUDA_TRY(cub::DeviceScan::ExclusiveSum(tmp.p, tb, cnt.as<int64_t>(), rp_out,
-                                               (int64_t)nrows + 1, s));
-    k_compact<<<grid_for(nrows), kBlock, 0, s>>>(rp, ci, v, nrows, rp_out, ci_out, v_out);
+    const int steps = drop_steps(nrows), rows = steps * kDropStep;
+    const int64_t nb = (nrows + rows - 1) / rows;
+    k_drop<false><<<(unsigned)nb, kDropThreads, 0, s>>>(rp, ci, v, nrows, steps, rp_out, nullptr, nullptr);
+    k_drop_scan<<<1, 1024, 0, s>>>(rp_out, nb, rows, nrows);
+    k_drop<true><<<(unsigned)nb, kDropThreads, 0, s>>>(rp, ci, v, nrows, steps, rp_out, ci_out, v_out);
     MAG_CUDA_TRY(cudaGetLastError());
     MAG_CUDA_TRY(cudaMemcpyAsync(nnz_out, rp_out + nrows, 8, cudaMemcpyDeviceToHost, s));
     MAG_CUDA_TRY(cudaStreamSynchronize(s));

@@ -824,3 +824,33 @@ def test_tile_plan_forms(oracle_port, form):
     _, _, Vk = oracle_port.curl_curl(m, nu, qw, curl)
     assert_csr_equal(plan.row_ptr, plan.col_idx, plan.stiffness(dev(nu)), oracle_matrix(oracle_port, I, J, Vk, E, False))
     plan.check()
+
+
+@pytest.mark.parametrize("nrows,longest,zeros", [(1, 3, 0.0), (31, 20, 1.0), (32, 33, 0.3), (33, 255, 0.5), (1000, 19, 0.1),
+                                                 (200001, 7, 0.4), (262145, 40, 0.05)])
+def test_drop_zeros_of_any_csr(nrows, longest, zeros):
+    """mag_csr_drop_zeros on random CSRs: empty rows, rows longer than a warp, a row count that does
+    and does not fill a CTA, no and only zeros (of both signs), NaN and infinities kept."""
+    rng = np.random.default_rng(nrows)
+    n = rng.integers(0, longest + 1, nrows)
+    n[0] = longest
+    rp = np.r_[0, np.cumsum(n)]
+    ci = rng.integers(0, 1 << 30, rp[-1]).astype(np.int32)
+    v = rng.normal(size=rp[-1])
+    v[rng.random(rp[-1]) < zeros] = 0.0
+    v[rng.random(rp[-1]) < 0.5 * zeros] *= -0.0
+    if zeros < 1.0:
+        v[: 3] = [np.nan, np.inf, -np.inf]
+    keep = v != 0.0
+    want_rp = np.r_[0, np.cumsum(keep)][rp]
+    L = _lib.lib()
+    d_rp, d_ci, d_v = dev(rp, torch.int64), dev(ci, torch.int32), dev(v)
+    o_rp, o_ci, o_v = torch.empty_like(d_rp), torch.empty_like(d_ci), torch.empty_like(d_v)
+    nnz = C.c_int64(-1)
+    ptr = lambda t: C.c_void_p(t.data_ptr())  # noqa: E731
+    _lib.check(L.mag_csr_drop_zeros(ptr(d_rp), ptr(d_ci), ptr(d_v), nrows, ptr(o_rp), ptr(o_ci), ptr(o_v), C.byref(nnz),
+                                    _lib.stream_ptr()))
+    assert nnz.value == keep.sum()
+    assert np.array_equal(host(o_rp), want_rp)
+    assert np.array_equal(host(o_ci)[: nnz.value], ci[keep])
+    assert np.array_equal(host(o_v)[: nnz.value].view(np.int64), v[keep].view(np.int64))
