@@ -194,33 +194,47 @@ class Assembler:
     def _dev(self, a):
         return torch.as_tensor(np.ascontiguousarray(a, dtype=np.float64), device="cuda")
 
+    def _by_tag(self, table) -> torch.Tensor:
+        """table[tag] of every element: the small table is copied, the elements stay on the device.
+        The tags are the plan's, which were checked to lie in 1..255."""
+        return self._dev(table).index_select(0, self.plan.tags)
+
+    def _coefficients(self, map_or_array) -> torch.Tensor:
+        """expand_material_map on the device (a map's values, or one per element or tag)."""
+        if not isinstance(map_or_array, dict):
+            return self._dev(self.expand_material_map(map_or_array))
+        table = np.zeros(256)
+        for k, v in map_or_array.items():
+            if np.isscalar(v) and 0 < int(k) < 256:
+                table[int(k)] = v
+        return self._by_tag(table)
+
     # ---- Assembler.m surface --------------------------------------------------
     def assemble_stiffness(self, material_map) -> CSR:
-        nu = self._dev(self.expand_material_map(material_map))
-        return self._out(self.plan.stiffness(nu))
+        return self._out(self.plan.stiffness(self._coefficients(material_map)))
 
     def assemble_mass(self) -> CSR:
         return self._out(self.plan.mass(None))
 
     def assemble_mass_weighted(self, coeff_map) -> CSR:
-        sigma = self._dev(self.expand_material_map(coeff_map))
-        return self._out(self.plan.mass(sigma))
+        return self._out(self.plan.mass(self._coefficients(coeff_map)))
 
     def assemble_source(self, source_map) -> torch.Tensor:
         n = self.Mesh.num_elements
-        js = np.zeros((n, 3))
         if isinstance(source_map, dict):
+            table = np.zeros((256, 3))
             for k, v in source_map.items():
-                js[self.Mesh.RegionTags == int(k)] = np.asarray(v, dtype=np.float64).ravel()[:3]
+                if 0 < int(k) < 256:
+                    table[int(k)] = np.asarray(v, dtype=np.float64).ravel()[:3]
+            return self.plan.source(self._by_tag(table))
+        a = np.asarray(source_map, dtype=np.float64)
+        if a.size == 3:
+            js = self._dev(a.ravel()).expand(n, 3).contiguous()
+        elif a.shape == (n, 3):
+            js = self._dev(a)
         else:
-            a = np.asarray(source_map, dtype=np.float64)
-            if a.size == 3:
-                js[:] = a.ravel()
-            elif a.shape == (n, 3):
-                js = a
-            else:
-                raise ValueError("Source must be [3x1] or [Ne x 3].")
-        return self.plan.source(self._dev(js))
+            raise ValueError("Source must be [3x1] or [Ne x 3].")
+        return self.plan.source(js)
 
     def assemble_winding(self, winding) -> torch.Tensor:
         """Coil vector C [num_dofs] of one Winding (Turns / CrossSectionArea times its
