@@ -148,7 +148,7 @@ class Assembler:
         self.Mesh = mesh
         self.DofHandler = dof_handler
         self.matlab_storage = matlab_storage
-        self._plan = None
+        self._plan = self._plan_tags = None
 
     # ---- helpers -------------------------------------------------------------
     @property
@@ -157,6 +157,7 @@ class Assembler:
             if self.DofHandler.cell_dofs is None:
                 self.DofHandler.distribute_dofs()
             dofs, signs = self.DofHandler.pack_for_kernel()
+            self._plan_tags = self.Mesh.RegionTags.copy()
             self._plan = AssemblyPlan(self.Mesh.P, self.Mesh.T, dofs, self.DofHandler.NumGlobalDofs,
                                       self.Mesh.RegionTags, signs)
         return self._plan
@@ -194,20 +195,24 @@ class Assembler:
     def _dev(self, a):
         return torch.as_tensor(np.ascontiguousarray(a, dtype=np.float64), device="cuda")
 
-    def _by_tag(self, table) -> torch.Tensor:
-        """table[tag] of every element: the small table is copied, the elements stay on the device.
-        The tags are the plan's, which were checked to lie in 1..255."""
-        return self._dev(table).index_select(0, self.plan.tags)
+    def _by_tag(self, values, width=()):
+        """values[tag] of every element from a {tag: value} dict, 0 where a tag is not named: a small
+        table is copied and indexed by the plan's tags (in 1..255, checked when it was made). None if
+        the mesh's tags are no longer the plan's or a key is no possible tag."""
+        tags = self.plan.tags
+        if not all(0 <= k <= 255 for k in values) or not np.array_equal(self.Mesh.RegionTags, self._plan_tags):
+            return None
+        table = np.zeros((256,) + width)
+        for k, v in values.items():
+            table[k] = v
+        return self._dev(table).index_select(0, tags)
 
     def _coefficients(self, map_or_array) -> torch.Tensor:
-        """expand_material_map on the device (a map's values, or one per element or tag)."""
-        if not isinstance(map_or_array, dict):
-            return self._dev(self.expand_material_map(map_or_array))
-        table = np.zeros(256)
-        for k, v in map_or_array.items():
-            if np.isscalar(v) and 0 < int(k) < 256:
-                table[int(k)] = v
-        return self._by_tag(table)
+        """expand_material_map on the device."""
+        c = None
+        if isinstance(map_or_array, dict):
+            c = self._by_tag({int(k): v for k, v in map_or_array.items() if np.isscalar(v)})
+        return self._dev(self.expand_material_map(map_or_array)) if c is None else c
 
     # ---- Assembler.m surface --------------------------------------------------
     def assemble_stiffness(self, material_map) -> CSR:
@@ -222,18 +227,21 @@ class Assembler:
     def assemble_source(self, source_map) -> torch.Tensor:
         n = self.Mesh.num_elements
         if isinstance(source_map, dict):
-            table = np.zeros((256, 3))
-            for k, v in source_map.items():
-                if 0 < int(k) < 256:
-                    table[int(k)] = np.asarray(v, dtype=np.float64).ravel()[:3]
-            return self.plan.source(self._by_tag(table))
-        a = np.asarray(source_map, dtype=np.float64)
-        if a.size == 3:
-            js = self._dev(a.ravel()).expand(n, 3).contiguous()
-        elif a.shape == (n, 3):
-            js = self._dev(a)
+            values = {int(k): np.asarray(v, dtype=np.float64).ravel()[:3] for k, v in source_map.items()}
+            js = self._by_tag(values, (3,))
+            if js is None:
+                js = np.zeros((n, 3))
+                for k, v in values.items():
+                    js[self.Mesh.RegionTags == k] = v
+                js = self._dev(js)
         else:
-            raise ValueError("Source must be [3x1] or [Ne x 3].")
+            a = np.asarray(source_map, dtype=np.float64)
+            if a.size == 3:
+                js = self._dev(a.ravel()).expand(n, 3).contiguous()
+            elif a.shape == (n, 3):
+                js = self._dev(a)
+            else:
+                raise ValueError("Source must be [3x1] or [Ne x 3].")
         return self.plan.source(js)
 
     def assemble_winding(self, winding) -> torch.Tensor:

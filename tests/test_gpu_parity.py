@@ -854,3 +854,30 @@ def test_drop_zeros_of_any_csr(nrows, longest, zeros):
     assert np.array_equal(host(o_rp), want_rp)
     assert np.array_equal(host(o_ci)[: nnz.value], ci[keep])
     assert np.array_equal(host(o_v)[: nnz.value].view(np.int64), v[keep].view(np.int64))
+
+
+@pytest.mark.parametrize("form", ["map", "unknown_tags", "float_keys", "outside_keys", "retagged", "nonscalar"])
+def test_assembler_maps_equal_expanded_arrays(form):
+    """The device expansion of {tag: value} maps gives what expand_material_map gives, for maps that
+    leave tags out, name absent or impossible tags, and meshes whose tags change after the plan."""
+    mesh = synth.kuhn_box(5, 4, 6, seed=9)
+    tags = synth.cube_layout(mesh)
+    m = Mesh(mesh.P, mesh.T, tags)
+    dh = DofHandler(m)
+    dh.distribute_dofs()
+    asm = Assembler(m, dh, matlab_storage=False)
+    cmap = {"map": {1: 2.0, 2: 0.5, 3: 7.0}, "unknown_tags": {2: 0.5, 9: 3.0}, "float_keys": {1.0: 2.0, 3.0: 4.0},
+            "outside_keys": {1: 2.0, 300: 5.0, -4: 1.0}, "retagged": {1: 2.0, 7: 9.0},
+            "nonscalar": {1: 2.0, 2: [1.0, 2.0]}}[form]
+    smap = {int(k): (1.0 + int(k), -2.0, 0.5) for k in cmap}
+    asm.plan
+    if form == "retagged":
+        m.RegionTags[::3] = 7
+        m.RegionTags[1::7] = 400
+    want = asm.expand_material_map(cmap)
+    assert bits_equal(host(asm.assemble_stiffness(cmap).values), host(asm.plan.stiffness(dev(want))))
+    assert bits_equal(host(asm.assemble_mass_weighted(cmap).values), host(asm.plan.mass(dev(want))))
+    js = np.zeros((m.num_elements, 3))
+    for k, v in smap.items():
+        js[m.RegionTags == k] = v
+    assert bits_equal(host(asm.assemble_source(smap)), host(asm.plan.source(dev(js))))
