@@ -166,7 +166,10 @@ def sync(stream=None) -> None:
 
 
 def stream_ptr(stream=None):
+    """The stream's handle (None: the current stream of the current device). The current stream is
+    asked for its handle directly: a Stream object for it costs 3 us, a quarter of a small call."""
     import torch
 
-    s = stream if stream is not None else torch.cuda.current_stream()
-    return C.c_void_p(s.cuda_stream)
+    if stream is None:
+        return C.c_void_p(torch._C._cuda_getCurrentRawStream(torch.cuda.current_device()))
+    return C.c_void_p(stream.cuda_stream)
