@@ -450,19 +450,25 @@ __global__ void __launch_bounds__(kRows, 6) k_mlp_forward(MlpForwardArgs a) {
 // ---- backward --------------------------------------------------------------------
 //
 // 256 threads per 128-row tile: warp w serves rows 32 (w & 3) .. + 31 (the TMEM lanes it can
-// read), columns 32 (w >> 2) .. + 31. The weight gradients dW = dZ^T H (FP32 dZ, BF16-valued H)
-// are register-tiled outer products over the rows, 4 x 4 outputs a thread, summed in row order;
-// they run while the tensor core forms the next layer's dZ W. Measured at 32,768 rows: 130 us
-// with one thread per row and 32 outputs a thread read from shared memory one by one, 43 us here,
-// most of it the shared-memory reads of the outer products (8 words for 16 products).
+// read), columns 32 (w >> 2) .. + 31. The weight gradients dW = dZ^T H contract over the tile's
+// rows: dZ is FP32 and H has BF16 values, so dZ is split into three BF16 parts that add up to it
+// exactly (8 + 8 + 8 bits) and each part's products with H, which are exact, are summed by the
+// tensor cores in FP32. They run beside the tcgen05 MMA that forms the next layer's dZ W; these
+// operands lie row by row in shared memory, the transposed form mma.sync takes by ldmatrix
+// (16 x 32 outputs a warp). Bias and output gradients are sums over rows by a shuffle tree.
+// Measured at 32,768 rows: 130 us with one thread per row and 32 outputs a thread read from shared
+// memory one by one; 43 us as FP32 outer products, 4 x 4 outputs a thread (bound by 8 words of
+// shared memory per 16 products); 30 us so. The gradient then differs from the FP32 sums by 3e-7 in norm,
+// and its error against 64 bits (7e-3, the BF16 layer inputs) is the same.
 constexpr int kBwd = 256;
-constexpr int kLd = kH + 4;  // row stride of the FP32 tiles: a column's rows fall into different banks
+constexpr int kLd = kH + 8;  // row stride of the BF16 tiles: eight rows of an 8x8 matrix fall into different banks
 
 struct BwdSmem {
     Smem s;
-    alignas(16) float dz[kRows * kLd];   // current layer's dZ (FP32)
-    alignas(16) float hin[kRows * kLd];  // current layer's input (BF16-rounded, held as FP32)
-    float dy[kRows];
+    alignas(16) __nv_bfloat16 dz[3][kRows * kLd];  // current layer's dZ: leading, middle, trailing part
+    alignas(16) __nv_bfloat16 hin[kRows * kLd];    // current layer's input
+    float sum[4][kH];                              // column sums of the four groups of 32 rows
+    float dy[4];
 };
 
 // 32 consecutive pre-activations.
@@ -482,11 +488,6 @@ __device__ __forceinline__ void load_z32(const float *src, bool valid, bool vec,
     }
 }
 
-__device__ __forceinline__ void put32(float *dst, const float v[32]) {
-#pragma unroll
-    for (int i = 0; i < 32; i += 4) *reinterpret_cast<float4 *>(dst + i) = make_float4(v[i], v[i + 1], v[i + 2], v[i + 3]);
-}
-
 // 32 columns c0.. of one row as BF16 into a K=64 core-matrix image.
 __device__ __forceinline__ void put_bf16_32(__nv_bfloat16 *img, int row, int c0, const float v[32]) {
 #pragma unroll
@@ -498,46 +499,146 @@ __device__ __forceinline__ void put_bf16_32(__nv_bfloat16 *img, int row, int c0,
     }
 }
 
-// Sum over the tile's rows, in order, of column o of an FP32 tile.
-__device__ __forceinline__ float column_sum(const float *m, int o) {
-    float s = 0.0f;
-#pragma unroll 16
-    for (int r = 0; r < kRows; r++) s += m[r * kLd + o];
-    return s;
+// 32 BF16 values (bits) to a tile row.
+__device__ __forceinline__ void put_bits32(__nv_bfloat16 *dst, const uint32_t v[16]) {
+#pragma unroll
+    for (int i = 0; i < 16; i += 4) *reinterpret_cast<uint4 *>(dst + 2 * i) = make_uint4(v[i], v[i + 1], v[i + 2], v[i + 3]);
 }
 
-// gW[o][i] += sum_r dz[r][o] hin[r][i], gb[o] += sum_r dz[r][o] (64 x 64, row order).
-__device__ __forceinline__ void weight_grads(const BwdSmem &B, float *gW, float *gb, bool first) {
-    const int o0 = (threadIdx.x >> 4) * 4, i0 = (threadIdx.x & 15) * 4;
-    uint64_t acc[4][2];
+// The three parts of 32 FP32 values: each the leading 8 bits of what the parts before leave, so
+// that they add up exactly. Infinities and NaN stay in the leading part.
+__device__ __forceinline__ void put_split32(BwdSmem &B, int row, int c0, const float v[32]) {
+    float x[32];
 #pragma unroll
-    for (int k = 0; k < 4; k++) acc[k][0] = acc[k][1] = pk2(0.0f, 0.0f);
-#pragma unroll 4
-    for (int r = 0; r < kRows; r++) {
-        const float4 d = *reinterpret_cast<const float4 *>(B.dz + r * kLd + o0);
-        const ulonglong2 h = *reinterpret_cast<const ulonglong2 *>(B.hin + r * kLd + i0);
-        const uint64_t dd[4] = {pk2(d.x, d.x), pk2(d.y, d.y), pk2(d.z, d.z), pk2(d.w, d.w)};
+    for (int i = 0; i < 32; i++) x[i] = v[i];
 #pragma unroll
-        for (int k = 0; k < 4; k++) {
-            acc[k][0] = fma2(dd[k], h.x, acc[k][0]);
-            acc[k][1] = fma2(dd[k], h.y, acc[k][1]);
+    for (int k = 0; k < 3; k++) {
+        uint32_t w[16];
+#pragma unroll
+        for (int i = 0; i < 16; i++) {
+            const uint32_t a = __float_as_uint(x[2 * i]) & 0xFFFF0000u, b = __float_as_uint(x[2 * i + 1]) & 0xFFFF0000u;
+            w[i] = (a >> 16) | b;
+            x[2 * i] = (a & 0x7F800000u) == 0x7F800000u ? 0.0f : x[2 * i] - __uint_as_float(a);
+            x[2 * i + 1] = (b & 0x7F800000u) == 0x7F800000u ? 0.0f : x[2 * i + 1] - __uint_as_float(b);
+        }
+        put_bits32(B.dz[k] + row * kLd + c0, w);
+    }
+}
+
+// BF16 of 32 values to a tile row.
+__device__ __forceinline__ void put_input32(BwdSmem &B, int row, int c0, const float v[32]) {
+    uint32_t w[16];
+#pragma unroll
+    for (int i = 0; i < 16; i++) {
+        const __nv_bfloat162 t = __floats2bfloat162_rn(v[2 * i], v[2 * i + 1]);
+        w[i] = *reinterpret_cast<const uint32_t *>(&t);
+    }
+    put_bits32(B.hin + row * kLd + c0, w);
+}
+
+// Sums over a warp's 32 rows (lanes) of 32 columns: lane c gets column c's.
+__device__ __forceinline__ float warp_columns(const float v[32]) {
+    float x[16];
+    const int lane = threadIdx.x & 31;
+#pragma unroll
+    for (int i = 0; i < 16; i++) {
+        const float keep = lane & 16 ? v[i + 16] : v[i], send = lane & 16 ? v[i] : v[i + 16];
+        x[i] = keep + __shfl_xor_sync(0xffffffffu, send, 16);
+    }
+#pragma unroll
+    for (int o = 8; o > 0; o >>= 1)
+#pragma unroll
+        for (int i = 0; i < o; i++) {
+            const float keep = lane & o ? x[i + o] : x[i], send = lane & o ? x[i] : x[i + o];
+            x[i] = keep + __shfl_xor_sync(0xffffffffu, send, o);
+        }
+    return x[0];
+}
+
+__device__ __forceinline__ void ldm_x4_trans(uint32_t r[4], const __nv_bfloat16 *p) {
+    asm volatile("ldmatrix.sync.aligned.m8n8.x4.trans.shared.b16 {%0, %1, %2, %3}, [%4];"
+                 : "=r"(r[0]), "=r"(r[1]), "=r"(r[2]), "=r"(r[3])
+                 : "r"(smem_u32(p))
+                 : "memory");
+}
+
+__device__ __forceinline__ void mma_16816(float c[4], const uint32_t a[4], uint32_t b0, uint32_t b1) {
+    asm volatile("mma.sync.aligned.m16n8k16.row.col.f32.bf16.bf16.f32 {%0, %1, %2, %3}, {%4, %5, %6, %7}, {%8, %9}, {%0, %1, %2, %3};"
+                 : "+f"(c[0]), "+f"(c[1]), "+f"(c[2]), "+f"(c[3])
+                 : "r"(a[0]), "r"(a[1]), "r"(a[2]), "r"(a[3]), "r"(b0), "r"(b1));
+}
+
+__device__ __forceinline__ void add_to(float *g, float v, bool first) { *g = first ? v : *g + v; }
+
+// gW[o][i] += sum_r dz[r][o] hin[r][i] (64 x 64): warp w the outputs o in 16 (w & 3) .. + 15,
+// i in 32 (w >> 2) .. + 31; the smaller parts first.
+__device__ __forceinline__ void weight_grads(const BwdSmem &B, float *gW, bool first) {
+    const int lane = threadIdx.x & 31, w = threadIdx.x >> 5, m0 = (w & 3) * 16, n0 = (w >> 2) * 32;
+    const int ar = (lane & 7) + (lane >> 4) * 8, ac = m0 + ((lane >> 3) & 1) * 8;
+    const int br = (lane & 7) + ((lane >> 3) & 1) * 8, bc = n0 + (lane >> 4) * 8;
+    float acc[4][4];
+#pragma unroll
+    for (int n = 0; n < 4; n++)
+#pragma unroll
+        for (int j = 0; j < 4; j++) acc[n][j] = 0.0f;
+#pragma unroll 2
+    for (int k0 = 0; k0 < kRows; k0 += 16) {
+        uint32_t b[2][4];
+        ldm_x4_trans(b[0], B.hin + (k0 + br) * kLd + bc);
+        ldm_x4_trans(b[1], B.hin + (k0 + br) * kLd + bc + 16);
+#pragma unroll
+        for (int p = 2; p >= 0; p--) {
+            uint32_t a[4];
+            ldm_x4_trans(a, B.dz[p] + (k0 + ar) * kLd + ac);
+#pragma unroll
+            for (int n = 0; n < 4; n++) mma_16816(acc[n], a, b[n >> 1][2 * (n & 1)], b[n >> 1][2 * (n & 1) + 1]);
         }
     }
 #pragma unroll
-    for (int k = 0; k < 4; k++) {
-        float4 v;
-        upk2(acc[k][0], v.x, v.y);
-        upk2(acc[k][1], v.z, v.w);
-        float4 *dst = reinterpret_cast<float4 *>(gW + (o0 + k) * kH + i0);
-        if (!first) {
-            const float4 p = *dst;
-            v = make_float4(p.x + v.x, p.y + v.y, p.z + v.z, p.w + v.w);
+    for (int n = 0; n < 4; n++)
+#pragma unroll
+        for (int h = 0; h < 2; h++) {
+            float2 *dst = reinterpret_cast<float2 *>(gW + (m0 + (lane >> 2) + 8 * h) * kH + n0 + 8 * n + 2 * (lane & 3));
+            float2 v = make_float2(acc[n][2 * h], acc[n][2 * h + 1]);
+            if (!first) {
+                const float2 p = *dst;
+                v = make_float2(p.x + v.x, p.y + v.y);
+            }
+            *dst = v;
         }
-        *dst = v;
+}
+
+// The same for the first layer: four inputs, in the first eight columns of the input tile.
+__device__ __forceinline__ void weight_grads4(const BwdSmem &B, float *gW, bool first) {
+    const int lane = threadIdx.x & 31, w = threadIdx.x >> 5, m0 = (w & 3) * 16;
+    if (w >= 4) return;
+    const int ar = (lane & 7) + (lane >> 4) * 8, ac = m0 + ((lane >> 3) & 1) * 8;
+    float acc[4] = {0.0f, 0.0f, 0.0f, 0.0f};
+    for (int k0 = 0; k0 < kRows; k0 += 32) {
+        uint32_t b[4];  // rows k0 .. k0 + 31 of the eight columns
+        ldm_x4_trans(b, B.hin + (k0 + lane) * kLd);
+#pragma unroll
+        for (int h = 0; h < 2; h++)
+#pragma unroll
+            for (int p = 2; p >= 0; p--) {
+                uint32_t a[4];
+                ldm_x4_trans(a, B.dz[p] + (k0 + 16 * h + ar) * kLd + ac);
+                mma_16816(acc, a, b[2 * h], b[2 * h + 1]);
+            }
     }
+    if ((lane & 3) < 2)
+#pragma unroll
+        for (int h = 0; h < 2; h++)
+#pragma unroll
+            for (int j = 0; j < 2; j++)
+                add_to(gW + (m0 + (lane >> 2) + 8 * h) * 4 + 2 * (lane & 3) + j, acc[2 * h + j], first);
+}
+
+// Column sums over the tile from the warps' (after a barrier), by 64 threads.
+__device__ __forceinline__ void tile_columns(const BwdSmem &B, float *g, bool first) {
     if (threadIdx.x < kH) {
-        const float b = column_sum(B.dz, threadIdx.x);
-        gb[threadIdx.x] = first ? b : gb[threadIdx.x] + b;
+        const int o = threadIdx.x;
+        add_to(g + o, (B.sum[0][o] + B.sum[1][o]) + (B.sum[2][o] + B.sum[3][o]), first);
     }
 }
 
@@ -598,7 +699,7 @@ __global__ void __launch_bounds__(kBwd, 2) k_mlp_backward(MlpBackwardArgs a) {
     const __nv_bfloat16 *W2T = S.w, *W3T = S.w + kWElems;
     float *G = a.grad_partial + (size_t)blockIdx.x * kMlpPartial;  // this CTA's partial gradient
     const bool zvec = ((uintptr_t)a.z & 15) == 0;
-    float *my_dz = B.dz + lr * kLd + c0, *my_hin = B.hin + lr * kLd + c0;
+    float *my_sum = B.sum[(t >> 5) & 3] + c0 + (t & 31);  // where this lane's column sum goes
     uint32_t phase = 0;
     bool first = true;
     for (int tile = blockIdx.x; tile * kRows < a.n; tile += gridDim.x, first = false) {
@@ -608,68 +709,72 @@ __global__ void __launch_bounds__(kBwd, 2) k_mlp_backward(MlpBackwardArgs a) {
         float z[32], v[32], dz[32];
         load_z32(zr + 2 * kH, valid, zvec, z);
         const float dy = valid ? (a.y[row] - a.target[row]) * a.loss_scale : 0.0f;
-        if (c0 == 0) B.dy[lr] = dy;
-        // last layer: dz3, and dy h3 for dw4 in the input tile
+        // last layer: dz3, and the sums of dy h3 (dw4) and dy (db4)
 #pragma unroll
         for (int o = 0; o < 32; o++) {
             dz[o] = dy * __ldg(a.params + ow4 + c0 + o) * dsilu(z[o]);
             v[o] = dy * silu(z[o]);
         }
-        put32(my_dz, dz);
-        put32(my_hin, v);
-        put_bf16_32(S.act, lr, c0, dz);
         load_z32(zr + kH, valid, zvec, z);
-        layer_issue(S, W3T);  // dh2 = dz3 W3
-        if (t < kH) {
-            const float w = column_sum(B.hin, t);
-            G[ow4 + t] = first ? w : G[ow4 + t] + w;
-        } else if (t == kBwd - 1) {
-            float b = 0.0f;
-            for (int r = 0; r < kRows; r++) b += B.dy[r];
-            G[ob4] = first ? b : G[ob4] + b;
-        }
-        __syncthreads();
+        put_bf16_32(S.act, lr, c0, dz);
+        *my_sum = warp_columns(v);
+        if (c0 == 0) {
+            float d = dy;
 #pragma unroll
-        for (int o = 0; o < 32; o++) v[o] = __bfloat162float(__float2bfloat16_rn(silu(z[o])));
-        put32(my_hin, v);
+            for (int o = 16; o > 0; o >>= 1) d += __shfl_xor_sync(0xffffffffu, d, o);
+            if ((t & 31) == 0) B.dy[t >> 5] = d;
+        }
+        layer_issue(S, W3T);  // dh2 = dz3 W3
+        tile_columns(B, G + ow4, first);
+        if (t == 0) add_to(G + ob4, (B.dy[0] + B.dy[1]) + (B.dy[2] + B.dy[3]), first);
+        put_split32(B, lr, c0, dz);
+#pragma unroll
+        for (int o = 0; o < 32; o++) v[o] = silu(z[o]);
+        put_input32(B, lr, c0, v);
+        const float sum3 = warp_columns(dz);
         __syncthreads();
+        *my_sum = sum3;
         // layer 3: dW3 += dz3^T h2
-        weight_grads(B, G + oW3, G + ob3, first);
+        weight_grads(B, G + oW3, first);
         if (!layer_finish(S, phase, a.spin_limit)) break;
+        tile_columns(B, G + ob3, first);
         tmem_cols32(S.tmem, c0, v);
 #pragma unroll
         for (int o = 0; o < 32; o++) dz[o] = v[o] * dsilu(z[o]);
         // layer 2: dW2 += dz2^T h1, dh1 = dz2 W2
         load_z32(zr, valid, zvec, z);
-        put32(my_dz, dz);
         put_bf16_32(S.act, lr, c0, dz);
+        put_split32(B, lr, c0, dz);
+        const float sum2 = warp_columns(dz);
 #pragma unroll
-        for (int o = 0; o < 32; o++) v[o] = __bfloat162float(__float2bfloat16_rn(silu(z[o])));
-        put32(my_hin, v);
+        for (int o = 0; o < 32; o++) v[o] = silu(z[o]);
+        put_input32(B, lr, c0, v);
         layer_issue(S, W2T);
-        weight_grads(B, G + oW2, G + ob2, first);
+        *my_sum = sum2;
+        weight_grads(B, G + oW2, first);
         if (!layer_finish(S, phase, a.spin_limit)) break;
+        tile_columns(B, G + ob2, first);
         tmem_cols32(S.tmem, c0, v);
 #pragma unroll
         for (int o = 0; o < 32; o++) dz[o] = v[o] * dsilu(z[o]);
-        // layer 1: dW1 += dz1^T x, one output a thread
-        put32(my_dz, dz);
-        if (c0 == 0)
-#pragma unroll
-            for (int i = 0; i < 4; i++)
-                B.hin[lr * kLd + i] = valid ? __bfloat162float(__float2bfloat16_rn(a.feats[row * 4 + i])) : 0.0f;
-        __syncthreads();
-        {
-            const int o = t >> 2, i = t & 3;
-            float acc = 0.0f;
-#pragma unroll 16
-            for (int r = 0; r < kRows; r++) acc += B.dz[r * kLd + o] * B.hin[r * kLd + i];
-            G[oW1 + t] = first ? acc : G[oW1 + t] + acc;
-            if (t < kH) {
-                const float b = column_sum(B.dz, t);
-                G[ob1 + t] = first ? b : G[ob1 + t] + b;
+        // layer 1: dW1 += dz1^T x
+        put_split32(B, lr, c0, dz);
+        const float sum1 = warp_columns(dz);
+        if (c0 == 0) {
+            uint32_t w[4] = {0, 0, 0, 0};
+            if (valid) {
+                const float *f = a.feats + row * 4;
+                const __nv_bfloat162 f01 = __floats2bfloat162_rn(f[0], f[1]), f23 = __floats2bfloat162_rn(f[2], f[3]);
+                w[0] = *reinterpret_cast<const uint32_t *>(&f01);
+                w[1] = *reinterpret_cast<const uint32_t *>(&f23);
             }
+            *reinterpret_cast<uint4 *>(B.hin + lr * kLd) = make_uint4(w[0], w[1], w[2], w[3]);
         }
+        __syncthreads();
+        *my_sum = sum1;
+        weight_grads4(B, G + oW1, first);
+        __syncthreads();
+        tile_columns(B, G + ob1, first);
         __syncthreads();
     }
     if (t == 0 && S.fail && a.err) atomicExch(a.err, 1);

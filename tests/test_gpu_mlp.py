@@ -150,3 +150,26 @@ def test_train_epoch_equals_train_steps():
     b.check()
     assert np.array_equal(a.params().view(np.int32), b.params().view(np.int32))
     assert abs(float(loss[0]) - ref) <= 1e-4 * ref
+
+
+@pytest.mark.parametrize("n", [1, 31, 129, 2000, 40000])
+def test_gradient_row_counts(n):
+    """Partial tiles, one tile and more tiles than CTAs (a CTA then adds up several): each parameter
+    block against the oracle, and the gradient of all rows against the sum over two parts of them
+    (the same products, added in FP32 in another order)."""
+    p, x, t = _case(n, 6)
+    net = MLP(p)
+    xd, td = torch.as_tensor(x, device="cuda"), torch.as_tensor(t, device="cuda")
+    _, g = net.gradient(xd, td, 2.0 / n)
+    g_all = g.cpu().numpy().astype(np.float64)
+    net.check()
+    _, g_ref = mlp_ref.gradient(p, x, t, 2.0 / n)
+    for a, b in ((0, 256), (256, 320), (320, 4416), (4416, 4480), (4480, 8576), (8576, 8640), (8640, 8704), (8704, 8705)):
+        r = np.linalg.norm(g_all[a:b] - g_ref[a:b]) / max(np.linalg.norm(g_ref[a:b]), 1e-12)
+        assert r < 2e-2, (a, b, r)
+    if n > 1:
+        k = n // 3
+        parts = [net.gradient(xd[s].contiguous(), td[s].contiguous(), 2.0 / n)[1].cpu().numpy().astype(np.float64)
+                 for s in (slice(0, k), slice(k, n))]
+        # FP32 sums of up to 40,000 terms: a relative error of a few 2^-24 times the root of the count
+        assert np.linalg.norm(g_all - parts[0] - parts[1]) <= 4 * np.sqrt(n) * 2.0**-24 * sum(map(np.linalg.norm, parts))
