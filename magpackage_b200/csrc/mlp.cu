@@ -133,7 +133,7 @@ __device__ __forceinline__ void mma_issue(uint32_t tmem, const __nv_bfloat16 *A,
 
 // Columns c..c+15 of this thread's accumulator row from TMEM.
 __device__ __forceinline__ void tmem_cols16(uint32_t tmem, int c, float out[16]) {
-    const uint32_t lane_base = (uint32_t)((threadIdx.x >> 5) * 32) << 16;
+    const uint32_t lane_base = (uint32_t)(((threadIdx.x >> 5) & 3) * 32) << 16;
     uint32_t r[16];
     asm volatile(
         "tcgen05.ld.sync.aligned.32x32b.x16.b32 {%0,%1,%2,%3,%4,%5,%6,%7,%8,%9,%10,%11,%12,%13,%14,%15}, [%16];"
@@ -235,26 +235,26 @@ __device__ __forceinline__ void hidden_epilogue_infer(uint32_t tmem, const float
     }
 }
 
+// The backward kernel's images and barrier.
 struct Smem {
-    __nv_bfloat16 act[kRows * kH];      // layer input image (K=64) or the K=16 input image
-    __nv_bfloat16 w[2 * kWElems + kW1pElems];
-    float vec[4 * kH + 1];              // b1 | b2 | b3 | w4 | b4 (forward kernel)
+    __nv_bfloat16 act[kRows * kH];  // dZ image of the running layer
+    __nv_bfloat16 w[2 * kWElems];   // W2T | W3T
     uint64_t bar;
     uint32_t tmem;
     int fail;
 };
 
-__device__ __forceinline__ void load_ops(Smem &S, const __nv_bfloat16 *ops, int first, int count) {
+__device__ __forceinline__ void load_ops(__nv_bfloat16 *w, const __nv_bfloat16 *ops, int first, int count) {
     const uint4 *src = reinterpret_cast<const uint4 *>(ops + first);
-    uint4 *dst = reinterpret_cast<uint4 *>(S.w);
+    uint4 *dst = reinterpret_cast<uint4 *>(w);
     for (int i = threadIdx.x; i < count / 8; i += blockDim.x) dst[i] = src[i];
 }
 
 // load_ops with every weight halved (a power-of-two scale: exact for every weight above
 // 2^-125 in magnitude, where BF16 values are normal).
-__device__ __forceinline__ void load_ops_halved(Smem &S, const __nv_bfloat16 *ops, int first, int count) {
+__device__ __forceinline__ void load_ops_halved(__nv_bfloat16 *w, const __nv_bfloat16 *ops, int first, int count) {
     const uint4 *src = reinterpret_cast<const uint4 *>(ops + first);
-    uint4 *dst = reinterpret_cast<uint4 *>(S.w);
+    uint4 *dst = reinterpret_cast<uint4 *>(w);
     const __nv_bfloat162 half2 = __floats2bfloat162_rn(0.5f, 0.5f);
     for (int i = threadIdx.x; i < count / 8; i += blockDim.x) {
         uint4 v = src[i];
@@ -265,43 +265,72 @@ __device__ __forceinline__ void load_ops_halved(Smem &S, const __nv_bfloat16 *op
     }
 }
 
-__device__ __forceinline__ void tmem_alloc(Smem &S) {
+__device__ __forceinline__ void tmem_alloc(uint32_t *addr, uint32_t cols) {
     if (threadIdx.x < 32) {
-        asm volatile("tcgen05.alloc.cta_group::1.sync.aligned.shared::cta.b32 [%0], %1;" ::"r"(smem_u32(&S.tmem)),
-                     "r"(kH));
+        asm volatile("tcgen05.alloc.cta_group::1.sync.aligned.shared::cta.b32 [%0], %1;" ::"r"(smem_u32(addr)), "r"(cols));
         asm volatile("tcgen05.relinquish_alloc_permit.cta_group::1.sync.aligned;");
         tc_fence_before();  // the allocated address is read by every thread after the next barrier
     }
 }
 
-__device__ __forceinline__ void tmem_free(Smem &S) {
+__device__ __forceinline__ void tmem_free(uint32_t addr, uint32_t cols) {
     tc_fence_before();
     __syncthreads();
     if (threadIdx.x < 32) {
         tc_fence_after();
-        asm volatile("tcgen05.dealloc.cta_group::1.sync.aligned.b32 %0, %1;" ::"r"(S.tmem), "r"(kH));
+        asm volatile("tcgen05.dealloc.cta_group::1.sync.aligned.b32 %0, %1;" ::"r"(addr), "r"(cols));
     }
 }
 
-// The forward kernel's layer: one block-wide barrier per layer. The barrier before the
+// The forward kernel's shared memory: the weights, and per tile in flight an image and a
+// completion barrier.
+template <int TILES>
+struct FwdSmem {
+    __nv_bfloat16 act[TILES][kRows * kH];
+    __nv_bfloat16 w[2 * kWElems + kW1pElems];
+    float vec[4 * kH + 1];  // b1 | b2 | b3 | w4 | b4
+    uint64_t bar[TILES];
+    uint32_t tmem;
+    int fail;
+};
+
+// OR over the kRows threads of named barrier ID.
+template <int ID>
+__device__ __forceinline__ bool named_barrier_or(bool v) {
+    uint32_t any;
+    asm volatile(
+        "{\n\t.reg .pred p, q;\n\tsetp.ne.b32 q, %1, 0;\n\tbar.red.or.pred p, %2, %3, q;\n\tselp.b32 %0, 1, 0, p;\n\t}"
+        : "=r"(any)
+        : "r"((uint32_t)v), "n"(ID), "n"(kRows)
+        : "memory");
+    return any != 0;
+}
+
+// The barrier of tile `id` (0 or 1) of the CTA; the branch is uniform over the tile's warps.
+__device__ __forceinline__ bool tile_barrier_or(int id, bool v) {
+    return id == 0 ? named_barrier_or<1>(v) : named_barrier_or<2>(v);
+}
+
+// One layer of one tile: one barrier of the tile's threads per layer. The barrier before the
 // MMA issue also settles whether any thread's previous wait gave up (`ok` is this
 // thread's outcome of its last wait): then every thread leaves the tile loop together.
 // A wait that gives up drains first: the issued MMAs still read shared memory and write TMEM,
 // so the kernel waits for their commit (default bound) before it leaves the tile loop.
-__device__ __forceinline__ bool run_layer_fwd(Smem &S, const __nv_bfloat16 *W, int K, uint32_t &phase,
-                                              long long limit, bool &ok) {
+__device__ __forceinline__ bool run_layer_fwd(int tile_id, uint32_t tmem, const __nv_bfloat16 *act, const __nv_bfloat16 *W,
+                                              int K, uint64_t *bar, int *fail, uint32_t &phase, long long limit, bool &ok) {
     asm volatile("fence.proxy.async.shared::cta;" ::: "memory");  // smem writes -> tensor core
     tc_fence_before();
-    if (__syncthreads_or(ok ? 0 : 1) != 0) {
-        if (threadIdx.x == 0) S.fail = 1;
+    const bool issuer = threadIdx.x % kRows == 0;
+    if (tile_barrier_or(tile_id, !ok)) {
+        if (issuer) *fail = 1;
         return false;
     }
-    if (threadIdx.x == 0) {
+    if (issuer) {
         tc_fence_after();
-        mma_issue(S.tmem, S.act, W, K, &S.bar);
+        mma_issue(tmem, act, W, K, bar);
     }
-    ok = mbar_wait(&S.bar, phase, limit);
-    if (!ok) mbar_wait(&S.bar, phase);
+    ok = mbar_wait(bar, phase, limit);
+    if (!ok) mbar_wait(bar, phase);
     phase ^= 1u;
     tc_fence_after();
     return true;
@@ -310,30 +339,34 @@ __device__ __forceinline__ bool run_layer_fwd(Smem &S, const __nv_bfloat16 *W, i
 // ---- forward ---------------------------------------------------------------------
 
 // INFER: no pre-activations kept (prediction); the epilogues use the packed forms above.
-template <bool INFER>
-__global__ void __launch_bounds__(kRows, 6) k_mlp_forward(MlpForwardArgs a) {
+// TILES tiles run in a CTA, each with its kRows threads, image, TMEM columns and barriers; they
+// share the weights, so that 32 warps fit an SM instead of 24: 14.8 to 12.8 us at 100,000 rows; at 8M
+// rows 445 and 444 us, bound by the transcendental unit and its queue.
+template <bool INFER, int TILES>
+__global__ void __launch_bounds__(TILES * kRows, TILES == 2 ? 4 : 6) k_mlp_forward(MlpForwardArgs a) {
     extern __shared__ __align__(1024) unsigned char smem_raw[];
-    Smem &S = *reinterpret_cast<Smem *>(smem_raw);
-    const int t = threadIdx.x;
-    if (t == 0) {
-        mbar_init(&S.bar);
-        S.fail = 0;
-    }
+    FwdSmem<TILES> &S = *reinterpret_cast<FwdSmem<TILES> *>(smem_raw);
+    const int ct = threadIdx.x, t = ct % kRows, id = ct / kRows;
+    if (t == 0) mbar_init(&S.bar[id]);
+    if (ct == 0) S.fail = 0;
     // all weight images: W1p | W2 | W3 (contiguous in the operand buffer). Inference halves
     // W1..W3 and b1..b3 (exact), so that the accumulators hold z/2 (silu2h_bf16).
     const float hs = INFER ? 0.5f : 1.0f;
-    if (INFER) load_ops_halved(S, a.ops, bW1p, kW1pElems + 2 * kWElems);
-    else load_ops(S, a.ops, bW1p, kW1pElems + 2 * kWElems);
-    for (int i = t; i < kH; i += kRows) {
+    if (INFER) load_ops_halved(S.w, a.ops, bW1p, kW1pElems + 2 * kWElems);
+    else load_ops(S.w, a.ops, bW1p, kW1pElems + 2 * kWElems);
+    for (int i = ct; i < kH; i += TILES * kRows) {
         S.vec[i] = hs * a.params[ob1 + i];
         S.vec[kH + i] = hs * a.params[ob2 + i];
         S.vec[2 * kH + i] = hs * a.params[ob3 + i];
         S.vec[3 * kH + i] = a.params[ow4 + i];
     }
-    if (t == 0) S.vec[4 * kH] = a.params[ob4];
-    tmem_alloc(S);
+    if (ct == 0) S.vec[4 * kH] = a.params[ob4];
+    tmem_alloc(&S.tmem, TILES * kH);
     __syncthreads();
     tc_fence_after();
+    const uint32_t tmem = S.tmem + (uint32_t)(id * kH);  // this tile's accumulator columns
+    __nv_bfloat16 *act = S.act[id];
+    const int stride = (int)gridDim.x * TILES;
     const __nv_bfloat16 *W1 = S.w, *W2 = S.w + kW1pElems, *W3 = S.w + kW1pElems + kWElems;
     const float *sb1 = S.vec, *sb2 = S.vec + kH, *sb3 = S.vec + 2 * kH, *sw4 = S.vec + 3 * kH;
     const bool zvec = ((uintptr_t)a.z_out & 15) == 0;
@@ -346,19 +379,19 @@ __global__ void __launch_bounds__(kRows, 6) k_mlp_forward(MlpForwardArgs a) {
     float4 f_next = make_float4(0.f, 0.f, 0.f, 0.f);
     int64_t dst_next = 0;
     {
-        const int64_t r0 = (int64_t)blockIdx.x * kRows + t;
+        const int64_t r0 = ((int64_t)blockIdx.x * TILES + id) * kRows + t;
         if (r0 < a.n) {
             f_next = __ldg(feats4 + r0);
             dst_next = a.rows ? (int64_t)__ldg(a.rows + r0) : r0;
         }
     }
-    for (int tile = blockIdx.x; tile * kRows < a.n; tile += gridDim.x) {
-        const int64_t row = (int64_t)tile * kRows + t;
+    for (int64_t tile = (int64_t)blockIdx.x * TILES + id; tile * kRows < a.n; tile += stride) {
+        const int64_t row = tile * kRows + t;
         const bool valid = row < a.n;
         const float4 f = f_next;
         const int64_t dst = dst_next;
         {
-            const int64_t rn = row + (int64_t)gridDim.x * kRows;
+            const int64_t rn = row + (int64_t)stride * kRows;
             if (rn < a.n) {
                 f_next = __ldg(feats4 + rn);
                 dst_next = a.rows ? (int64_t)__ldg(a.rows + rn) : rn;
@@ -374,30 +407,30 @@ __global__ void __launch_bounds__(kRows, 6) k_mlp_forward(MlpForwardArgs a) {
         {  // input image, K = 16 (features 4..15 are zero)
             __align__(16) __nv_bfloat16 v[16];
             for (int i = 0; i < 16; i++) v[i] = __float2bfloat16_rn(i < 4 ? x[i] : 0.0f);
-            *reinterpret_cast<uint4 *>(S.act + core_off(t, 0, 16)) = *reinterpret_cast<uint4 *>(v);
-            *reinterpret_cast<uint4 *>(S.act + core_off(t, 8, 16)) = *reinterpret_cast<uint4 *>(v + 8);
+            *reinterpret_cast<uint4 *>(act + core_off(t, 0, 16)) = *reinterpret_cast<uint4 *>(v);
+            *reinterpret_cast<uint4 *>(act + core_off(t, 8, 16)) = *reinterpret_cast<uint4 *>(v + 8);
         }
         float *zr = (a.z_out && valid) ? a.z_out + row * 3 * kH : nullptr;
         // layer 1
         // (a completed MMA has read its input image; the next layer's issue barrier orders
         // every thread's TMEM reads and image writes before the next MMA, also across tiles:
         // the next tile's first MMA is issued after its own barrier)
-        if (!run_layer_fwd(S, W1, 16, phase, a.spin_limit, ok)) break;
-        if (INFER) hidden_epilogue_infer(S.tmem, sb1, S.act, t);
-        else hidden_epilogue(S.tmem, sb1, S.act, t, zr, zvec);
+        if (!run_layer_fwd(id, tmem, act, W1, 16, &S.bar[id], &S.fail, phase, a.spin_limit, ok)) break;
+        if (INFER) hidden_epilogue_infer(tmem, sb1, act, t);
+        else hidden_epilogue(tmem, sb1, act, t, zr, zvec);
         // layer 2
-        if (!run_layer_fwd(S, W2, kH, phase, a.spin_limit, ok)) break;
-        if (INFER) hidden_epilogue_infer(S.tmem, sb2, S.act, t);
-        else hidden_epilogue(S.tmem, sb2, S.act, t, zr ? zr + kH : nullptr, zvec);
+        if (!run_layer_fwd(id, tmem, act, W2, kH, &S.bar[id], &S.fail, phase, a.spin_limit, ok)) break;
+        if (INFER) hidden_epilogue_infer(tmem, sb2, act, t);
+        else hidden_epilogue(tmem, sb2, act, t, zr ? zr + kH : nullptr, zvec);
         // layer 3 and the 64 -> 1 output, 16 columns at a time
-        if (!run_layer_fwd(S, W3, kH, phase, a.spin_limit, ok)) break;
+        if (!run_layer_fwd(id, tmem, act, W3, kH, &S.bar[id], &S.fail, phase, a.spin_limit, ok)) break;
         float y = 0.0f;
         if (INFER) {  // pairs of halved pre-activations: single-precision tanh (the output is not rounded to BF16)
             uint64_t yacc = pk2(0.0f, 0.0f);
 #pragma unroll
             for (int c = 0; c < kH; c += 16) {
                 float z[16];
-                tmem_cols16(S.tmem, c, z);
+                tmem_cols16(tmem, c, z);
 #pragma unroll
                 for (int i = 0; i < 8; i++) {
                     // biases and output weights by 16-byte shared loads, two pairs each
@@ -423,7 +456,7 @@ __global__ void __launch_bounds__(kRows, 6) k_mlp_forward(MlpForwardArgs a) {
 #pragma unroll
             for (int c = 0; c < kH; c += 16) {
                 float z[16];
-                tmem_cols16(S.tmem, c, z);
+                tmem_cols16(tmem, c, z);
 #pragma unroll
                 for (int i = 0; i < 16; i++) {
                     z[i] += sb3[c + i];
@@ -443,8 +476,8 @@ __global__ void __launch_bounds__(kRows, 6) k_mlp_forward(MlpForwardArgs a) {
         }
     }
     if (!ok) S.fail = 1;  // a wait of the last layer gave up
-    tmem_free(S);         // (its barrier makes S.fail visible to thread 0)
-    if (t == 0 && S.fail && a.err) atomicExch(a.err, 1);
+    tmem_free(S.tmem, TILES * kH);  // (its barrier makes S.fail visible to thread 0)
+    if (ct == 0 && S.fail && a.err) atomicExch(a.err, 1);
 }
 
 // ---- backward --------------------------------------------------------------------
@@ -692,8 +725,8 @@ __global__ void __launch_bounds__(kBwd, 2) k_mlp_backward(MlpBackwardArgs a) {
         mbar_init(&S.bar);
         S.fail = 0;
     }
-    load_ops(S, a.ops, bW2T, 2 * kWElems);  // W2T | W3T
-    tmem_alloc(S);
+    load_ops(S.w, a.ops, bW2T, 2 * kWElems);  // W2T | W3T
+    tmem_alloc(&S.tmem, kH);
     __syncthreads();
     tc_fence_after();
     const __nv_bfloat16 *W2T = S.w, *W3T = S.w + kWElems;
@@ -778,7 +811,7 @@ __global__ void __launch_bounds__(kBwd, 2) k_mlp_backward(MlpBackwardArgs a) {
         __syncthreads();
     }
     if (t == 0 && S.fail && a.err) atomicExch(a.err, 1);
-    tmem_free(S);
+    tmem_free(S.tmem, kH);
 }
 
 // grad[p] = sum over CTAs (fixed order) of the partials. A CTA of eight warps takes 32
@@ -880,31 +913,39 @@ int mlp_sqerr(const float *y, const float *t, int64_t b, float *acc, cudaStream_
     return cudaPeekAtLastError() == cudaSuccess ? MAG_OK : MAG_E_CUDA;
 }
 
-size_t mlp_forward_smem() { return sizeof(Smem) + 1024; }
-size_t mlp_backward_smem() { return sizeof(BwdSmem) + 1024; }
 
 int mlp_pack(const float *params, __nv_bfloat16 *ops, cudaStream_t s) {
     k_mlp_pack<<<(kH * kH + 255) / 256, 256, 0, s>>>(params, ops);
     return cudaPeekAtLastError() == cudaSuccess ? MAG_OK : MAG_E_CUDA;
 }
 
-int mlp_forward(const MlpForwardArgs &a, int grid, cudaStream_t s) {
-    size_t sm = sizeof(Smem);
-    auto kern = a.z_out ? k_mlp_forward<false> : k_mlp_forward<true>;
+namespace {
+
+template <bool INFER, int TILES>
+int launch_forward(const MlpForwardArgs &a, int tiles, cudaStream_t s) {
+    constexpr size_t sm = sizeof(FwdSmem<TILES>);
+    auto kern = k_mlp_forward<INFER, TILES>;
     cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)sm);
-    // The CTAs loop over tiles; launching several waves of them (48 per SM, about 9 tiles
-    // each at 8M rows) lets SMs that finish early take more CTAs, which evens out the tail
-    // (measured at 7.99M rows: 8 per SM 0.514 ms, 24 0.474, 48 0.467, 96 0.470, one tile per
-    // CTA 0.654: the per-CTA weight load and TMEM allocation then dominate). A build option.
-#ifndef MAG_MLP_CTAS_PER_SM
-#define MAG_MLP_CTAS_PER_SM 48
+    // The CTAs loop over tiles; launching several waves of them (about 9 tiles each at 8M rows)
+    // lets SMs that finish early take more CTAs, which evens out the tail (measured at 7.99M rows
+    // with one tile per CTA at a time: 8 CTAs per SM 0.514 ms, 24 0.474, 48 0.467, 96 0.470, one
+    // tile per CTA 0.654: the per-CTA weight load and TMEM allocation then dominate).
+#ifndef MAG_MLP_TILES_PER_SM
+#define MAG_MLP_TILES_PER_SM 48
 #endif
-    int dev = 0, nsm = 0;
+    int grid = (tiles + TILES - 1) / TILES, dev = 0, nsm = 0;
+    constexpr int most = MAG_MLP_TILES_PER_SM / TILES;
     if (cudaGetDevice(&dev) == cudaSuccess && cudaDeviceGetAttribute(&nsm, cudaDevAttrMultiProcessorCount, dev) == cudaSuccess &&
-        nsm > 0 && grid > MAG_MLP_CTAS_PER_SM * nsm)
-        grid = MAG_MLP_CTAS_PER_SM * nsm;
-    kern<<<grid, kRows, sm, s>>>(a);
+        nsm > 0 && grid > most * nsm)
+        grid = most * nsm;
+    kern<<<grid, TILES * kRows, sm, s>>>(a);
     return cudaPeekAtLastError() == cudaSuccess ? MAG_OK : MAG_E_CUDA;
+}
+
+}  // namespace
+
+int mlp_forward(const MlpForwardArgs &a, int tiles, cudaStream_t s) {
+    return a.z_out ? launch_forward<false, 1>(a, tiles, s) : launch_forward<true, 2>(a, tiles, s);
 }
 
 int mlp_backward(const MlpBackwardArgs &a, int grid, cudaStream_t s) {

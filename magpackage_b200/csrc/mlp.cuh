@@ -40,10 +40,8 @@ struct MlpBackwardArgs {
     long long spin_limit;
 };
 
-size_t mlp_forward_smem();
-size_t mlp_backward_smem();
 int mlp_pack(const float *params, __nv_bfloat16 *ops, cudaStream_t s);
-int mlp_forward(const MlpForwardArgs &a, int grid, cudaStream_t s);
+int mlp_forward(const MlpForwardArgs &a, int tiles, cudaStream_t s);  // tiles of 128 rows
 int mlp_backward(const MlpBackwardArgs &a, int grid, cudaStream_t s);
 int mlp_adam(float *params, const float *grad, float *m, float *v, float lr, float b1, float b2, float eps,
              int step, cudaStream_t s);
