@@ -152,32 +152,35 @@ __global__ void __launch_bounds__(128, 3) k_hbfem_elems(HbArgs A) {
 // A CTA of six warps takes kHbElems = 32 elements, lane = element:
 //   1. warp i loads the harmonic values of local edge i; warp 0 the geometry (curls with the
 //      edge signs folded in: negation commutes with rounding);
-//   2. warp i evaluates samples i, i + 6, ...: A(t), B(t), nu(t), H(t) into shared memory,
-//      kHbSamples at a time (one load of a harmonic value serves them all, and their spline
-//      searches run side by side: the lookup is a chain of dependent loads);
+//   2. warp i evaluates samples i, i + 6, ...: A(t), B(t), nu(t), H(t), kHbSamples at a time
+//      (one load of a harmonic value serves them all, and their spline searches run side by
+//      side: the lookup is a chain of dependent loads). NT > 0: it has the curls of all six
+//      edges in registers, so it leaves v(t) = w C_i . H(t) of every edge in shared memory,
+//      where H would be read and multiplied again by six threads, and keeps nu in registers
+//      until the harmonic values' place is free;
 //   3. warp i sums the 2K residual entries of edge i. NT > 0: N <= NT samples, padded with
-//      zeros (adding +0 changes no sum, which starts from +0 and so is never -0); v(t) =
-//      w C_i . H(t) goes to the thread's own column of shared memory, over H and nu, so that
-//      only the products are held in registers and three CTAs fit an SM. NT = 0: any N,
-//      kHbGroup sums at a time, v(t) formed in the loop.
+//      zeros (adding +0 changes no sum, which starts from +0 and so is never -0); v(t) is read
+//      from the thread's own column of shared memory, so that only the products are held in
+//      registers and three CTAs fit an SM. NT = 0: any N, kHbGroup sums at a time, H from
+//      shared memory and v(t) formed in the loop.
 // Work per element, without FMA (parity): 2 K 6 N (nq + 1) operations for the sums, N (24 K +
 // 75) for the fields; at 40^3 (384,000 elements), K = 3, N = 32 that is 0.24 ms of the FP64
 // pipe. Measured there, whole call: one thread per element with the time loop inside the point
 // loop 1687 us; this split with v in registers (160 of them, two CTAs per SM, one sample at a
-// time) 736 us; with v in shared memory and three CTAs 624 us (two CTAs: 721 us). Latency of
-// the sums' dependent additions and of the spline lookups bounds it now.
+// time) 736 us; with v in shared memory, formed from H by step 3, and three CTAs 624 us (two
+// CTAs: 721 us); with v formed by step 2, 602 us (two CTAs, nothing spilled: 662 us). Latency
+// of the sums' dependent additions and of the spline lookups bounds it now.
 constexpr int kHbElems = 32;
 constexpr int kHbThreads = 6 * kHbElems;
 constexpr int kHbSamples = 3;
 constexpr int kHbGroup = 8;
 constexpr size_t kHbMaxSmem = 200 * 1024;
 
-// Shared memory: curls and weight [19][32]; harmonic values [6][2K][32], reused for the
-// results; D and P [4K][np]; then H [np][3][32] and nu [np][32], which v [np][6][32] overlays
-// when NT > 0.
+// Shared memory: curls and weight [19][32]; harmonic values [6][2K][32], reused for nu (NT > 0)
+// and the results; D and P [4K][np]; then v [np][6][32] (NT > 0) or H [np][3][32] and nu [np][32].
 size_t hb_smem_bytes(int K, int N, int NT) {
-    const int np = NT > 0 ? NT : N;
-    return sizeof(double) * ((size_t)kHbElems * (19 + 6 * 2 * K) + (size_t)4 * K * np +
+    const int np = NT > 0 ? NT : N, held = NT > 0 && 12 * K < np ? np : 12 * K;
+    return sizeof(double) * ((size_t)kHbElems * (19 + held) + (size_t)4 * K * np +
                              (size_t)kHbElems * np * (NT > 0 ? 6 : 4));
 }
 
@@ -257,10 +260,10 @@ __global__ void __launch_bounds__(kHbThreads, NT > 0 ? 3 : 1) k_hbfem_std(HbArgs
     double *sC = hb_smem;                    // [18][32] signed curls
     double *sw = sC + 18 * kHbElems;         // [32] weight
     double *sa = sw + kHbElems;              // [6][2K][32] harmonic values; the results at the end
-    double *sd = sa + 6 * W * kHbElems;      // [2K][NP] D re | im
+    double *sd = sa + (NT > 0 && 6 * W < NP ? NP : 6 * W) * kHbElems;  // [2K][NP] D re | im
     double *sp = sd + W * NP;                // [2K][NP] P re | im
-    double *sH = sp + W * NP;                // [NP][3][32]
-    double *snu = sH + 3 * NP * kHbElems;    // [NP][32]
+    double *sH = sp + W * NP;                // [NP][3][32]; NT > 0: v [NP][6][32]
+    double *snu = NT > 0 ? sa : sH + 3 * NP * kHbElems;  // [NP][32]
     const int wi = threadIdx.x >> 5, lane = threadIdx.x & 31;
     const int64_t e0 = (int64_t)blockIdx.x * kHbElems, e = e0 + lane;
     const bool valid = e < A.m.ne;
@@ -293,15 +296,18 @@ __global__ void __launch_bounds__(kHbThreads, NT > 0 ? 3 : 1) k_hbfem_std(HbArgs
         sw[lane] = A.qp.qw[0] * g.adet;
     }
     __syncthreads();
+    constexpr int kPasses = NT > 0 ? (NT + 6 * kHbSamples - 1) / (6 * kHbSamples) : 1;
+    double nuk[kPasses][kHbSamples];  // NT > 0: nu of this thread's samples
     if (valid) {
         double C[6][3];
+        const double wq = sw[lane];
 #pragma unroll
         for (int i = 0; i < 6; i++)
 #pragma unroll
             for (int r = 0; r < 3; r++) C[i][r] = sC[(3 * i + r) * kHbElems + lane];
-        for (int t = wi; t < N; t += 6 * kHbSamples) {
+        auto samples = [&](int t, double (&nu)[kHbSamples]) {
             int ts[kHbSamples];
-            double at[kHbSamples][6], B[kHbSamples][3], s[kHbSamples], nu[kHbSamples];
+            double at[kHbSamples][6], B[kHbSamples][3], s[kHbSamples];
 #pragma unroll
             for (int u = 0; u < kHbSamples; u++) {  // past the end: the first sample again
                 ts[u] = t + 6 * u < N ? t + 6 * u : t;
@@ -340,16 +346,44 @@ __global__ void __launch_bounds__(kHbThreads, NT > 0 ? 3 : 1) k_hbfem_std(HbArgs
             material_nu<kHbSamples>(A.mp, tag, s, nu);
 #pragma unroll
             for (int u = 0; u < kHbSamples; u++) {
-                snu[ts[u] * kHbElems + lane] = nu[u];
+                const double H[3] = {nu[u] * B[u][0], nu[u] * B[u][1], nu[u] * B[u][2]};
+                if constexpr (NT > 0) {
 #pragma unroll
-                for (int c = 0; c < 3; c++) sH[(3 * ts[u] + c) * kHbElems + lane] = nu[u] * B[u][c];
+                    for (int i = 0; i < 6; i++)
+                        sH[(6 * ts[u] + i) * kHbElems + lane] =
+                            wq * (C[i][0] * H[0] + C[i][1] * H[1] + C[i][2] * H[2]);
+                } else {
+                    snu[ts[u] * kHbElems + lane] = nu[u];
+#pragma unroll
+                    for (int c = 0; c < 3; c++) sH[(3 * ts[u] + c) * kHbElems + lane] = H[c];
+                }
             }
+        };
+        if constexpr (NT > 0) {
+#pragma unroll
+            for (int p = 0; p < kPasses; p++)
+                if (wi + 6 * kHbSamples * p < N) samples(wi + 6 * kHbSamples * p, nuk[p]);
+        } else {
+            for (int t = wi; t < N; t += 6 * kHbSamples) samples(t, nuk[0]);
         }
     }
+    if constexpr (NT > 0)
+        for (int t = N; t < NT; t++) sH[(6 * t + wi) * kHbElems + lane] = 0.0;
     __syncthreads();
     const double c0 = sC[(3 * wi) * kHbElems + lane], c1 = sC[(3 * wi + 1) * kHbElems + lane],
                  c2 = sC[(3 * wi + 2) * kHbElems + lane], w = sw[lane];  // (not read for an invalid lane)
     const int nq = A.qp.nq;
+    if (NT > 0 && (A.scratch || A.nu_dc)) {  // the harmonic values are used up
+        if (valid)
+#pragma unroll
+            for (int p = 0; p < kPasses; p++)
+#pragma unroll
+                for (int u = 0; u < kHbSamples; u++) {
+                    const int t = wi + 6 * kHbSamples * p + 6 * u;
+                    if (t < N) snu[t * kHbElems + lane] = nuk[p][u];
+                }
+        __syncthreads();
+    }
     if (valid && (A.scratch || (A.nu_dc && wi == 5))) {
         double sum_nu = 0.0;
         for (int t = 0; t < N; t++) sum_nu = sum_nu + snu[t * kHbElems + lane];
@@ -371,21 +405,8 @@ __global__ void __launch_bounds__(kHbThreads, NT > 0 ? 3 : 1) k_hbfem_std(HbArgs
     }
     double *out = sa + (lane * 6 + wi) * W;  // the harmonic values are used up
     if constexpr (NT > 0) {
-        double *sv = sH + threadIdx.x;  // [NT][6][32], this thread's column
-        {
-            double v[NT];
-#pragma unroll
-            for (int t = 0; t < NT; t++) {
-                v[t] = 0.0;
-                if (valid && t < N) {
-                    const double *H = sH + 3 * t * kHbElems + lane;
-                    v[t] = w * (c0 * H[0] + c1 * H[kHbElems] + c2 * H[2 * kHbElems]);
-                }
-            }
-            __syncthreads();  // H and nu are used up
-#pragma unroll
-            for (int t = 0; t < NT; t++) sv[t * kHbThreads] = v[t];
-        }
+        const double *sv = sH + threadIdx.x;  // [NT][6][32], this thread's column
+        if (A.scratch || A.nu_dc) __syncthreads();  // nu is used up
         if (valid)
 #pragma unroll 1
             for (int c = 0; c < W; c++) {
