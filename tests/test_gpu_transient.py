@@ -132,6 +132,52 @@ def test_pcg_auxiliary_space_cuts_iterations():
         prob.close()
 
 
+@pytest.mark.parametrize("n", [1, 31, 33, 5000])
+@pytest.mark.parametrize("aux", [False, True])
+def test_pcg_row_lengths_and_sizes_against_scipy(n, aux):
+    """One to thousands of rows of up to 40 entries, with and without a gradient space whose rows are
+    longer than an edge's two and whose transpose has rows of up to 193. kappa(A) < 100 (diagonally
+    dominant by a factor above 1.02), so the error is below kappa times the residual."""
+    rng = np.random.default_rng(n)
+    width = rng.integers(0, 4, n)
+    width[: max(1, n // 16)] = 30
+    rows = np.repeat(np.arange(n), width)
+    B = sp.csr_matrix((rng.normal(size=rows.size), (rows, rng.integers(0, n, rows.size))), shape=(n, n))
+    A = B + B.T
+    A.setdiag(0.0)
+    A = (A + sp.diags(1.05 * np.abs(A).sum(axis=1).A1 + 1.0)).tocsr()
+    A.sort_indices()
+    ni = max(1, n // 40)
+    G = sp.random(n, ni, density=min(1.0, 4.0 / ni), random_state=n, format="csr") if ni > 1 else sp.csr_matrix(
+        np.ones((n, 1)))
+    Gt = G.T.tocsr()
+    dn = 1.0 / ((Gt @ A @ G).diagonal() + 1.0)
+    b = rng.normal(size=n)
+
+    def dev(m):
+        return [torch.as_tensor(v, device="cuda") for v in (m.indptr.astype(np.int64), m.indices.astype(np.int32), m.data)]
+
+    da, dg, dgt = dev(A), dev(G), dev(Gt)
+    ddn, db = torch.as_tensor(dn, device="cuda"), torch.as_tensor(b, device="cuda")
+    L, h = _lib.lib(), C.c_void_p()
+    _lib.check(L.mag_pcg_create(n, C.byref(h)))
+    out = []
+    try:
+        if aux:
+            _lib.check(L.mag_pcg_set_aux(h, ni, *[_ptr(t) for t in dg + dgt + [ddn]]))
+        for _ in range(2):
+            x = torch.zeros_like(db)
+            it, rel, st = C.c_int(), C.c_double(), C.c_int()
+            _lib.check(L.mag_pcg_solve(h, *[_ptr(t) for t in da], _ptr(db), _ptr(x), 1e-11, 2000, C.byref(it),
+                                       C.byref(rel), C.byref(st), _lib.stream_ptr()))
+            assert st.value == 1 and rel.value <= 1e-11
+            out.append(x.cpu().numpy())
+    finally:
+        L.mag_pcg_destroy(h)
+    assert np.array_equal(out[0], out[1])
+    assert np.linalg.norm(A @ out[0] - b) <= 2e-11 * np.linalg.norm(b)
+
+
 def test_coil_source_is_discretely_divergence_free():
     from magpackage_b200.transient import TransientConfig, TransientProblem
 
