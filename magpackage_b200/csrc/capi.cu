@@ -352,6 +352,7 @@ struct mag_mesh {
     int schedule = MAG_SCHEDULE_ROW_BLOCKS;
     double *fres = nullptr;            // [Ne][6] residual entries (NULL: residuals by the tile kernel)
     cudaEvent_t fres_done = nullptr;   // after its last use
+    std::mutex turn;                   // threads that enqueue a use of fres, or make the pool
     cudaMemPool_t pool = nullptr;  // workspaces of single calls (NULL: the device's default pool)
     int64_t bytes = 0;
 
@@ -423,7 +424,10 @@ int workspace(mag_mesh *m, size_t bytes, cudaStream_t s, double **p) {
     void *v = nullptr;
     cudaStreamCaptureStatus cap = cudaStreamCaptureStatusNone;
     MAG_CUDA_TRY(cudaStreamIsCapturing(s, &cap));
-    if (!m->pool && cap == cudaStreamCaptureStatusNone) m->pool = make_pool();
+    {
+        std::lock_guard<std::mutex> lk(m->turn);
+        if (!m->pool && cap == cudaStreamCaptureStatusNone) m->pool = make_pool();
+    }
     if (m->pool && cap == cudaStreamCaptureStatusNone) MAG_CUDA_TRY(cudaMallocFromPoolAsync(&v, bytes, m->pool, s));
     else MAG_CUDA_TRY(cudaMallocAsync(&v, bytes, s));
     *p = static_cast<double *>(v);
@@ -450,7 +454,8 @@ void make_residual_buffer(mag_mesh *m) {
 
 // Whether that path serves this call: not inside a stream capture (the graph would hold the
 // handle's buffer) and not without the buffer. Calls on different streams take turns at the
-// buffer: each waits for the event recorded after the last use.
+// buffer: each waits for the event recorded after the last use. The caller holds m->turn from here
+// until it has recorded its own, so that no other thread's wait comes between.
 bool residual_begin(mag_mesh *m, cudaStream_t s) {
     cudaStreamCaptureStatus cap = cudaStreamCaptureStatusNone;
     if (m->fres && cudaStreamIsCapturing(s, &cap) == cudaSuccess && cap == cudaStreamCaptureStatusNone &&
@@ -686,10 +691,13 @@ int mag_assemble_jacobian(mag_mesh *m, const double *d_sol, double *d_vals, doub
     }
     cudaStream_t s = (cudaStream_t)stream;
     if (m->schedule == MAG_SCHEDULE_TILE_BLOCKS && m->tile.ok && m->qp.standard_curl) {
-        if (!calc_j && residual_begin(m, s)) {
-            MAG_TRY(launch_residual(m->elems(), m->rows(), d_sol, m->qp, m->mat.mp, m->fres, d_res, s));
-            MAG_CUDA_TRY(cudaEventRecord(m->fres_done, s));
-            return finish(s);
+        if (!calc_j && m->fres) {
+            std::lock_guard<std::mutex> lk(m->turn);
+            if (residual_begin(m, s)) {
+                MAG_TRY(launch_residual(m->elems(), m->rows(), d_sol, m->qp, m->mat.mp, m->fres, d_res, s));
+                MAG_CUDA_TRY(cudaEventRecord(m->fres_done, s));
+                return finish(s);
+            }
         }
         MAG_TRY(launch_tile_jacobian(m->tile, m->elems(), d_sol, m->qp, m->mat.mp, calc_j, calc_j ? d_vals : nullptr,
                                      d_res, m->status, s));

@@ -199,8 +199,11 @@ __global__ void __launch_bounds__(kThreads) k_pcg_init_reduce(PcgBufs B, double 
 // does. The sums keep the order of kThreads-thread blocks on grids of grid_for(8 n) (rows) and
 // grid_for(n) (vectors): a CTA holds kPcgSub such blocks. Measured on the E-core problem at
 // 40 x 40 x 20 (233,700 unknowns, 15,600 iterations): 39 us an iteration as launches, 30 us so;
-// of those the rows' product takes 13 us (latency of its three dependent loads, L1 lookups of
-// the gathers), each barrier 1.6 us, the rest 2 to 4 us each.
+// of those the rows' product takes 13 us, each barrier 1.6 us, the rest 2 to 4 us each. The
+// product is bound by the load/store unit (8 lanes a row; by count 60 of its cycles per warp and
+// pass), not by latency or L2. With the column indices kept in shared memory, 485 ms for the
+// problem's step against 487; with p gathered from shared memory by per-pass lists of distinct
+// columns, one pass ahead 571 ms, three ahead by cp.async 581 ms.
 constexpr int kPcgSub = 4;
 constexpr int kPcgThreads = kPcgSub * kThreads;
 constexpr int kPcgRows = 2;     // rows of one lane group in flight

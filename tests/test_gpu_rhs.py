@@ -187,3 +187,38 @@ def test_residual_alone_equals_jacobian_call(n, absent, weights):
         _, got = plan.jacobian(sol, calc_j=False)
     assert torch.equal(got, want) and float(want.abs().max()) > 0
     plan.check()
+
+
+def test_residuals_of_one_mesh_from_several_threads():
+    """Threads with a stream each evaluate residuals of their own states on one mesh handle; each
+    gets its state's, bit for bit."""
+    import threading
+
+    from magpackage_b200.material import pack_material_data
+    from magpackage_b200.plan import generate_edges
+
+    mesh = synth.kuhn_box(33, seed=2)
+    assert mesh.num_elements >= 200000
+    edges, t2e, sign = generate_edges(mesh.T)
+    plan = AssemblyPlan(mesh.P, mesh.T, t2e, int(edges.shape[0]), synth.cube_layout(mesh), sign)
+    plan.set_materials(pack_material_data(synth.standard_materials()))
+    g = torch.Generator(device="cuda").manual_seed(1)
+    sols = [3e-4 * torch.randn(plan.num_dofs, dtype=torch.float64, device="cuda", generator=g) for _ in range(4)]
+    want = [plan.jacobian(x)[1] for x in sols]
+    got = [[plan.new_vector() for _ in range(24)] for _ in sols]
+    torch.cuda.synchronize()
+
+    def work(x, outs):
+        with torch.cuda.stream(torch.cuda.Stream()):
+            for r in outs:
+                plan.jacobian(x, None, r, calc_j=False)
+            torch.cuda.current_stream().synchronize()
+
+    threads = [threading.Thread(target=work, args=a) for a in zip(sols, got)]
+    for t in threads:
+        t.start()
+    for t in threads:
+        t.join()
+    for w, outs in zip(want, got):
+        assert all(torch.equal(w, r) for r in outs)
+    plan.check()
