@@ -654,6 +654,12 @@ constexpr int kSmallMinB = 3;
 
 namespace {
 
+// A block at every limit of the plan (a chunk has a row that owns it, or lies inside one), with the
+// mass kernels' basis values, fits a CTA.
+static_assert((kTileMaxNnz + 1 + kTileSlotPad) * 8 + kTileMaxInc * 16 +
+                      (2 * kTileMaxRows + kTileMaxNnz / kTileChunk + 1) * 8 + 18 * kMaxQuad * 8 <= 227 * 1024,
+              "a block's shared memory");
+
 // Shared memory of one CTA: the block's values (an even count of doubles), the incidence
 // slots (double2), then the block's row table and store chunks (uint2 each).
 size_t tile_smem_bytes(const TilePlan &tp, TileArgs *a) {

@@ -12,6 +12,8 @@ namespace mag {
 
 constexpr int kTileMaxNnz = 8191;   // CSR nonzeros per block (13-bit offsets in the row table)
 constexpr int kTileMaxInc = 4095;   // (row, element) incidences per block (12-bit offsets)
+constexpr int kTileMaxRows = 1536;  // rows per block: more than 8191 / 6, so that only rows without an element (which
+                                    // have neither nonzeros nor incidences) and rows of a few entries reach it
 constexpr int kTileMaxColors = 8;   // element colour classes per block
 constexpr int kTileChunk = 256;     // nonzeros per store chunk (one warp stores a chunk)
 constexpr int kTileSlotPad = 32;    // doubles of slack after a block's values in shared memory (even):

@@ -3,7 +3,8 @@
 //   layers   the node coordinates of each axis, sorted; a layer ends where consecutive values
 //            lie more than 0.3 h apart or it would span more than h, h = (volume / Nn)^(1/3)
 //   rows     the tile of a row is that of its edge's lower node; rows sorted by tile (stable),
-//            tiles cut into blocks of at most kTileMaxNnz nonzeros and kTileMaxInc incidences
+//            tiles cut into blocks of at most kTileMaxNnz nonzeros, kTileMaxInc incidences and
+//            kTileMaxRows rows
 //   records  the incidences sorted by (block, element): one record per group
 //   colours  per block, one CTA: which records share an off-diagonal slot, a two-colouring of
 //            that graph by label propagation (smallest record of the component, parity of the
@@ -289,7 +290,7 @@ __global__ void k_cut_tiles(int64_t ntiles, int64_t ndof, const uint32_t *__rest
         int64_t lo = k + 1, hi = k1;  // the last end that fits (one row always does)
         while (lo < hi) {
             const int64_t mid = (lo + hi + 1) >> 1;
-            if (pn[mid] - pn[k] <= kTileMaxNnz && pi[mid] - pi[k] <= kTileMaxInc) lo = mid;
+            if (pn[mid] - pn[k] <= kTileMaxNnz && pi[mid] - pi[k] <= kTileMaxInc && mid - k <= kTileMaxRows) lo = mid;
             else hi = mid - 1;
         }
         k = lo;

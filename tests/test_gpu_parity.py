@@ -826,6 +826,46 @@ def test_tile_plan_forms(oracle_port, form):
     plan.check()
 
 
+@pytest.mark.parametrize("where", ["end", "middle"])
+def test_tile_schedule_with_a_long_run_of_unused_dofs(oracle_port, where):
+    """50,000 dofs without an element (another field's unknowns in the same numbering) in one run:
+    every assembly of the tile schedule equals the oracle's, and the other rows are zero."""
+    from magpackage_b200.hbfem import AFT, assemble_hbfem
+
+    mesh = synth.kuhn_box(9, 8, 7, seed=4)
+    tags = synth.cube_layout(mesh)
+    edges, t2e, sign = oracle_port.generate_edges(mesh.T)
+    E, extra = edges.shape[0], 50000
+    n = E + extra
+    dofs = t2e if where == "end" else np.where(t2e < E // 2, t2e, t2e + extra).astype(t2e.dtype)
+    m = mex_inputs(mesh.P, mesh.T, dofs, sign, tags)
+    pk = material.pack_material_data(synth.standard_materials())
+    plan = AssemblyPlan(mesh.P, mesh.T, dofs, n, tags, sign)
+    plan.set_materials(pk)
+    assert plan.info.schedule == _lib.SCHEDULE_TILE_BLOCKS
+    rng = np.random.default_rng(8)
+    sol = rng.normal(0, 0.05, n)
+    qw, val, curl = quadrature.reference_data(2)
+    I, J, V, Ri, Rv = oracle_port.jacobian(m, sol, qw, curl, pk, True)
+    vals, res = plan.jacobian(dev(sol))
+    assert_csr_equal(plan.row_ptr, plan.col_idx, vals, oracle_matrix(oracle_port, I, J, V, n, False))
+    assert bits_equal(host(res), oracle_port.sparse_vec(Ri, Rv, n))
+    nu = rng.uniform(0.5, 2.0, mesh.num_elements)
+    Ik, Jk, Vk = oracle_port.curl_curl(m, nu, qw, curl)
+    assert_csr_equal(plan.row_ptr, plan.col_idx, plan.stiffness(dev(nu)), oracle_matrix(oracle_port, Ik, Jk, Vk, n, False))
+    Im, Jm, Vm = oracle_port.mass(m, nu, qw, val)
+    assert_csr_equal(plan.row_ptr, plan.col_idx, plan.mass(dev(nu)), oracle_matrix(oracle_port, Im, Jm, Vm, n, False))
+    aft = AFT((1, 3), n_time_steps=16)
+    hsol = 0.05 * (rng.normal(size=(n, 2)) + 1j * rng.normal(size=(n, 2)))
+    Ih, Jh, Vh, Rr, Rc, Rre, Rim = oracle_port.hbfem(m, hsol, aft.D, aft.P, qw, curl, pk, True)
+    R, hvals = assemble_hbfem(plan, hsol, aft, True)
+    R, lin, first = host(R), Rr + (Rc - 1) * n, Ih <= n
+    assert bits_equal(np.real(R), oracle_port.sparse_vec(lin, Rre, n * 2).reshape(2, n))
+    assert bits_equal(np.imag(R), oracle_port.sparse_vec(lin, Rim, n * 2).reshape(2, n))
+    assert_csr_equal(plan.row_ptr, plan.col_idx, hvals, oracle_matrix(oracle_port, Ih[first], Jh[first], Vh[first], n, False))
+    plan.check()
+
+
 @pytest.mark.parametrize("nrows,longest,zeros", [(1, 3, 0.0), (31, 20, 1.0), (32, 33, 0.3), (33, 255, 0.5), (1000, 19, 0.1),
                                                  (200001, 7, 0.4), (262145, 40, 0.05)])
 def test_drop_zeros_of_any_csr(nrows, longest, zeros):
