@@ -715,13 +715,12 @@ int launch_rows_reduce(const RowPlan &rp, int max_row, const double *scratch, do
     const int b = 128;
     unsigned g = blocks(rp.ndof, b);
     size_t smem = vals ? (size_t)b * max_row * sizeof(double) : 0;
-    if (smem > 200 * 1024) return MAG_E_UNSUPPORTED;
+    if (smem > (size_t)kMaxDynSmem) return MAG_E_UNSUPPORTED;
     bool mat = vals != nullptr, v = vec != nullptr;
 #define MAG_P2(M, V, W)                                                                          \
     do {                                                                                         \
         auto kern = k_rows_reduce<M, V, W>;                                                      \
-        if (smem > 48 * 1024)                                                                    \
-            cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);  \
+        if (smem > 48 * 1024 && !allow_max_smem((const void *)kern)) return MAG_E_CUDA;          \
         kern<<<g, b, smem, s>>>(rp, scratch, vals, vec);                                         \
     } while (0)
     if (rp.wide) {

@@ -36,6 +36,17 @@ constexpr int kScratchPerElem = 6 * kScratchStride;
 constexpr int kCompactMaxRow = 31;   // 5-bit in-row positions; 31 marks "no dof"
 constexpr int kWideMaxRow = 255;     // 8-bit positions; 255 marks "no dof"
 
+// Dynamic shared memory of a block, at most, of the kernels whose launches ask for different
+// amounts. The limit set on a kernel is one for the whole process: set to each launch's own size, a
+// thread with a smaller mesh could lower it between another thread's setting and its launch, which
+// then failed. So it is always set to the same value.
+constexpr int kMaxDynSmem = 200 * 1024;
+inline bool allow_max_smem(const void *kern) {
+    if (cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, kMaxDynSmem) == cudaSuccess) return true;
+    cudaGetLastError();
+    return false;
+}
+
 // Local edges (1,2),(1,3),(1,4),(2,3),(2,4),(3,4) of src/Mesh.m:118.
 __host__ __device__ constexpr int edge_a(int k) { return k < 3 ? 0 : (k < 5 ? 1 : 2); }
 __host__ __device__ constexpr int edge_b(int k) { return k == 0 ? 1 : (k == 1 || k == 3) ? 2 : 3; }

@@ -174,7 +174,6 @@ constexpr int kHbElems = 32;
 constexpr int kHbThreads = 6 * kHbElems;
 constexpr int kHbSamples = 3;
 constexpr int kHbGroup = 8;
-constexpr size_t kHbMaxSmem = 200 * 1024;
 
 // Shared memory: curls and weight [19][32]; harmonic values [6][2K][32], reused for nu (NT > 0)
 // and the results; D and P [4K][np]; then v [np][6][32] (NT > 0) or H [np][3][32] and nu [np][32].
@@ -472,8 +471,7 @@ namespace {
 template <int NT>
 int launch_hb_std(const HbArgs &A, size_t smem, cudaStream_t s) {
     auto kern = k_hbfem_std<NT>;
-    if (cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem) != cudaSuccess)
-        return MAG_E_CUDA;
+    if (!allow_max_smem((const void *)kern)) return MAG_E_CUDA;
     kern<<<(unsigned)((A.m.ne + kHbElems - 1) / kHbElems), 6 * kHbElems, smem, s>>>(A);
     return cudaPeekAtLastError() == cudaSuccess ? MAG_OK : MAG_E_CUDA;
 }
@@ -482,7 +480,7 @@ int launch_hb_std(const HbArgs &A, size_t smem, cudaStream_t s) {
 
 bool hbfem_constant_curls(const QuadParams &qp, int K, int N) {
     const int nt = N <= 16 ? 16 : N <= 24 ? 24 : N <= 32 ? 32 : 0;
-    return qp.standard_curl && qp.uniform_w && hb_smem_bytes(K, N, nt) <= kHbMaxSmem;
+    return qp.standard_curl && qp.uniform_w && hb_smem_bytes(K, N, nt) <= (size_t)kMaxDynSmem;
 }
 
 int launch_hbfem(const ElemData &m, const RowPlan &rp, int max_row, const double *sr, const double *si, int K,

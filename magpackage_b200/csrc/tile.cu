@@ -657,7 +657,7 @@ namespace {
 // A block at every limit of the plan (a chunk has a row that owns it, or lies inside one), with the
 // mass kernels' basis values, fits a CTA.
 static_assert((kTileMaxNnz + 1 + kTileSlotPad) * 8 + kTileMaxInc * 16 +
-                      (2 * kTileMaxRows + kTileMaxNnz / kTileChunk + 1) * 8 + 18 * kMaxQuad * 8 <= 227 * 1024,
+                      (2 * kTileMaxRows + kTileMaxNnz / kTileChunk + 1) * 8 + 18 * kMaxQuad * 8 <= kMaxDynSmem,
               "a block's shared memory");
 
 // Shared memory of one CTA: the block's values (an even count of doubles), the incidence
@@ -675,8 +675,7 @@ size_t tile_smem_bytes(const TilePlan &tp, TileArgs *a) {
 // far ahead a CTA prefetches).
 int resident_ctas(const void *kern, int threads, size_t smem, int *out) {
     int dev = 0, nsm = 0, per = 0;
-    if (cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem) != cudaSuccess ||
-        cudaGetDevice(&dev) != cudaSuccess ||
+    if (!allow_max_smem(kern) || cudaGetDevice(&dev) != cudaSuccess ||
         cudaDeviceGetAttribute(&nsm, cudaDevAttrMultiProcessorCount, dev) != cudaSuccess ||
         cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per, kern, threads, smem) != cudaSuccess || per < 1)
         return MAG_E_CUDA;

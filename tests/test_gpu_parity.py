@@ -866,6 +866,49 @@ def test_tile_schedule_with_a_long_run_of_unused_dofs(oracle_port, where):
     plan.check()
 
 
+def test_meshes_of_different_block_sizes_from_several_threads():
+    """Handles whose launches need different amounts of shared memory, each used by a thread of its
+    own: every call succeeds and gives what it gives alone."""
+    import threading
+
+    from magpackage_b200.hbfem import AFT, assemble_hbfem
+
+    calls, want = [], []
+    for n, harmonics, samples in ((1, (1,), 8), (12, (1, 3, 5, 7), 32), (5, (1,), 16), (24, (1, 3), 24)):
+        mesh = synth.kuhn_box(n, seed=n)
+        edges, t2e, sign = generate_edges(mesh.T)
+        plan = AssemblyPlan(mesh.P, mesh.T, t2e, int(edges.shape[0]), synth.cube_layout(mesh), sign)
+        plan.set_materials(material.pack_material_data(synth.standard_materials()))
+        g = torch.Generator(device="cuda").manual_seed(n)
+        sol = 1e-3 * torch.randn(plan.num_dofs, dtype=torch.float64, device="cuda", generator=g)
+        pair = tuple(1e-3 * torch.randn((len(harmonics), plan.num_dofs), dtype=torch.float64, device="cuda", generator=g)
+                     for _ in range(2))
+        aft = AFT(harmonics, n_time_steps=samples)
+        aft.device_operators()
+        calls.append(lambda p=plan, x=sol, y=pair, a=aft: p.jacobian(x) + (p.mass(),) + assemble_hbfem(p, y, a))
+        want.append(calls[-1]())
+    torch.cuda.synchronize()
+    wrong = []
+
+    def work(k):
+        try:
+            with torch.cuda.stream(torch.cuda.Stream()):
+                for _ in range(400):
+                    got = calls[k]()
+                torch.cuda.current_stream().synchronize()
+            if not all(torch.equal(a, b) for a, b in zip(got, want[k])):
+                wrong.append((k, "outputs differ"))
+        except _lib.MagError as e:
+            wrong.append((k, str(e)))
+
+    threads = [threading.Thread(target=work, args=(k,)) for k in range(len(calls))]
+    for t in threads:
+        t.start()
+    for t in threads:
+        t.join()
+    assert not wrong
+
+
 @pytest.mark.parametrize("nrows,longest,zeros", [(1, 3, 0.0), (31, 20, 1.0), (32, 33, 0.3), (33, 255, 0.5), (1000, 19, 0.1),
                                                  (200001, 7, 0.4), (262145, 40, 0.05)])
 def test_drop_zeros_of_any_csr(nrows, longest, zeros):
