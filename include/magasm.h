@@ -98,7 +98,14 @@ const char *mag_last_error(void);
 /* Threading. Every handle-based entry point only enqueues work on its stream and
  * returns; mag_sync waits for the stream (MAG_E_CUDA with the CUDA error text if
  * work on it failed). Different handles may be used from different host threads at
- * once; one handle is used by one thread at a time. The MEX entry points run one at
+ * once. The mag_assemble_* calls of one mesh handle may come from several threads and
+ * go to several streams: calls that share a buffer of the handle take turns at it, on
+ * the host and on the device. Everything else that takes a handle (set, tune, check,
+ * create, destroy, and the batch, PCG and MLP handles) is used by one thread at a time,
+ * with no other call of that handle under way. A captured call of
+ * mag_assemble_source, and any captured call that runs as two passes, uses the
+ * handle's scratch when the graph is replayed: the caller orders such replays with
+ * each other and with direct calls of the same kind. The MEX entry points run one at
  * a time (they share the mesh cache and the staging buffers) and return with their
  * outputs on the host, as the reference's gateways do (they are single-threaded
  * callees of MATLAB: assemble_jacobian_kernel_mex.cpp:8-153). */

@@ -340,6 +340,7 @@ struct mag_mesh {
     int max_tag = 0;
     PatternBuffers pat;
     double *scratch = nullptr;
+    cudaEvent_t scratch_done = nullptr;  // after its last use
     QuadParams qp{};
     double *d_ref = nullptr;
     MaterialStore mat;
@@ -352,7 +353,7 @@ struct mag_mesh {
     int schedule = MAG_SCHEDULE_ROW_BLOCKS;
     double *fres = nullptr;            // [Ne][6] residual entries (NULL: residuals by the tile kernel)
     cudaEvent_t fres_done = nullptr;   // after its last use
-    std::mutex turn;                   // threads that enqueue a use of fres, or make the pool
+    std::mutex turn;                   // threads that enqueue a use of fres or scratch, or make the pool
     cudaMemPool_t pool = nullptr;  // workspaces of single calls (NULL: the device's default pool)
     int64_t bytes = 0;
 
@@ -376,6 +377,7 @@ void destroy_mesh(mag_mesh *m) {
     free_rowblock_plan(&m->rowshared);
     cudaDeviceSynchronize();
     if (m->fres_done) cudaEventDestroy(m->fres_done);
+    if (m->scratch_done) cudaEventDestroy(m->scratch_done);
     if (m->pool) cudaMemPoolDestroy(m->pool);
     delete m;
 }
@@ -463,6 +465,22 @@ bool residual_begin(mag_mesh *m, cudaStream_t s) {
         return true;
     cudaGetLastError();
     return false;
+}
+
+// enqueue() uses the handle's element scratch on stream s. Calls from different threads and on
+// different streams take turns at it, as at the residual entries above: without that, the second
+// call's elements overwrote entries which the first one's row sums had yet to read. Inside a stream
+// capture the order is the caller's (a graph cannot wait for an event of other streams' calls).
+template <typename F>
+int with_scratch(mag_mesh *m, cudaStream_t s, F enqueue) {
+    cudaStreamCaptureStatus cap = cudaStreamCaptureStatusNone;
+    MAG_CUDA_TRY(cudaStreamIsCapturing(s, &cap));
+    if (cap != cudaStreamCaptureStatusNone) return enqueue();
+    std::lock_guard<std::mutex> lk(m->turn);
+    MAG_CUDA_TRY(cudaStreamWaitEvent(s, m->scratch_done, 0));
+    const int rc = enqueue();
+    MAG_CUDA_TRY(cudaEventRecord(m->scratch_done, s));  // also after a failure: a first kernel may run
+    return rc;
 }
 
 int finish(cudaStream_t s) {
@@ -577,6 +595,7 @@ int mag_mesh_create(const double *d_P, int64_t Nn, const int32_t *d_T, int64_t N
         set_error("mag_mesh_create: out of device memory for the element scratch");
         return fail(MAG_E_NOMEM);
     }
+    if (cudaEventCreateWithFlags(&m->scratch_done, cudaEventDisableTiming) != cudaSuccess) return fail(MAG_E_CUDA);
     m->bytes += (int64_t)Ne * kScratchPerElem * 8;
     // optional schedules; the two-pass kernels always work
     if (build_rowblock_plan(m->rows(), &m->rowblock, s) == MAG_OK) {
@@ -721,8 +740,10 @@ int mag_assemble_jacobian(mag_mesh *m, const double *d_sol, double *d_vals, doub
                                          calc_j ? d_vals : nullptr, d_res, s));
         return finish(s);
     }
-    MAG_TRY(launch_jacobian_elems(m->elems(), d_sol, m->qp, m->mat.mp, calc_j, m->scratch, s));
-    MAG_TRY(launch_rows_reduce(m->rows(), m->pat.max_row, m->scratch, calc_j ? d_vals : nullptr, d_res, s));
+    MAG_TRY(with_scratch(m, s, [&] {
+        MAG_TRY(launch_jacobian_elems(m->elems(), d_sol, m->qp, m->mat.mp, calc_j, m->scratch, s));
+        return launch_rows_reduce(m->rows(), m->pat.max_row, m->scratch, calc_j ? d_vals : nullptr, d_res, s);
+    }));
     return finish(s);
 }
 
@@ -742,8 +763,10 @@ int mag_assemble_stiffness(mag_mesh *m, const double *d_nu, double *d_vals, void
         MAG_TRY(launch_rowblock_nz_stiffness(m->rowshared, m->elems(), m->rows(), d_nu, m->qp, d_vals, s));
         return finish(s);
     }
-    MAG_TRY(launch_stiffness_elems(m->elems(), d_nu, m->qp, m->scratch, s));
-    MAG_TRY(launch_rows_reduce(m->rows(), m->pat.max_row, m->scratch, d_vals, nullptr, s));
+    MAG_TRY(with_scratch(m, s, [&] {
+        MAG_TRY(launch_stiffness_elems(m->elems(), d_nu, m->qp, m->scratch, s));
+        return launch_rows_reduce(m->rows(), m->pat.max_row, m->scratch, d_vals, nullptr, s);
+    }));
     return finish(s);
 }
 
@@ -764,8 +787,10 @@ int mag_assemble_jacobian_seeded(mag_mesh *m, const double *d_sol, const double 
                                    s));
         return finish(s);
     }
-    MAG_TRY(launch_jacobian_seeded_elems(m->elems(), d_sol, d_bscale, m->qp, m->mat.mp, m->scratch, s));
-    MAG_TRY(launch_rows_reduce(m->rows(), m->pat.max_row, m->scratch, d_vals, d_res, s));
+    MAG_TRY(with_scratch(m, s, [&] {
+        MAG_TRY(launch_jacobian_seeded_elems(m->elems(), d_sol, d_bscale, m->qp, m->mat.mp, m->scratch, s));
+        return launch_rows_reduce(m->rows(), m->pat.max_row, m->scratch, d_vals, d_res, s);
+    }));
     return finish(s);
 }
 
@@ -789,8 +814,11 @@ int mag_assemble_hbfem(mag_mesh *m, const double *d_sol_re, const double *d_sol_
     double *rscr = nullptr;
     MAG_TRY(workspace(m, (nres + (tile_dc ? (size_t)m->ne : 0)) * sizeof(double), s, &rscr));
     double *nu_dc = tile_dc ? rscr + nres : nullptr;
-    int rc = launch_hbfem(m->elems(), m->rows(), m->pat.max_row, d_sol_re, d_sol_im, K, d_d_re, d_d_im, d_p_re,
-                          d_p_im, N, m->qp, m->mat.mp, m->scratch, rscr, nu_dc, d_vals, d_res_re, d_res_im, s);
+    auto harmonics = [&] {
+        return launch_hbfem(m->elems(), m->rows(), m->pat.max_row, d_sol_re, d_sol_im, K, d_d_re, d_d_im, d_p_re,
+                            d_p_im, N, m->qp, m->mat.mp, m->scratch, rscr, nu_dc, d_vals, d_res_re, d_res_im, s);
+    };
+    int rc = d_vals && !tile_dc ? with_scratch(m, s, harmonics) : harmonics();  // (DC block rows in the scratch)
     if (rc == MAG_OK && tile_dc)
         rc = launch_tile_harmonic_dc(m->tile, m->elems(), nu_dc, m->qp, d_vals, m->status, s);
     cudaFreeAsync(rscr, s);
@@ -828,8 +856,10 @@ int mag_assemble_mass(mag_mesh *m, const double *d_sigma, double *d_vals, void *
         MAG_TRY(launch_tile_mass(m->tile, m->elems(), d_sigma, m->qp, d_vals, m->status, s));
         return finish(s);
     }
-    MAG_TRY(launch_mass_elems(m->elems(), d_sigma, m->qp, m->scratch, s));
-    MAG_TRY(launch_rows_reduce(m->rows(), m->pat.max_row, m->scratch, d_vals, nullptr, s));
+    MAG_TRY(with_scratch(m, s, [&] {
+        MAG_TRY(launch_mass_elems(m->elems(), d_sigma, m->qp, m->scratch, s));
+        return launch_rows_reduce(m->rows(), m->pat.max_row, m->scratch, d_vals, nullptr, s);
+    }));
     return finish(s);
 }
 
@@ -840,7 +870,9 @@ int mag_assemble_source(mag_mesh *m, const double *d_js, double *d_out, void *st
         return MAG_E_ARG;
     }
     cudaStream_t s = (cudaStream_t)stream;
-    MAG_TRY(launch_source(m->elems(), m->rows(), d_js, m->qp, m->scratch, d_out, s));
+    MAG_TRY(with_scratch(m, s, [&] {
+        return launch_source(m->elems(), m->rows(), d_js, m->qp, m->scratch, d_out, s);
+    }));
     return finish(s);
 }
 

@@ -222,3 +222,43 @@ def test_residuals_of_one_mesh_from_several_threads():
     for w, outs in zip(want, got):
         assert all(torch.equal(w, r) for r in outs)
     plan.check()
+
+
+@pytest.mark.parametrize("beside", ["source", "two_pass"])
+def test_sources_of_one_mesh_from_several_threads(beside):
+    """Threads with a stream each assemble source vectors of their own densities on one mesh handle,
+    or sources beside two-pass mass matrices (which use the same scratch); each gets its own result,
+    bit for bit."""
+    import threading
+
+    from magpackage_b200.plan import generate_edges
+
+    mesh = synth.kuhn_box(33, seed=2)
+    edges, t2e, sign = generate_edges(mesh.T)
+    plan = AssemblyPlan(mesh.P, mesh.T, t2e, int(edges.shape[0]), synth.cube_layout(mesh), sign)
+    g = torch.Generator(device="cuda").manual_seed(1)
+    js = [torch.randn((mesh.num_elements, 3), dtype=torch.float64, device="cuda", generator=g) for _ in range(4)]
+    calls = [lambda out, j=j: plan.source(j, out) for j in js]
+    outs = [[plan.new_vector() for _ in range(24)] for _ in js]
+    if beside == "two_pass":
+        plan.set_schedule(_lib.SCHEDULE_TWO_PASS)
+        for k in (1, 3):
+            calls[k] = lambda out, s=js[k][:, 0].abs().contiguous(): plan.mass(s, out)
+            outs[k] = [plan.new_values() for _ in range(24)]
+    want = [f(torch.empty_like(o[0])) for f, o in zip(calls, outs)]
+    torch.cuda.synchronize()
+
+    def work(f, mine):
+        with torch.cuda.stream(torch.cuda.Stream()):
+            for r in mine:
+                f(r)
+            torch.cuda.current_stream().synchronize()
+
+    threads = [threading.Thread(target=work, args=a) for a in zip(calls, outs)]
+    for t in threads:
+        t.start()
+    for t in threads:
+        t.join()
+    for w, mine in zip(want, outs):
+        assert float(w.abs().max()) > 0 and all(torch.equal(w, r) for r in mine)
+    plan.check()
