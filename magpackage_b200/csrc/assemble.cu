@@ -339,10 +339,16 @@ __global__ void __launch_bounds__(128) k_source_elems(ElemData m, const double *
     if (e >= m.ne) return;
     const double jp[3] = {js[3 * e], js[3 * e + 1], js[3 * e + 2]};
     double f[6] = {0, 0, 0, 0, 0, 0};
+    const bool on = fabs(jp[0]) > 1e-12 || fabs(jp[1]) > 1e-12 || fabs(jp[2]) > 1e-12;
+    // An element without a source gives 0 * sign, which is -0 on a reversed edge: the triplets keep
+    // it, the row sums (from +0) do not see it.
+    int4 t = make_int4(0, 0, 0, 0);
     unsigned sb = 0;
-    if (fabs(jp[0]) > 1e-12 || fabs(jp[1]) > 1e-12 || fabs(jp[2]) > 1e-12) {
-        const int4 t = m.tet[e];
+    if (on || !COMPACT) {
+        t = m.tet[e];
         sb = m.signbits ? m.signbits[e] : derived_signs(t);
+    }
+    if (on) {
         Geo g;
         geometry(m.xyz, t, g);
         double iv[3][3];

@@ -43,6 +43,28 @@ def test_mex_winding_and_source_match_golden(name):
     assert bits_equal(I, d["src_I"]) and bits_equal(V, d["src_V"])
 
 
+def test_mex_source_signs_of_zeros(oracle_port):
+    """f * sign of an element without a source is a zero with the edge's sign, as in the reference's
+    pairs (assemble_source_kernel_mex.cpp:46-114): signs of zeros included, every bit is the oracle's."""
+    mesh = synth.kuhn_box(3, 2, 4, seed=8)
+    edges, t2e, sign = oracle_port.generate_edges(mesh.T)
+    sign = sign.copy()
+    sign[::2] *= -1
+    m = mex_inputs(mesh.P, mesh.T, t2e, sign, synth.cube_layout(mesh))
+    qw, val, curl = quadrature.reference_data(2)
+    js = np.random.default_rng(8).normal(size=(m.ne, 3))
+    js[1::3] = 0.0
+    js[2::3] = 1e-13  # below the reference's cut-off
+    Io, Vo = oracle_port.source(m, js, qw, val)
+    I, V = np.ones(6 * m.ne), np.ones(6 * m.ne)
+    p = _lib.dptr
+    _lib.check(_lib.lib().mag_mex_source(p(m.P), m.nn, p(m.T), m.ne, p(m.Dofs), p(m.Signs), p(js), p(qw), qw.size,
+                                         p(val), p(I), p(V)))
+    assert np.array_equal(I, Io)
+    assert np.sum((Vo == 0) & np.signbit(Vo)) > 100
+    assert np.array_equal(V.view(np.int64), Vo.view(np.int64))
+
+
 def _vector(port, I, V, n):
     k = I > 0
     return port.sparse_vec(I[k], V[k], n)
