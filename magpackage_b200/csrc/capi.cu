@@ -809,7 +809,7 @@ int mag_assemble_hbfem(mag_mesh *m, const double *d_sol_re, const double *d_sol_
     cudaStream_t s = (cudaStream_t)stream;
     // the DC block is K(nu_dc): one launch of the tile kernel where the mesh has a tile plan
     const bool tile_dc = d_vals && m->schedule == MAG_SCHEDULE_TILE_BLOCKS && m->tile.ok &&
-                         hbfem_constant_curls(m->qp, K, N);
+                         hbfem_constant_curls(m->qp, K, N, m->ne, true);
     const size_t nres = (size_t)m->ne * 6 * 2 * K;
     double *rscr = nullptr;
     MAG_TRY(workspace(m, (nres + (tile_dc ? (size_t)m->ne : 0)) * sizeof(double), s, &rscr));

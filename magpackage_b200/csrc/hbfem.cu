@@ -1,15 +1,17 @@
 // Harmonic-balance (HBFEM) assembly, FP64 (sm_100a).
 //
-// Element phase (one thread per element) restates assemble_hbfem_kernel_mex.cpp:108-226
+// Element phase restates assemble_hbfem_kernel_mex.cpp:108-226
 // operation for operation: the signed harmonic edge values, per quadrature point the
 // physical curls, per time sample t the edge values A(t) = sum_h (Re A_h Re D(t,h) -
 // Im A_h Im D(t,h)), B(t), nu(|B(t)|^2) from the B-H table (with the coefficient offsets
 // the reference gateway forgets to set), H = nu B, and the harmonic residual
 // R_h += w (C_i . H) P(h,t); the Jacobian block is w nu_dc C_r . C_c with nu_dc the
-// time average of nu. Per (element, local row) it writes the signed block row into
-// the common element scratch (reduced by k_rows_reduce) and its 2K residual entries
-// into a second scratch that k_rows_reduce_harm sums per CSR row, in ascending element
-// order, as MATLAB's sparse() does with the gateway's triplets.
+// time average of nu. Two kernels: k_hbfem_std, six threads per element, for the standard curl
+// table with equal weights, and k_hbfem_elems, one thread per element, for any table, weights and
+// sample count. Per (element, local row) they write the 2K residual entries into a workspace that
+// k_rows_reduce_harm sums per CSR row, in ascending element order, as MATLAB's sparse() does with
+// the gateway's triplets. The DC block is one tile assembly from k_hbfem_std's nu_dc, or block rows
+// in the common element scratch (reduced by k_rows_reduce).
 #include "assemble.cuh"
 #include "common.cuh"
 #include "element.cuh"
@@ -38,14 +40,18 @@ struct HbArgs {
 // Index of (r, c), r <= c, in the upper triangle of a 6 x 6 block stored row by row.
 __host__ __device__ constexpr int kb_at(int r, int c) { return r * 6 - r * (r - 1) / 2 + (c - r); }
 
-// General form, one thread per element: any curl table, any weights, any sample count
-// (harmonic arrays sized for kMaxHarm, in local memory).
-template <bool CALCJ>
-__global__ void __launch_bounds__(128, 3) k_hbfem_elems(HbArgs A) {
-    constexpr int KA = kMaxHarm;
+// General form, one thread per element: any curl table, any weights, any sample count. KC: the
+// harmonic count as a compile-time constant, so that the harmonic loops unroll and their arrays are
+// registers (up to 255, two CTAs per SM); 0: A.K at run time, arrays sized for kMaxHarm in local
+// memory. Measured, ms, residual and DC block of 384,000 elements with run-time / constant count: 3
+// harmonics, 256 samples 24.4 / 11.0, 32 samples with unequal weights 3.25 / 1.89; 1 harmonic, 256
+// samples 9.03 / 4.68.
+template <bool CALCJ, int KC>
+__global__ void __launch_bounds__(128, KC > 0 ? 2 : 3) k_hbfem_elems(HbArgs A) {
+    constexpr int KA = KC > 0 ? KC : kMaxHarm;
     const int64_t e = blockIdx.x * (int64_t)blockDim.x + threadIdx.x;
     if (e >= A.m.ne) return;
-    const int K = A.K, N = A.N;
+    const int K = KC > 0 ? KC : A.K, N = A.N;
     const int4 tt = A.m.tet[e];
     int d[6];
     load_dofs(A.m.dofs, e, d);
@@ -478,10 +484,30 @@ int launch_hb_std(const HbArgs &A, size_t smem, cudaStream_t s) {
 
 }  // namespace
 
-bool hbfem_constant_curls(const QuadParams &qp, int K, int N) {
+// With more samples than the register forms hold, k_hbfem_std<0> forms v(t) again for every group of
+// sums: for one or two harmonics the general kernel, compiled for the count, is then the faster one
+// once its one thread per element fills the GPU. Measured, us, constant-curl / general kernel: 1
+// harmonic, 64 samples, residual and DC block at 29,478 elements 166 / 235, 48,000 252 / 252, 82,944
+// 401 / 346, 384,000 1825 / 1440, residual alone at 29,478 155 / 212, 48,000 239 / 225; 2 harmonics, residual alone, 33 samples at 82,944 elements 252 / 287, 196,608 599 /
+// 552, 663,552 2025 / 1751, 160 samples there 7257 / 7159; with the DC block, 64 samples, 3428 / 3502.
+bool hbfem_constant_curls(const QuadParams &qp, int K, int N, int64_t ne, bool dc) {
     const int nt = N <= 16 ? 16 : N <= 24 ? 24 : N <= 32 ? 32 : 0;
-    return qp.standard_curl && qp.uniform_w && hb_smem_bytes(K, N, nt) <= (size_t)kMaxDynSmem;
+    if (!qp.standard_curl || !qp.uniform_w || hb_smem_bytes(K, N, nt) > (size_t)kMaxDynSmem) return false;
+    if (nt == 0 && K == 1 && ne >= (dc ? 60000 : 45000)) return false;
+    if (nt == 0 && K == 2 && !dc && N <= 128 && ne >= 190000) return false;
+    return true;
 }
+
+namespace {
+
+template <int KC>
+void launch_hb_elems(const HbArgs &A, bool rows, cudaStream_t s) {
+    const unsigned g = (unsigned)((A.m.ne + 127) / 128);
+    if (rows) k_hbfem_elems<true, KC><<<g, 128, 0, s>>>(A);
+    else k_hbfem_elems<false, KC><<<g, 128, 0, s>>>(A);
+}
+
+}  // namespace
 
 int launch_hbfem(const ElemData &m, const RowPlan &rp, int max_row, const double *sr, const double *si, int K,
                  const double *dr, const double *di, const double *pr, const double *pi, int N,
@@ -489,7 +515,7 @@ int launch_hbfem(const ElemData &m, const RowPlan &rp, int max_row, const double
                  double *vals, double *out_re, double *out_im, cudaStream_t s) {
     const bool rows = vals && !nu_dc;  // DC block rows through the element scratch
     HbArgs A{m, sr, si, dr, di, pr, pi, K, N, rp.ndof, qp, mp, rows ? scratch : nullptr, rscr, nu_dc};
-    if (hbfem_constant_curls(qp, K, N)) {
+    if (hbfem_constant_curls(qp, K, N, m.ne, vals != nullptr)) {
         const int nt = N <= 16 ? 16 : N <= 24 ? 24 : N <= 32 ? 32 : 0;
         const size_t smem = hb_smem_bytes(K, N, nt);
         MAG_TRY(nt == 16   ? launch_hb_std<16>(A, smem, s)
@@ -497,9 +523,13 @@ int launch_hbfem(const ElemData &m, const RowPlan &rp, int max_row, const double
                 : nt == 32 ? launch_hb_std<32>(A, smem, s)
                            : launch_hb_std<0>(A, smem, s));
     } else {
-        const unsigned g = (unsigned)((m.ne + 127) / 128);
-        if (rows) k_hbfem_elems<true><<<g, 128, 0, s>>>(A);
-        else k_hbfem_elems<false><<<g, 128, 0, s>>>(A);
+        switch (K) {
+            case 1: launch_hb_elems<1>(A, rows, s); break;
+            case 2: launch_hb_elems<2>(A, rows, s); break;
+            case 3: launch_hb_elems<3>(A, rows, s); break;
+            case 4: launch_hb_elems<4>(A, rows, s); break;
+            default: launch_hb_elems<0>(A, rows, s);
+        }
         if (cudaPeekAtLastError() != cudaSuccess) return MAG_E_CUDA;
     }
     const int64_t nt = rp.ndof * 2 * K;

@@ -9,9 +9,9 @@ namespace mag {
 
 constexpr int kMaxHarm = 16;  // harmonics per call
 
-// Whether the constant-curl kernel serves these tables and sample count (it can also hand
-// back the time-averaged reluctivity, from which the DC block is one stiffness assembly).
-bool hbfem_constant_curls(const QuadParams &qp, int K, int N);
+// Whether the constant-curl kernel serves this call (it can also hand back the time-averaged
+// reluctivity, from which the DC block is one stiffness assembly). dc: the DC block is wanted.
+bool hbfem_constant_curls(const QuadParams &qp, int K, int N, int64_t ne, bool dc);
 
 // Residual (and, when vals is given, the DC block) of one harmonic field. rscr: [Ne][6][2K]
 // workspace. nu_dc [Ne], only with hbfem_constant_curls: receives the time-averaged

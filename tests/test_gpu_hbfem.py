@@ -116,3 +116,44 @@ def test_hbfem_sample_counts_and_weights(oracle_port, harmonics, samples, weight
     first = I <= E
     _, _, rv = oracle_port.sparse_csr(I[first], J[first], V[first], E, drop_zeros=False)
     assert bits_equal(vals.cpu().numpy(), rv)
+
+
+@pytest.mark.parametrize("harmonics,samples,weights,n", [
+    ((1,), 256, "equal", (1, 1, 59)),            # more samples than the constant-curl kernel's shared memory
+    ((1, 3), 256, "equal", (1, 1, 59)),          # holds: the general kernel compiled for 1 to 4 harmonics
+    ((1, 3, 5), 256, "equal", (1, 1, 59)),
+    ((0, 1, 3, 5), 256, "equal", (1, 1, 59)),
+    ((1, 3, 5, 7, 9), 256, "equal", (1, 1, 59)),  # and with the count at run time
+    ((1,), 32, "uneven", (1, 1, 59)),
+    ((1, 3, 5), 32, "uneven", (1, 1, 59)),
+    ((0, 1, 3, 5), 17, "uneven", (1, 1, 59)),
+    ((1,), 33, "equal", (22, 22, 21)),           # one harmonic on 60,984 elements: general kernel
+])
+def test_hbfem_general_kernel(oracle_port, harmonics, samples, weights, n):
+    """The general element kernel against the oracle, with and without the DC block."""
+    plan, m, pk, sol, E = _case(oracle_port, harmonics, n=n, seed=4)
+    aft = AFT(harmonics, n_time_steps=samples)
+    assert aft.num_time_steps == samples
+    qw, val, curl = quadrature.reference_data(2)
+    if weights == "uneven":
+        qw = qw * np.array([1.0, 0.5, 1.25, 1.25])
+        plan.set_quadrature(qw, curl, val)
+    K = len(harmonics)
+    I, J, V, Rr, Rc, Rre, Rim = oracle_port.hbfem(m, sol, aft.D, aft.P, qw, curl, pk, True)
+    R, vals = assemble_hbfem(plan, sol, aft, True)
+    assert torch.equal(assemble_hbfem(plan, sol, aft, False)[0], R)
+    R = R.cpu().numpy()
+    lin = Rr + (Rc - 1) * E
+    assert bits_equal(np.real(R), oracle_port.sparse_vec(lin, Rre, E * K).reshape(K, E))
+    assert bits_equal(np.imag(R), oracle_port.sparse_vec(lin, Rim, E * K).reshape(K, E))
+    first = I <= E
+    _, _, rv = oracle_port.sparse_csr(I[first], J[first], V[first], E, drop_zeros=False)
+    assert bits_equal(vals.cpu().numpy(), rv)
+
+
+def test_hbfem_both_kernels_give_the_same_bits(oracle_port):
+    """Two harmonics on 196,608 elements: a residual alone takes the general kernel, one with the DC
+    block the constant-curl kernel."""
+    plan, m, pk, sol, E = _case(oracle_port, (1, 3), n=(32, 32, 32), seed=5)
+    aft = AFT((1, 3), n_time_steps=33)
+    assert torch.equal(assemble_hbfem(plan, sol, aft, False)[0], assemble_hbfem(plan, sol, aft, True)[0])
