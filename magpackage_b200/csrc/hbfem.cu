@@ -445,6 +445,9 @@ __global__ void __launch_bounds__(kHbThreads, NT > 0 ? 3 : 1) k_hbfem_std(HbArgs
                 if (cb + j < W) out[cb + j] = acc[j];
         }
     }
+    // without Im P the imaginary sums are +0 whatever the samples hold (0 x infinity is NaN)
+    if (!A.pi)
+        for (int c = K; c < W; c++) out[c] = 0.0;
     __syncthreads();
     const int64_t left = A.m.ne - e0;
     const int count = (int)(left < kHbElems ? left : kHbElems) * 6 * W;
@@ -488,8 +491,9 @@ int launch_hb_std(const HbArgs &A, size_t smem, cudaStream_t s) {
 // sums: for one or two harmonics the general kernel, compiled for the count, is then the faster one
 // once its one thread per element fills the GPU. Measured, us, constant-curl / general kernel: 1
 // harmonic, 64 samples, residual and DC block at 29,478 elements 166 / 235, 48,000 252 / 252, 82,944
-// 401 / 346, 384,000 1825 / 1440, residual alone at 29,478 155 / 212, 48,000 239 / 225; 2 harmonics, residual alone, 33 samples at 82,944 elements 252 / 287, 196,608 599 /
-// 552, 663,552 2025 / 1751, 160 samples there 7257 / 7159; with the DC block, 64 samples, 3428 / 3502.
+// 401 / 346, 384,000 1825 / 1440, residual alone at 29,478 155 / 212, 48,000 239 / 225; 2 harmonics,
+// residual alone, 33 samples at 82,944 elements 252 / 287, 196,608 599 / 552, 663,552 2025 / 1751,
+// 160 samples there 7257 / 7159; with the DC block, 64 samples, 3428 / 3502.
 bool hbfem_constant_curls(const QuadParams &qp, int K, int N, int64_t ne, bool dc) {
     const int nt = N <= 16 ? 16 : N <= 24 ? 24 : N <= 32 ? 32 : 0;
     if (!qp.standard_curl || !qp.uniform_w || hb_smem_bytes(K, N, nt) > (size_t)kMaxDynSmem) return false;

@@ -157,3 +157,31 @@ def test_hbfem_both_kernels_give_the_same_bits(oracle_port):
     plan, m, pk, sol, E = _case(oracle_port, (1, 3), n=(32, 32, 32), seed=5)
     aft = AFT((1, 3), n_time_steps=33)
     assert torch.equal(assemble_hbfem(plan, sol, aft, False)[0], assemble_hbfem(plan, sol, aft, True)[0])
+
+
+@pytest.mark.parametrize("samples", [9, 20, 32, 40, 256])
+def test_hbfem_real_transform_of_an_infinite_field(oracle_port, samples):
+    """Without Im P the imaginary residual is zero, also where a field value is infinite and its
+    samples are infinities and NaN; entries the value does not reach keep the finite field's bits."""
+    import ctypes as C
+
+    from magpackage_b200 import _lib
+
+    harmonics = (0, 1, 2)
+    plan, m, pk, sol, E = _case(oracle_port, harmonics, n=(3, 2, 3), seed=6)
+    dr, di, pr, _ = AFT(harmonics, n_time_steps=samples).device_operators()
+    K, res = len(harmonics), []
+    for bad in (False, True):
+        sr = torch.as_tensor(np.ascontiguousarray(sol.real.T), device="cuda")
+        si = torch.as_tensor(np.ascontiguousarray(sol.imag.T), device="cuda")
+        if bad:
+            sr[1, 5] = float("inf")
+        re, im = torch.full_like(sr, 7.0), torch.full_like(sr, 7.0)
+        p = lambda t: C.c_void_p(t.data_ptr())
+        _lib.check(_lib.lib().mag_assemble_hbfem(plan._h, p(sr), p(si), K, p(dr), p(di), p(pr), None, samples, None,
+                                                 p(re), p(im), _lib.stream_ptr()))
+        assert torch.count_nonzero(im) == 0
+        res.append(re)
+    bad = ~torch.isfinite(res[1])
+    assert 0 < int(bad[0].sum()) < E
+    assert torch.equal(res[0][~bad], res[1][~bad])
