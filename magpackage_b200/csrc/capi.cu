@@ -351,9 +351,7 @@ struct mag_mesh {
     TilePlan tile;              // spatial-tile blocks (default schedule)
     int *status = nullptr;      // device word: a tile kernel skipped an out-of-range plan index
     int schedule = MAG_SCHEDULE_ROW_BLOCKS;
-    double *fres = nullptr;            // [Ne][6] residual entries (NULL: residuals by the tile kernel)
-    cudaEvent_t fres_done = nullptr;   // after its last use
-    std::mutex turn;                   // threads that enqueue a use of fres or scratch, or make the pool
+    std::mutex turn;                   // threads that enqueue a use of scratch, or make the pool
     cudaMemPool_t pool = nullptr;  // workspaces of single calls (NULL: the device's default pool)
     int64_t bytes = 0;
 
@@ -368,7 +366,7 @@ namespace {
 void destroy_mesh(mag_mesh *m) {
     if (!m) return;
     void *ptrs[] = {m->xyz, m->tet, m->dofs, m->tags, m->signbits, m->scratch, m->d_ref, m->mat.mem, m->second,
-                    m->status, m->fres};
+                    m->status};
     for (void *p : ptrs)
         if (p) cudaFree(p);
     free_pattern(&m->pat, nullptr);
@@ -376,7 +374,6 @@ void destroy_mesh(mag_mesh *m) {
     free_rowblock_plan(&m->rowblock);
     free_rowblock_plan(&m->rowshared);
     cudaDeviceSynchronize();
-    if (m->fres_done) cudaEventDestroy(m->fres_done);
     if (m->scratch_done) cudaEventDestroy(m->scratch_done);
     if (m->pool) cudaMemPoolDestroy(m->pool);
     delete m;
@@ -437,40 +434,25 @@ int workspace(mag_mesh *m, size_t bytes, cudaStream_t s, double **p) {
 }
 
 // A residual alone: from this many elements on one evaluation per element and a gather per row
-// (two launches, 48 bytes an element of workspace) beat the tile kernel's 1.5 evaluations, below
+// (two launches, 48 bytes an element of the scratch) beat the tile kernel's 1.5 evaluations, below
 // it the tile kernel's one launch wins. Measured, us, tile / two launches: 27,000 hexahedra
 // (162,000 elements) 17.9 / 19.0, 39,304 21.0 / 18.8, 74,088 33.4 / 26.7, 216,000 97 / 67.
 constexpr int64_t kResidualElems = 200000;
 
-void make_residual_buffer(mag_mesh *m) {
-    if (!m->tile.ok || m->ne < kResidualElems) return;
-    const size_t b = (size_t)m->ne * 6 * sizeof(double);
-    if (cudaEventCreateWithFlags(&m->fres_done, cudaEventDisableTiming) != cudaSuccess ||
-        cudaMalloc(&m->fres, b) != cudaSuccess) {
-        cudaGetLastError();
-        m->fres = nullptr;  // the tile kernel serves
-    } else {
-        m->bytes += (int64_t)b;
-    }
-}
-
-// Whether that path serves this call: not inside a stream capture (the graph would hold the
-// handle's buffer) and not without the buffer. Calls on different streams take turns at the
-// buffer: each waits for the event recorded after the last use. The caller holds m->turn from here
-// until it has recorded its own, so that no other thread's wait comes between.
-bool residual_begin(mag_mesh *m, cudaStream_t s) {
+// Whether s is being captured (or cannot be asked).
+bool capturing(cudaStream_t s) {
     cudaStreamCaptureStatus cap = cudaStreamCaptureStatusNone;
-    if (m->fres && cudaStreamIsCapturing(s, &cap) == cudaSuccess && cap == cudaStreamCaptureStatusNone &&
-        cudaStreamWaitEvent(s, m->fres_done, 0) == cudaSuccess)
-        return true;
+    if (cudaStreamIsCapturing(s, &cap) == cudaSuccess) return cap != cudaStreamCaptureStatusNone;
     cudaGetLastError();
-    return false;
+    return true;
 }
 
 // enqueue() uses the handle's element scratch on stream s. Calls from different threads and on
-// different streams take turns at it, as at the residual entries above: without that, the second
-// call's elements overwrote entries which the first one's row sums had yet to read. Inside a stream
-// capture the order is the caller's (a graph cannot wait for an event of other streams' calls).
+// different streams take turns at it: each waits for the event recorded after the last use, and the
+// mutex is held until it has recorded its own, so that no other thread's wait comes between.
+// Without that, the second call's elements overwrote entries which the first one's row sums had yet
+// to read. Inside a stream capture the order is the caller's (a graph cannot wait for an event of
+// other streams' calls).
 template <typename F>
 int with_scratch(mag_mesh *m, cudaStream_t s, F enqueue) {
     cudaStreamCaptureStatus cap = cudaStreamCaptureStatusNone;
@@ -621,7 +603,6 @@ int mag_mesh_create(const double *d_P, int64_t Nn, const int32_t *d_T, int64_t N
         rc = build_tile_plan(ti, m->scratch, (size_t)Ne * kScratchPerElem * sizeof(double), &m->tile, s);
         if (rc != MAG_OK) return fail(rc);
         if (m->tile.ok) m->bytes += m->tile.bytes;
-        make_residual_buffer(m);
     }
     m->schedule = m->tile.ok               ? MAG_SCHEDULE_TILE_BLOCKS
                   : m->rowshared.nz_ok     ? MAG_SCHEDULE_NZ_ROW_BLOCKS
@@ -710,13 +691,12 @@ int mag_assemble_jacobian(mag_mesh *m, const double *d_sol, double *d_vals, doub
     }
     cudaStream_t s = (cudaStream_t)stream;
     if (m->schedule == MAG_SCHEDULE_TILE_BLOCKS && m->tile.ok && m->qp.standard_curl) {
-        if (!calc_j && m->fres) {
-            std::lock_guard<std::mutex> lk(m->turn);
-            if (residual_begin(m, s)) {
-                MAG_TRY(launch_residual(m->elems(), m->rows(), d_sol, m->qp, m->mat.mp, m->fres, d_res, s));
-                MAG_CUDA_TRY(cudaEventRecord(m->fres_done, s));
-                return finish(s);
-            }
+        // (a captured residual stays one launch that needs nothing of the handle's)
+        if (!calc_j && m->ne >= kResidualElems && !capturing(s)) {
+            MAG_TRY(with_scratch(m, s, [&] {
+                return launch_residual(m->elems(), m->rows(), d_sol, m->qp, m->mat.mp, m->scratch, d_res, s);
+            }));
+            return finish(s);
         }
         MAG_TRY(launch_tile_jacobian(m->tile, m->elems(), d_sol, m->qp, m->mat.mp, calc_j, calc_j ? d_vals : nullptr,
                                      d_res, m->status, s));

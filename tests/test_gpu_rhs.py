@@ -9,7 +9,7 @@ from conftest import bits_equal, load_golden
 
 from magpackage_b200 import _lib, quadrature, synth
 from magpackage_b200.assembler import Assembler, DofHandler, Mesh, Winding
-from magpackage_b200.plan import AssemblyPlan
+from magpackage_b200.plan import AssemblyPlan, generate_edges
 from oracle.oracle import mex_inputs
 
 pytestmark = pytest.mark.gpu
@@ -283,4 +283,44 @@ def test_sources_of_one_mesh_from_several_threads(beside):
         t.join()
     for w, mine in zip(want, outs):
         assert float(w.abs().max()) > 0 and all(torch.equal(w, r) for r in mine)
+    plan.check()
+
+
+def test_residual_needs_no_memory_of_its_own():
+    """From 200,000 elements on a residual alone goes through element entries: they lie in the handle's
+    element scratch, so that a mesh above that size holds no more bytes an element than one below (an
+    own buffer was 48; the two meshes' rows per element differ by 1 %)."""
+    held = []
+    for n in (32, 34):
+        mesh = synth.kuhn_box(n, seed=2)
+        edges, t2e, sign = generate_edges(mesh.T)
+        plan = AssemblyPlan(mesh.P, mesh.T, t2e, edges.shape[0], synth.cube_layout(mesh), sign)
+        held.append(plan.info.device_bytes / plan.num_elements)
+        assert (plan.num_elements >= 200000) == (n == 34)
+        plan.close()
+    assert abs(held[1] - held[0]) < 16, held
+
+
+def test_residuals_beside_sources_of_one_mesh():
+    """Residuals on one stream and sources on another, in turn from one thread, share the handle's
+    scratch: every result is the same bits as alone."""
+    from magpackage_b200.material import pack_material_data
+
+    mesh = synth.kuhn_box(33, seed=2)
+    edges, t2e, sign = generate_edges(mesh.T)
+    plan = AssemblyPlan(mesh.P, mesh.T, t2e, int(edges.shape[0]), synth.cube_layout(mesh), sign)
+    plan.set_materials(pack_material_data(synth.standard_materials()))
+    g = torch.Generator(device="cuda").manual_seed(3)
+    sol = 3e-4 * torch.randn(plan.num_dofs, dtype=torch.float64, device="cuda", generator=g)
+    js = torch.randn((mesh.num_elements, 3), dtype=torch.float64, device="cuda", generator=g)
+    want_r, want_s = plan.jacobian(sol, calc_j=False)[1], plan.source(js)
+    rs, ss = ([plan.new_vector() for _ in range(24)] for _ in range(2))
+    s1, s2 = torch.cuda.Stream(), torch.cuda.Stream()
+    torch.cuda.synchronize()
+    for r, v in zip(rs, ss):
+        plan.jacobian(sol, None, r, calc_j=False, stream=s1)
+        plan.source(js, v, stream=s2)
+    torch.cuda.synchronize()
+    assert float(want_r.abs().max()) > 0 and float(want_s.abs().max()) > 0
+    assert all(torch.equal(want_r, r) for r in rs) and all(torch.equal(want_s, v) for v in ss)
     plan.check()
