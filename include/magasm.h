@@ -54,7 +54,7 @@ typedef struct {
     int32_t schedule;       /* MAG_SCHEDULE_* used by the Jacobian assembly */
     int32_t tile_blocks;    /* CTA blocks of MAG_SCHEDULE_TILE_BLOCKS (0 = not available) */
     int32_t tile_colors;    /* largest number of element colour classes in one of its blocks */
-    int64_t device_bytes;   /* memory held by the handle */
+    int64_t device_bytes;   /* memory held by the handle, with what its workspace pool holds now */
     int32_t shared_blocks;  /* row blocks of MAG_SCHEDULE_SHARED_ROW_BLOCKS (0 = not available) */
     int32_t reserved0;      /* 0 */
     int32_t nz_pass;        /* 1 if MAG_SCHEDULE_NZ_ROW_BLOCKS is available for this mesh */

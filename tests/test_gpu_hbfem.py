@@ -185,3 +185,49 @@ def test_hbfem_real_transform_of_an_infinite_field(oracle_port, samples):
     bad = ~torch.isfinite(res[1])
     assert 0 < int(bad[0].sum()) < E
     assert torch.equal(res[0][~bad], res[1][~bad])
+
+
+def test_hbfem_workspace_is_bounded_and_reported():
+    """A handle's pool keeps no more workspace than the handle's own arrays hold; the rest goes back at
+    the next synchronisation, and what it keeps counts in device_bytes. Up to three harmonics on a
+    large mesh need no workspace at all."""
+    import ctypes as C
+
+    from magpackage_b200 import _lib
+    from magpackage_b200.plan import generate_edges
+
+    def held(plan):
+        torch.cuda.synchronize()
+        info = _lib.MeshInfo()
+        _lib.check(_lib.lib().mag_mesh_get_info(plan._h, C.byref(info)))
+        return int(info.device_bytes)
+
+    mesh = synth.kuhn_box(54, seed=2)  # 944,784 elements: 96 bytes an element and harmonic
+    edges, t2e, sign = generate_edges(mesh.T)
+    plan = AssemblyPlan(mesh.P, mesh.T, t2e, edges.shape[0], synth.cube_layout(mesh), sign)
+    plan.set_materials(material.pack_material_data(synth.standard_materials()))
+    small, base = 256 << 20, held(plan)
+    assert base > small
+    for K, calc_j in ((3, True), (3, False), (1, True), (6, False), (16, False)):
+        aft = AFT(tuple(range(K)), n_time_steps=33)
+        need = plan.num_elements * 96 * K
+        g = torch.Generator(device="cuda").manual_seed(K)
+        sol = tuple(1e-3 * torch.randn((K, plan.num_dofs), dtype=torch.float64, device="cuda", generator=g) for _ in range(2))
+        aft.device_operators()
+        torch.cuda.synchronize()
+        torch.cuda.empty_cache()
+        free0 = torch.cuda.mem_get_info()[0] + torch.cuda.memory_reserved()
+        R, _ = assemble_hbfem(plan, sol, aft, calc_j)
+        torch.cuda.synchronize()
+        free1 = torch.cuda.mem_get_info()[0] + torch.cuda.memory_reserved()
+        grown = held(plan) - base
+        assert free0 - free1 <= base + (64 << 20), (K, free0 - free1)  # (64 MB: kernels loaded at their first launch)
+        assert grown <= base + (32 << 20), (K, grown)                  # (32 MB: granularity of the pool)
+        if K == 3:
+            assert need > small and grown == 0
+        if K == 1:
+            assert need < small and grown >= need
+        if K == 16:
+            assert need > base + (64 << 20)
+        del R, sol
+    plan.close()
