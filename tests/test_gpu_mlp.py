@@ -173,3 +173,28 @@ def test_gradient_row_counts(n):
                  for s in (slice(0, k), slice(k, n))]
         # FP32 sums of up to 40,000 terms: a relative error of a few 2^-24 times the root of the count
         assert np.linalg.norm(g_all - parts[0] - parts[1]) <= 4 * np.sqrt(n) * 2.0**-24 * sum(map(np.linalg.norm, parts))
+
+
+@pytest.mark.parametrize("n", [1, 129, 40000])
+def test_weight_gradients_keep_all_bits_of_dz(n):
+    """With the same features in every row each layer's input is a constant c (BF16), so that dW = c db:
+    db sums dZ in FP32, dW its three BF16 parts. Without the trailing part they differ by 1e-5 and
+    more, without the last two by 3e-3. Bound: a tile's 128 rows are 24 accumulating MMAs, each off
+    by less than 2^-23 of the running sum; the sums over tiles add a few 1e-7."""
+    p = init_params(7)
+    p[256:320] = np.random.default_rng(7).normal(0, 0.1, 64)
+    c1 = np.array([0.5, -1.25, 0.8125, 2.0], dtype=np.float32)  # exact in BF16
+    x = np.tile(c1, (n, 1))
+    t = np.random.default_rng(8).normal(0, 1, n).astype(np.float32)
+    net = MLP(p)
+    _, g = net.gradient(torch.as_tensor(x, device="cuda"), torch.as_tensor(t, device="cuda"), 2.0 / n)
+    net.check()
+    g = g.cpu().double()
+    layers = [(g[0:256].view(64, 4), g[256:320]), (g[320:4416].view(64, 64), g[4416:4480]),
+              (g[4480:8576].view(64, 64), g[8576:8640])]
+    for k, (dW, db) in enumerate(layers):
+        big = db.abs() > 0.1 * db.abs().max()
+        c = torch.as_tensor(c1).double() if k == 0 else (dW[big] / db[big, None]).median(0).values.bfloat16().double()
+        want = db[:, None] * c[None, :]
+        assert float(want.norm()) > 0
+        assert float((dW - want).norm() / want.norm()) < 24 * 2.0**-23, k
