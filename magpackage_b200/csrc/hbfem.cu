@@ -445,9 +445,6 @@ __global__ void __launch_bounds__(kHbThreads, NT > 0 ? 3 : 1) k_hbfem_std(HbArgs
                 if (cb + j < W) out[cb + j] = acc[j];
         }
     }
-    // without Im P the imaginary sums are +0 whatever the samples hold (0 x infinity is NaN)
-    if (!A.pi)
-        for (int c = K; c < W; c++) out[c] = 0.0;
     __syncthreads();
     const int64_t left = A.m.ne - e0;
     const int count = (int)(left < kHbElems ? left : kHbElems) * 6 * W;
@@ -456,8 +453,9 @@ __global__ void __launch_bounds__(kHbThreads, NT > 0 ? 3 : 1) k_hbfem_std(HbArgs
 }
 
 // out_re[h][row], out_im[h][row]: per CSR row and residual component, the incidences'
-// entries summed from zero in ascending element order.
-__global__ void __launch_bounds__(128) k_rows_reduce_harm(RowPlan rp, const double *__restrict__ rscr, int K,
+// entries summed from zero in ascending element order. parts: the residual components to sum (2K, or
+// K without Im P: the imaginary residual is then zero whatever the entries hold, 0 x infinity is NaN).
+__global__ void __launch_bounds__(128) k_rows_reduce_harm(RowPlan rp, const double *__restrict__ rscr, int K, int parts,
                                                           double *__restrict__ out_re, double *__restrict__ out_im) {
     const int64_t idx = blockIdx.x * (int64_t)blockDim.x + threadIdx.x;
     const int W = 2 * K;
@@ -465,7 +463,8 @@ __global__ void __launch_bounds__(128) k_rows_reduce_harm(RowPlan rp, const doub
     const int64_t a = idx / W;
     const int c = (int)(idx % W);
     double r = 0.0;
-    for (int32_t t = rp.inc_ptr[a]; t < rp.inc_ptr[a + 1]; t++) {
+    const int32_t t1 = c < parts ? rp.inc_ptr[a + 1] : 0;
+    for (int32_t t = rp.inc_ptr[a]; t < t1; t++) {
         const uint32_t ew = rp.inc_elem[t];
         r = r + __ldg(rscr + ((int64_t)(ew & 0x1FFFFFFFu) * 6 + (ew >> 29)) * W + c);
     }
@@ -537,7 +536,7 @@ int launch_hbfem(const ElemData &m, const RowPlan &rp, int max_row, const double
         if (cudaPeekAtLastError() != cudaSuccess) return MAG_E_CUDA;
     }
     const int64_t nt = rp.ndof * 2 * K;
-    k_rows_reduce_harm<<<(unsigned)((nt + 127) / 128), 128, 0, s>>>(rp, rscr, K, out_re, out_im);
+    k_rows_reduce_harm<<<(unsigned)((nt + 127) / 128), 128, 0, s>>>(rp, rscr, K, pi ? 2 * K : K, out_re, out_im);
     if (cudaPeekAtLastError() != cudaSuccess) return MAG_E_CUDA;
     if (rows) return launch_rows_reduce(rp, max_row, scratch, vals, nullptr, s);
     return MAG_OK;
