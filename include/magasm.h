@@ -344,7 +344,8 @@ int mag_csr_apply_dirichlet(int64_t n, const int64_t *d_row_ptr, const int32_t *
  * iterations. Jacobi preconditioner, plus the auxiliary gradient space when set.
  * Deterministic (fixed-order reductions). Outputs: iterations, ||r||/||b||,
  * status 1 converged / 2 iteration limit / 3 breakdown (returns MAG_E_GEOMETRY).
- * Synchronises the host once per 256 iterations. */
+ * MAG_E_TIMEOUT, with d_x unchanged, if a grid barrier of the solver's kernel gave up
+ * waiting. Synchronises the host once per 256 iterations. */
 typedef struct mag_pcg mag_pcg;
 int mag_pcg_create(int64_t n, mag_pcg **out);
 int mag_pcg_destroy(mag_pcg *pcg);
@@ -356,6 +357,9 @@ int mag_pcg_destroy(mag_pcg *pcg);
 int mag_pcg_set_aux(mag_pcg *pcg, int64_t ni, const int64_t *d_g_row_ptr, const int32_t *d_g_col_idx,
                     const double *d_g_vals, const int64_t *d_gt_row_ptr, const int32_t *d_gt_col_idx,
                     const double *d_gt_vals, const double *d_dn_inv);
+/* Polls a CTA makes at a grid barrier before it gives up; 0 restores the default bound
+ * (some seconds). Small values exist to test that path. */
+int mag_pcg_set_spin_limit(mag_pcg *pcg, int64_t polls);
 int mag_pcg_solve(mag_pcg *pcg, const int64_t *d_row_ptr, const int32_t *d_col_idx, const double *d_vals,
                   const double *d_b, double *d_x, double rtol, int max_iter, int *iters, double *relres,
                   int *status, void *stream);

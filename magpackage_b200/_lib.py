@@ -68,6 +68,7 @@ _PROTOS = {
     "mag_pcg_create": ([_i64, C.POINTER(_vp)], _int),
     "mag_pcg_destroy": ([_vp], _int),
     "mag_pcg_set_aux": ([_vp, _i64, _vp, _vp, _vp, _vp, _vp, _vp, _vp], _int),
+    "mag_pcg_set_spin_limit": ([_vp, _i64], _int),
     "mag_pcg_solve": ([_vp, _vp, _vp, _vp, _vp, _vp, C.c_double, _int, C.POINTER(_int), _dp, C.POINTER(_int),
                        _vp], _int),
     "mag_batch_create": ([_vp, _int, _vp, _vp, _dp, _vp, C.POINTER(_vp), _vp], _int),

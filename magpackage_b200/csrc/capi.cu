@@ -1472,6 +1472,15 @@ int mag_pcg_set_aux(mag_pcg *p, int64_t ni, const int64_t *g_rp, const int32_t *
     return rc;
 }
 
+int mag_pcg_set_spin_limit(mag_pcg *p, int64_t polls) {
+    if (!p || polls < 0) {
+        set_error("mag_pcg_set_spin_limit: bad arguments");
+        return MAG_E_ARG;
+    }
+    pcg_set_spin_limit(p->s, polls);
+    return MAG_OK;
+}
+
 int mag_pcg_solve(mag_pcg *p, const int64_t *rp, const int32_t *ci, const double *v, const double *b, double *x,
                   double rtol, int max_iter, int *iters, double *relres, int *status, void *stream) {
     if (!p || !rp || !ci || !v || !b || !x || !(rtol >= 0) || max_iter <= 0) {

@@ -211,7 +211,7 @@ constexpr int kPcgAhead = 3;    // entries per lane and row loaded ahead (8 lane
 constexpr int kPcgKeep = 2;     // elements of r' and z a thread keeps between phases
 constexpr int kPcgGtLanes = 4;  // lanes per row of G^T, and entries each loads ahead
 constexpr int kPcgGtAhead = 4;
-constexpr long long kPcgSpin = 1LL << 24;  // polls before a grid barrier gives up
+constexpr long long kPcgSpin = 1LL << 24;  // polls before a grid barrier gives up, unless set
 
 struct PcgShared {
     double part[kPcgThreads / 32][2];
@@ -223,7 +223,7 @@ struct PcgShared {
 // since the launch. The caller has passed a __syncthreads after its last global write, except
 // for writes of warp 0, which the __syncwarp orders; the release and the acquire of thread 0
 // carry the CTA's writes and reads with them. L1 is not read stale: the acquire invalidates it.
-__device__ __forceinline__ bool pcg_barrier(PcgShared &S, unsigned *bar, unsigned &target, int *err) {
+__device__ __forceinline__ bool pcg_barrier(PcgShared &S, unsigned *bar, unsigned &target, int *err, long long spin) {
     target += gridDim.x;
     if (threadIdx.x < 32) {
         __syncwarp();
@@ -231,11 +231,11 @@ __device__ __forceinline__ bool pcg_barrier(PcgShared &S, unsigned *bar, unsigne
             asm volatile("red.release.gpu.global.add.u32 [%0], 1;" ::"l"(bar) : "memory");
             unsigned v = 0;
             long long i = 0;
-            for (; i < kPcgSpin; i++) {
+            for (; i < spin; i++) {
                 asm volatile("ld.acquire.gpu.global.u32 %0, [%1];" : "=r"(v) : "l"(bar) : "memory");
                 if ((int)(v - target) >= 0) break;
             }
-            if (i == kPcgSpin) {
+            if (i == spin) {
                 S.fail = 1;
                 atomicExch(err, 1);
             }
@@ -324,8 +324,12 @@ struct PcgLoop {
     unsigned *bar;
     int *err;
     int gs, gv;
+    long long spin;
 };
 
+// SPIN_SET: the barriers' poll limit is L.spin. (The default, a constant: as a value of L it took 1 %
+// of the time.)
+template <bool SPIN_SET>
 __global__ void __launch_bounds__(kPcgThreads, 1) k_pcg_iterate(PcgLoop L) {
     __shared__ PcgShared S;
     const Csr &A = L.A;
@@ -391,7 +395,7 @@ __global__ void __launch_bounds__(kPcgThreads, 1) k_pcg_iterate(PcgLoop L) {
                     }
             }
         pcg_block_sums<1>(S, acc, 0.0, b0, L.gs, L.part);
-        if (!pcg_barrier(S, L.bar, target, L.err)) return;
+        if (!pcg_barrier(S, L.bar, target, L.err, SPIN_SET ? L.spin : kPcgSpin)) return;
         // alpha
         {
             double pq[2];
@@ -459,7 +463,7 @@ __global__ void __launch_bounds__(kPcgThreads, 1) k_pcg_iterate(PcgLoop L) {
                 if (gl == 0 && j < j1) a.w[j] = __ldg(a.dn_inv + j) * s;
             }
             __syncthreads();
-            if (!pcg_barrier(S, L.bar, target, L.err)) return;
+            if (!pcg_barrier(S, L.bar, target, L.err, SPIN_SET ? L.spin : kPcgSpin)) return;
         }
         // Z (each thread reads its own r', and w of any node)
         double zr = 0.0, zz = 0.0;
@@ -481,7 +485,7 @@ __global__ void __launch_bounds__(kPcgThreads, 1) k_pcg_iterate(PcgLoop L) {
         }
         for (int64_t i = vfirst + kPcgKeep * vstep; i < n; i += vstep) L.z[i] = precond(i, rout[i]);
         pcg_block_sums<2>(S, zr, zz, b0, L.gv, part_rz);
-        if (!pcg_barrier(S, L.bar, target, L.err)) return;
+        if (!pcg_barrier(S, L.bar, target, L.err, SPIN_SET ? L.spin : kPcgSpin)) return;
         // beta and the stopping test
         {
             double t[2];
@@ -509,7 +513,7 @@ __global__ void __launch_bounds__(kPcgThreads, 1) k_pcg_iterate(PcgLoop L) {
         }
         for (int64_t i = vfirst + kPcgKeep * vstep; i < n; i += vstep) L.p[i] = fma(be, L.p[i], L.z[i]);
         __syncthreads();
-        if (!pcg_barrier(S, L.bar, target, L.err)) return;
+        if (!pcg_barrier(S, L.bar, target, L.err, SPIN_SET ? L.spin : kPcgSpin)) return;
     }
     if (blockIdx.x == 0 && threadIdx.x == 0) {
         PcgState &st = *L.st;
@@ -545,6 +549,7 @@ struct PcgSolver {
     int64_t w_cap = 0;
     cudaStream_t s = nullptr;
     PcgState *h_st = nullptr;  // pinned; the barrier words after it
+    long long spin = kPcgSpin;
 };
 
 int csr_spmv(int64_t n, const int64_t *rp, const int32_t *ci, const double *v, const double *x, double *y,
@@ -596,6 +601,8 @@ void pcg_destroy(PcgSolver *P) {
     delete P;
 }
 
+void pcg_set_spin_limit(PcgSolver *P, int64_t polls) { P->spin = polls > 0 ? (long long)polls : kPcgSpin; }
+
 int pcg_set_aux(PcgSolver *P, int64_t ni, const int64_t *g_rp, const int32_t *g_ci, const double *g_v,
                 const int64_t *gt_rp, const int32_t *gt_ci, const double *gt_v, const double *dn_inv) {
     if (ni <= 0) {
@@ -629,11 +636,12 @@ cudaError_t launch_iterations(PcgSolver *P, const Csr &A, cudaStream_t s) {
     const PcgBufs &B = P->B;
     const int gs = grid_for(P->n * kLanes), gv = grid_for(P->n);
     PcgLoop L{A, P->aux, B.x, {B.r, B.r2}, B.p, B.q, B.z, B.dinv, B.part, B.st, B.bar,
-              reinterpret_cast<int *>(B.bar + 1), gs, gv};
+              reinterpret_cast<int *>(B.bar + 1), gs, gv, P->spin};
     cudaError_t e = cudaMemsetAsync(B.bar, 0, 2 * sizeof(unsigned), s);
     if (e != cudaSuccess) return e;
     void *args[] = {&L};
-    return cudaLaunchCooperativeKernel((const void *)k_pcg_iterate, dim3((gs + kPcgSub - 1) / kPcgSub),
+    const auto kern = P->spin == kPcgSpin ? k_pcg_iterate<false> : k_pcg_iterate<true>;
+    return cudaLaunchCooperativeKernel((const void *)kern, dim3((gs + kPcgSub - 1) / kPcgSub),
                                        dim3(kPcgThreads), args, 0, s);
 }
 

@@ -178,6 +178,83 @@ def test_pcg_row_lengths_and_sizes_against_scipy(n, aux):
     assert np.linalg.norm(A @ out[0] - b) <= 2e-11 * np.linalg.norm(b)
 
 
+def _spd(n, ni, seed):
+    """Diagonally dominant A (kappa < 100), a gradient-like G of two entries a row, 1 / diag(G^T A G + 1), b."""
+    rng = np.random.default_rng(seed)
+    rows = np.repeat(np.arange(n), 3)
+    B = sp.csr_matrix((rng.normal(size=rows.size), (rows, rng.integers(0, n, rows.size))), shape=(n, n))
+    A = B + B.T
+    A.setdiag(0.0)
+    A = (A + sp.diags(1.05 * np.asarray(np.abs(A).sum(axis=1)).ravel() + 1.0)).tocsr()
+    A.sort_indices()
+    G = sp.csr_matrix((np.tile([-1.0, 1.0], n), (np.repeat(np.arange(n), 2), rng.integers(0, ni, 2 * n))), shape=(n, ni))
+    Gt = G.T.tocsr()
+    dn = 1.0 / ((Gt @ A).multiply(Gt).sum(axis=1).A1 + 1.0)
+    return A, G, Gt, dn, rng.normal(size=n)
+
+
+def _csr(m):
+    return [torch.as_tensor(v, device="cuda") for v in (m.indptr.astype(np.int64), m.indices.astype(np.int32), m.data)]
+
+
+@pytest.mark.parametrize("aux", [False, True])
+def test_pcg_more_rows_than_the_threads_keep(aux):
+    """400,000 rows and 50,000 gradient rows: more than two rows a thread, the rest of whose z lies in
+    memory, and two passes over G^T, on 148 SMs. The error is below kappa times the residual."""
+    n, ni = 400000, 50000
+    A, G, Gt, dn, b = _spd(n, ni, 11)
+    da, dg, dgt = _csr(A), _csr(G), _csr(Gt)
+    ddn, db = torch.as_tensor(dn, device="cuda"), torch.as_tensor(b, device="cuda")
+    L, h = _lib.lib(), C.c_void_p()
+    _lib.check(L.mag_pcg_create(n, C.byref(h)))
+    try:
+        if aux:
+            _lib.check(L.mag_pcg_set_aux(h, ni, *[_ptr(t) for t in dg + dgt + [ddn]]))
+        out = []
+        for _ in range(2):
+            x = torch.zeros_like(db)
+            it, rel, st = C.c_int(), C.c_double(), C.c_int()
+            _lib.check(L.mag_pcg_solve(h, *[_ptr(t) for t in da], _ptr(db), _ptr(x), 1e-11, 2000, C.byref(it),
+                                       C.byref(rel), C.byref(st), _lib.stream_ptr()))
+            assert st.value == 1 and rel.value <= 1e-11
+            out.append(x.cpu().numpy())
+    finally:
+        L.mag_pcg_destroy(h)
+    assert np.array_equal(out[0], out[1])
+    assert np.linalg.norm(A @ out[0] - b) <= 2e-11 * np.linalg.norm(b)
+
+
+def test_pcg_barrier_gives_up_and_recovers():
+    """A grid barrier limited to one poll runs out (the other CTAs have not arrived): the solve returns
+    MAG_E_TIMEOUT with the guess unchanged, and the next one with the default bound is right."""
+    n = 100000
+    A, _, _, _, b = _spd(n, 10, 12)
+    da, db = _csr(A), torch.as_tensor(b, device="cuda")
+    L, h = _lib.lib(), C.c_void_p()
+    _lib.check(L.mag_pcg_create(n, C.byref(h)))
+    try:
+        x = torch.full_like(db, 0.25)
+        it, rel, st = C.c_int(), C.c_double(), C.c_int()
+
+        def solve():
+            _lib.check(L.mag_pcg_solve(h, *[_ptr(t) for t in da], _ptr(db), _ptr(x), 1e-11, 2000, C.byref(it),
+                                       C.byref(rel), C.byref(st), _lib.stream_ptr()))
+
+        _lib.check(L.mag_pcg_set_spin_limit(h, 1))
+        with pytest.raises(_lib.MagError) as ei:
+            solve()
+        assert ei.value.code == -5  # MAG_E_TIMEOUT
+        assert torch.equal(x, torch.full_like(db, 0.25))
+        _lib.check(L.mag_pcg_set_spin_limit(h, 0))
+        solve()
+        assert st.value == 1
+        assert np.linalg.norm(A @ x.cpu().numpy() - b) <= 2e-11 * np.linalg.norm(b)
+        with pytest.raises(_lib.MagError):
+            _lib.check(L.mag_pcg_set_spin_limit(h, -1))
+    finally:
+        L.mag_pcg_destroy(h)
+
+
 def test_coil_source_is_discretely_divergence_free():
     from magpackage_b200.transient import TransientConfig, TransientProblem
 
