@@ -2,8 +2,9 @@
 // activations, BF16 tensor-core GEMMs (tcgen05, FP32 accumulators in TMEM) and
 // FP32 master weights. Forward (inference and training) and backward kernels.
 //
-// Tile = 128 rows (elements) per CTA, 128 threads; thread t owns row t, and warp
-// w reads TMEM lanes 32w..32w+31 (accumulator row m lives in lane m for M=128).
+// Tile = 128 rows (elements). Forward: 128 threads a tile, thread t owns row t, and warp w reads
+// TMEM lanes 32w..32w+31 (accumulator row m lives in lane m for M=128); inference runs two tiles
+// in a CTA, which share the weights. Backward: 256 threads a tile, 32 columns a thread.
 // Operands live in shared memory in the no-swizzle K-major "core matrix"
 // layout: 8 rows x 16 bytes per core matrix, K-adjacent core matrices 128 B
 // apart (leading byte offset), 8-row groups K*16 B apart (stride byte offset).
@@ -13,8 +14,9 @@
 //
 // Rounding points (mirrored by oracle/mlp_ref.py): layer inputs are rounded to
 // BF16 before each MMA; accumulation, biases, activations, the last (64 -> 1)
-// layer and all gradients are FP32. Inference halves W1..W3 and b1..b3 (exact),
-// so that its accumulators hold z/2 and SiLU takes one FMA after the tanh.
+// layer and all gradients are FP32: dX takes dZ rounded to BF16 as its MMA's input, dW all of dZ as
+// three BF16 parts. Inference halves W1..W3 and b1..b3 (exact), so that its accumulators hold z/2
+// and SiLU takes one FMA after the tanh.
 #include <cuda_bf16.h>
 
 #include <cstdint>
@@ -341,7 +343,8 @@ __device__ __forceinline__ bool run_layer_fwd(int tile_id, uint32_t tmem, const 
 // INFER: no pre-activations kept (prediction); the epilogues use the packed forms above.
 // TILES tiles run in a CTA, each with its kRows threads, image, TMEM columns and barriers; they
 // share the weights, so that 32 warps fit an SM instead of 24: 14.8 to 12.8 us at 100,000 rows; at 8M
-// rows 445 and 444 us, bound by the transcendental unit and its queue.
+// rows 445 and 444 us: the transcendental unit is busy 81 % of the active cycles there, and the queue
+// it shares with shared memory (MIO throttle) is the longest stall.
 template <bool INFER, int TILES>
 __global__ void __launch_bounds__(TILES * kRows, TILES == 2 ? 4 : 6) k_mlp_forward(MlpForwardArgs a) {
     extern __shared__ __align__(1024) unsigned char smem_raw[];
@@ -539,7 +542,10 @@ __device__ __forceinline__ void put_bits32(__nv_bfloat16 *dst, const uint32_t v[
 }
 
 // The three parts of 32 FP32 values: each the leading 8 bits of what the parts before leave, so
-// that they add up exactly. Infinities and NaN stay in the leading part.
+// that they add up exactly (but for bits below 2^-133, the last of a BF16). Infinities and NaN stay
+// in the leading part. An input that rounds to an infinity meets a dZ that is NaN in its whole row
+// (dsilu of the next layer's infinite or NaN pre-activations), so 0 x infinity of a zero part adds
+// no NaN that FP32 products would not have.
 __device__ __forceinline__ void put_split32(BwdSmem &B, int row, int c0, const float v[32]) {
     float x[32];
 #pragma unroll

@@ -2,9 +2,10 @@
 // each element evaluated by one thread, about 1.5 times per assembly.
 //
 // Rows (edges) are grouped by the spatial tile of their lower node: nodes are binned
-// into coordinate layers along x, y and z, and 4 x 4 x 4 layers make a tile (a CTA
-// block holds at most kTileMaxNnz nonzeros and kTileMaxInc incidences; larger tiles
-// are cut). A CTA takes one block: its CSR rows, and every element incident to them.
+// into coordinate layers along x, y and z, and 4 x 4 x 4 layers make a tile, on small meshes
+// 3 x 3 x 3 or 4 x 2 x 2 (a CTA block holds at most kTileMaxNnz nonzeros, kTileMaxInc
+// incidences and kTileMaxRows rows; larger tiles are cut). A CTA takes one block: its CSR
+// rows, and every element incident to them.
 //   colour phases -- one thread per element evaluates geometry, the six curls, B and
 //              nu(|B|^2) once (the reference's arithmetic), then, for each of its local
 //              rows that belongs to the block, the row of the 6x6 tangent and the

@@ -173,7 +173,7 @@ class TransientProblem:
         a0 = vals0 + self.reg * self.m_reg
         self.dirichlet(a0, None)
         self._setup_aux(a0, fixed, on)
-        # the system matrix lives in one buffer, so the solver's captured iteration graph stays valid
+        # the system matrix lives in one buffer, which every Newton iteration fills anew
         self._A = torch.empty(self.plan.nnz, dtype=torch.float64, device=dev)
 
     # ---- small helpers -----------------------------------------------------
