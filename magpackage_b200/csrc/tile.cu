@@ -647,8 +647,12 @@ __global__ void __launch_bounds__(kMassBT, 2)
 // colour phase runs in one pass (256 threads left a second pass with one warp busy).
 constexpr int kTileBT = 320;
 constexpr int kTileMinB = 2;
-// Small tiles (4x2x2 or 3x3x3 layers): a colour class holds 90 to 135 elements.
-constexpr int kSmallBT = 160;
+// Small blocks (tiles of 4x2x2 or 3x3x3 layers, a colour class of 90 to 135 elements): each colour
+// phase in one pass. A tile that holds more than its layers' share (graded meshes, layers that nodes
+// of different depth fall into) is cut at a block's limits instead; its classes take two passes and
+// more of 160 threads, so that the plan says which shape suits. Jacobian, us, 160 x 3 / 320 x 2: 8^3
+// hexahedra 9.3 / 9.7, graded 20^3 21.6 / 17.5, 1 x 1 x 4000 16.5 / 11.1, two cubes far apart 19.7 / 14.7.
+constexpr int kSmallBT = kTileSmallThreads;
 constexpr int kSmallMinB = 3;
 
 }  // namespace
@@ -695,10 +699,10 @@ int launch_shape(const TileArgs &a, const TilePlan &tp, size_t smem, cudaStream_
     return cudaPeekAtLastError() == cudaSuccess ? MAG_OK : MAG_E_CUDA;
 }
 
-// The shape of the plan's tiles.
+// The shape of the plan's blocks.
 template <bool CALCJ, bool Q4, int MODE>
 int launch(const TileArgs &a, const TilePlan &tp, size_t smem, cudaStream_t s) {
-    return tp.small_tiles ? launch_shape<CALCJ, Q4, MODE, kSmallBT, kSmallMinB>(a, tp, smem, s)
+    return tp.small_blocks ? launch_shape<CALCJ, Q4, MODE, kSmallBT, kSmallMinB>(a, tp, smem, s)
                           : launch_shape<CALCJ, Q4, MODE, kTileBT, kTileMinB>(a, tp, smem, s);
 }
 
@@ -743,7 +747,7 @@ int launch_tile_jacobian(const TilePlan &tp, const ElemData &m, const double *so
 }
 
 const char *tile_variant_name(int v) {
-    static const char *names[kTileVariants] = {"320 threads x 2 CTAs/SM (small tiles: 160 x 3)", "288 threads x 2 CTAs/SM",
+    static const char *names[kTileVariants] = {"320 threads x 2 CTAs/SM (small blocks: 160 x 3)", "288 threads x 2 CTAs/SM",
                                                "256 threads x 2 CTAs/SM", "512 threads x 1 CTA/SM"};
     return v >= 0 && v < kTileVariants ? names[v] : "";
 }
@@ -767,8 +771,8 @@ int launch_tile_mass(const TilePlan &tp, const ElemData &m, const double *sigma,
     a.vals = vals;
     a.nnz_total = tp.nnz;
     const size_t smem = tile_smem_bytes(tp, &a) + (size_t)18 * qp.nq * sizeof(double);
-    const auto kern = tp.small_tiles ? k_tile_mass<kSmallBT, kSmallMinB> : k_tile_mass<kMassBT, 2>;
-    const int threads = tp.small_tiles ? kSmallBT : kMassBT;
+    const auto kern = tp.small_blocks ? k_tile_mass<kSmallBT, kSmallMinB> : k_tile_mass<kMassBT, 2>;
+    const int threads = tp.small_blocks ? kSmallBT : kMassBT;
     int resident = 0;
     MAG_TRY(resident_ctas((const void *)kern, threads, smem, &resident));
     const int ahead = tp.prefetch_waves > 0 ? resident * tp.prefetch_waves : tp.nblocks;

@@ -15,6 +15,7 @@ constexpr int kTileMaxInc = 4095;   // (row, element) incidences per block (12-b
 constexpr int kTileMaxRows = 1536;  // rows per block: more than 8191 / 6, so that only rows without an element (which
                                     // have neither nonzeros nor incidences) and rows of a few entries reach it
 constexpr int kTileMaxColors = 8;   // element colour classes per block
+constexpr int kTileSmallThreads = 160;  // threads of a CTA on small blocks
 constexpr int kTileChunk = 256;     // nonzeros per store chunk (one warp stores a chunk)
 constexpr int kTileSlotPad = 32;    // doubles of slack after a block's values in shared memory (even):
                                     // a row's first nonzero plus any 5-bit position stays inside
@@ -61,7 +62,9 @@ struct TilePlan {
     double build_ms = 0.0;
     int64_t bytes = 0;
     int ok = 0;
-    int small_tiles = 0;  // tiles of fewer than 4 x 4 x 4 node layers: launched with 160 threads x 3 CTAs/SM
+    int small_tiles = 0;   // tiles of fewer than 4 x 4 x 4 node layers
+    int small_blocks = 0;  // and no colour class of more than kTileSmallThreads elements: launched with
+                           // kTileSmallThreads threads x 3 CTAs/SM
     int variant = 0;  // launch shape of the Newton Jacobian (0 .. kTileVariants-1)
     int prefetch_waves = 1;  // staging depth: a CTA prefetches the block this many waves ahead (0: none)
 };

@@ -34,18 +34,23 @@ namespace {
 
 constexpr int kPB = 256;         // threads of the per-block kernels
 constexpr int kLayerB = 1024;    // threads of the layer walk
-// Node layers per tile: the first of these forms whose tiles are few enough, the last one
-// otherwise. A block's time is latency: where blocks would leave SMs idle (148 on the GPU),
+// Node layers per tile: the first of these forms whose tiles, and the blocks they are cut into, are
+// few enough, the last one otherwise. A block's time is latency: where blocks would leave SMs idle (148 on the GPU),
 // smaller ones finish sooner although they evaluate more elements twice (4x2x2 up to 1.9 times an
 // element, 3x3x3 1.67, 4x4x4 1.5). Measured on the device alone, us, with 4x4x4 / as chosen here:
 // Jacobian at 8^3 hexahedra (4x2x2) 14.9 / 10.3, 14^3 (3x3x3) 15.5 / 11.4, 16^3 15.7 / 12.5; M(1)
 // 18.6 / 10.5, 18.8 / 13.0, 19.0 / 14.9; at 20^3, where 4x4x4 stays, 3x3x3 has Jacobian 14.5
-// against 16.3 but at 24^3 23.3 against 20.0.
+// against 16.3 but at 24^3 23.3 against 20.0. Where tiles hold so many rows that a colour class is
+// more than kTileSmallThreads elements, a block is no small one, and one wave of them is the limit:
+// graded 16^3 (136 blocks) 11.5 against 14.2, 20^3 (232) 17.5 against 18.1 but M(1) 28.3 against 27.2,
+// 24^3 (335) 24.5 against 19.9.
 struct TileForm {
     int l[3];
     int64_t most;
 };
-constexpr TileForm kTileForms[] = {{{4, 2, 2}, 148}, {{3, 3, 3}, 2 * 148}, {{4, 4, 4}, INT64_MAX}};
+constexpr int kOneWave = 148;
+constexpr int kNumForms = 3;
+constexpr TileForm kTileForms[kNumForms] = {{{4, 2, 2}, kOneWave}, {{3, 3, 3}, 2 * kOneWave}, {{4, 4, 4}, INT64_MAX}};
 constexpr uint32_t kNone16 = 0xFFFFu;
 
 unsigned grid1(int64_t n, int b = 256) { return (unsigned)((n + b - 1) / b); }
@@ -63,7 +68,7 @@ struct PlanInfo {
     int unused_rows;   // rows without incidences
     int fail;          // the mesh does not suit the schedule
     int nblocks, nchunks, nrec;
-    int max_nnz, max_inc, max_colors, max_rows, max_chunks;
+    int max_nnz, max_inc, max_colors, max_rows, max_chunks, max_class;
 };
 
 __host__ __device__ inline unsigned long long ordered(double x) {
@@ -571,9 +576,14 @@ __global__ void __launch_bounds__(kPB) k_color_blocks(TilePlanInput in, const in
         B.nnz = nnz;
         B.ninc = i1 - i0;
         B.ncolors = ncol;
-        for (int c = 0; c < kTileMaxColors; c++) B.col_end[c] = S.col_end[c];
+        int most = 0;
+        for (int c = 0; c < kTileMaxColors; c++) {
+            B.col_end[c] = S.col_end[c];
+            if (c < ncol) most = max(most, S.col_end[c] - (c > 0 ? S.col_end[c - 1] : 0));
+        }
         blocks[b] = B;
         atomicMax(&info->max_colors, ncol);
+        atomicMax(&info->max_class, most);
     }
 }
 
@@ -664,7 +674,12 @@ struct CubTemp {
         if (!arena.get(&ptr, n)) return MAG_E_NOMEM; \
     } while (0)
 
-int build(const TilePlanInput &in, void *work, size_t work_bytes, bool large, TilePlan *p, cudaStream_t s) {
+// The plan with the first form from *form on whose tiles are few enough. p->ok stays 0 where the mesh
+// does not suit the schedule (*form is then kNumForms) or where the form's blocks turn out too many or
+// too large (*form is the next one to try).
+int build(const TilePlanInput &in, void *work, size_t work_bytes, int *form, TilePlan *p, cudaStream_t s) {
+    int k = *form;
+    *form = kNumForms;
     Arena arena(work, work_bytes, s);
     CubTemp temp;
     const int64_t nn = in.nn, ne = in.ne, ndof = in.ndof, ninc = in.ninc;
@@ -694,8 +709,8 @@ int build(const TilePlanInput &in, void *work, size_t work_bytes, bool large, Ti
     if (hi.fail) return MAG_OK;
     TileGrid g;
     int64_t tiles = 1;
-    for (const TileForm &f : kTileForms) {
-        if (large && f.most < INT64_MAX) continue;
+    for (;; k++) {
+        const TileForm &f = kTileForms[k];
         tiles = 1;
         for (int a = 0; a < 3; a++) {
             g.l[a] = f.l[a];
@@ -703,9 +718,9 @@ int build(const TilePlanInput &in, void *work, size_t work_bytes, bool large, Ti
             tiles *= g.n[a];
             if (tiles >= (int64_t(1) << 31)) return MAG_OK;
         }
-        p->small_tiles = f.most < INT64_MAX ? 1 : 0;
         if (tiles <= f.most) break;
     }
+    const bool small = k + 1 < kNumForms;
     uint32_t *node_tile = nullptr, *tile = nullptr, *tile_s = nullptr, *row = nullptr, *order = nullptr;
     int *last = nullptr, *pn = nullptr, *pi = nullptr;
     MAG_GET(node_tile, nn);
@@ -735,6 +750,10 @@ int build(const TilePlanInput &in, void *work, size_t work_bytes, bool large, Ti
     int nb = 0;
     MAG_CUDA_TRY(cudaMemcpyAsync(&nb, tcnt + tiles, sizeof(int), cudaMemcpyDeviceToHost, s));
     MAG_CUDA_TRY(cudaStreamSynchronize(s));
+    if (nb > kTileForms[k].most) {
+        *form = k + 1;
+        return MAG_OK;
+    }
     MAG_GET(bstart, nb + 1);
     k_cut_tiles<true><<<grid1(tiles + 1, 128), 128, 0, s>>>(tiles, ndof, tile_s, pn, pi, nullptr, tcnt, bstart);
     // rows padded by 16 bytes, like the chunks: the kernels' L2 prefetches round to 16 bytes
@@ -780,6 +799,10 @@ int build(const TilePlanInput &in, void *work, size_t work_bytes, bool large, Ti
                                                      info);
     MAG_TRY(read_info(info, &hi, s));
     if (hi.fail) return MAG_OK;
+    if (small && hi.max_class > kTileSmallThreads && nb > kOneWave) {
+        *form = k + 1;
+        return MAG_OK;
+    }
     if (nrec > 0)
         k_fill_records<<<grid1(nrec, 128), 128, 0, s>>>(in, nrec, start, keys_s, (uint64_t(1) << eb) - 1, inc_s, slotw, pos,
                                                        p->recs);
@@ -795,6 +818,8 @@ int build(const TilePlanInput &in, void *work, size_t work_bytes, bool large, Ti
     p->max_colors = hi.max_colors;
     p->max_rows = hi.max_rows;
     p->max_chunks = hi.max_chunks;
+    p->small_tiles = small ? 1 : 0;
+    p->small_blocks = small && hi.max_class <= kTileSmallThreads ? 1 : 0;
     p->evals_per_elem = (double)nrec / (double)ne;
     p->bytes = (int64_t)(b_blk + b_rows + b_ch + b_rec);
     p->ok = 1;
@@ -815,9 +840,13 @@ int build_tile_plan(const TilePlanInput &in, void *work, size_t work_bytes, Tile
     if (in.wide || in.ne <= 0 || in.ndof <= 0 || in.nn <= 0 || in.nnz >= (int64_t(1) << 32)) return MAG_OK;
     const auto t0 = std::chrono::steady_clock::now();
     TilePlan p;
-    const int rc = build(in, work, work_bytes, large, &p, s);
+    int rc = MAG_OK;
+    for (int form = large ? kNumForms - 1 : 0; form < kNumForms && !p.ok;) {
+        rc = build(in, work, work_bytes, &form, &p, s);
+        if (rc != MAG_OK || !p.ok) free_tile_plan(&p);
+        if (rc != MAG_OK) break;
+    }
     if (rc != MAG_OK || !p.ok) {
-        free_tile_plan(&p);
         if (rc != MAG_E_NOMEM) return rc;
         cudaGetLastError();
         return MAG_OK;  // no room: the other schedules remain

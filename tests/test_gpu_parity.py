@@ -964,3 +964,46 @@ def test_assembler_maps_equal_expanded_arrays(form):
     for k, v in smap.items():
         js[m.RegionTags == k] = v
     assert bits_equal(host(asm.assemble_source(smap)), host(asm.plan.source(dev(js))))
+
+
+@pytest.mark.parametrize("kind,most_blocks", [
+    ("graded 12", 148),    # 4x2x2 layers, tiles cut at a block's limits: blocks of two sizes
+    ("graded 24", 296),    # more blocks than 3x3x3 tiles: 4x4x4
+    ("graded 20", 231),    # 3x3x3 blocks of more than 160 elements a colour, more than one wave: 4x4x4
+    ("two cubes", 148),    # far apart: each cube in one tile
+    ("rod", 148),
+    ("thin", 296),
+])
+def test_tiles_cut_at_the_block_limits(kind, most_blocks):
+    """Meshes whose tiles hold more rows than their layers' share: the tile schedule's results are the
+    two-pass ones bit for bit, and no small tile form stays whose blocks are more than it is for."""
+    if kind.startswith("graded"):
+        m = synth.kuhn_box(int(kind[7:]), seed=1)
+        P, T = np.array(m.P) ** (3 if kind == "graded 24" else 2), np.array(m.T)
+    elif kind == "two cubes":
+        m = synth.kuhn_box(10, seed=1)
+        P, T = np.concatenate([m.P, np.array(m.P) + 1000.0]), np.concatenate([m.T, m.T + len(m.P)])
+    elif kind == "rod":
+        m = synth.kuhn_box(1, 1, 1500, seed=1)
+        P, T = np.array(m.P), np.array(m.T)
+    else:
+        m = synth.kuhn_box(30, 24, 20, seed=1)
+        P, T = np.array(m.P) * np.array([1.0, 1.0, 1000.0]), np.array(m.T)
+    T = np.ascontiguousarray(T, dtype=np.int32)
+    edges, t2e, sign = generate_edges(T)
+    E = int(edges.shape[0])
+    tags = np.where(np.arange(len(T)) % 3 == 0, synth.IRON, 1).astype(np.int32)
+    plan = AssemblyPlan(P, T, t2e, E, tags, sign)
+    plan.set_materials(material.pack_material_data(synth.standard_materials()))
+    assert plan.info.schedule == _lib.SCHEDULE_TILE_BLOCKS and plan.info.tile_blocks <= most_blocks
+    g = torch.Generator(device="cuda").manual_seed(1)
+    sol = 1e-2 * torch.randn(E, dtype=torch.float64, device="cuda", generator=g)
+    nu = torch.rand(len(T), dtype=torch.float64, device="cuda", generator=g) + 1.0
+
+    def results():
+        return [*plan.jacobian(sol), plan.jacobian(sol, calc_j=False)[1], plan.stiffness(nu), plan.mass(None), plan.mass(nu)]
+
+    got = results()
+    plan.check()
+    plan.set_schedule(_lib.SCHEDULE_TWO_PASS)
+    assert all(bits_equal(a.cpu().numpy(), b.cpu().numpy()) for a, b in zip(got, results()))
