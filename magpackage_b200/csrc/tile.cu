@@ -86,8 +86,11 @@ __device__ __forceinline__ double qsum_equal(double u, int nq) {
 
 __device__ __forceinline__ void flag(int *err) { atomicOr(err, 1); }
 
-// A record plane is read once: it does not displace the coordinates, solution and tables in L1.
+// A record plane is read once: with PASS it does not displace the coordinates, solution and tables
+// in L1 (records_pass says when that pays).
+template <bool PASS = true>
 __device__ __forceinline__ uint4 ld_record(const uint4 *p) {
+    if (!PASS) return __ldg(p);
     uint4 v;
     asm("ld.global.nc.L1::no_allocate.v4.u32 {%0, %1, %2, %3}, [%4];" : "=r"(v.x), "=r"(v.y), "=r"(v.z), "=r"(v.w) : "l"(p));
     return v;
@@ -107,12 +110,13 @@ enum TileMode { kJacobian = 0, kStiffness = 1, kSeeded = 2, kHarmonicDc = 3 };
 // class shares one), so an entry is stored rather than added: slot = v instead of
 // slot = 0 + v, the same value up to the sign of an exact zero, which the store phase
 // normalises (x + 0 turns -0 into +0 and leaves every other value unchanged).
-template <bool CALCJ, bool Q4, int MODE, bool FIRST = false>
+template <bool CALCJ, bool Q4, int MODE, bool PASS, bool FIRST = false>
 __device__ __forceinline__ uint32_t tile_element(const TileArgs &A, int64_t i, double *__restrict__ slot,
                                              double2 *__restrict__ incv, int bnnz, int binc) {
     const int64_t n = A.nrec;
-    const uint4 p0 = ld_record(A.recs + i), p1 = ld_record(A.recs + n + i), p2 = ld_record(A.recs + 2 * n + i);
-    const uint4 p3 = ld_record(A.recs + 3 * n + i), p4 = ld_record(A.recs + 4 * n + i), p5 = ld_record(A.recs + 5 * n + i);
+    const uint4 p0 = ld_record<PASS>(A.recs + i), p1 = ld_record<PASS>(A.recs + n + i),
+                p2 = ld_record<PASS>(A.recs + 2 * n + i), p3 = ld_record<PASS>(A.recs + 3 * n + i),
+                p4 = ld_record<PASS>(A.recs + 4 * n + i), p5 = ld_record<PASS>(A.recs + 5 * n + i);
     const int4 tt = make_int4((int)p0.x, (int)p0.y, (int)p0.z, (int)p0.w);
     const unsigned sb = (p2.w >> 8) & 0x3Fu;
     const unsigned pos[6] = {p3.x, p3.y, p3.z, p3.w, p4.x, p4.y};
@@ -257,7 +261,7 @@ __device__ __forceinline__ void cp_async_wait_all() { asm volatile("cp.async.wai
 // (ahead = the CTAs resident at once), the block the hardware starts about when b ends.
 // The block's row table and store chunks are copied into shared memory while its
 // elements run, so the row and store phases start without a global round trip.
-template <int BT, int MINB, bool CALCJ, bool Q4, int MODE>
+template <int BT, int MINB, bool CALCJ, bool Q4, int MODE, bool PASS>
 __global__ void __launch_bounds__(BT, MINB) k_tile(TileArgs A, int nblocks, int ahead) {
     constexpr bool STIFF = MODE == kStiffness || MODE == kHarmonicDc;
     extern __shared__ __align__(16) double tile_smem[];
@@ -290,10 +294,10 @@ __global__ void __launch_bounds__(BT, MINB) k_tile(TileArgs A, int nblocks, int 
                 const int c1 = Bp->col_end[c];
                 if (c == 0)
                     for (int i = c0 + tid; i < c1; i += BT)
-                        tile_element<CALCJ, Q4, MODE, true>(A, (int64_t)rec0 + i, slot, incv, nnz, ninc);
+                        tile_element<CALCJ, Q4, MODE, PASS, true>(A, (int64_t)rec0 + i, slot, incv, nnz, ninc);
                 else
                     for (int i = c0 + tid; i < c1; i += BT)
-                        tile_element<CALCJ, Q4, MODE>(A, (int64_t)rec0 + i, slot, incv, nnz, ninc);
+                        tile_element<CALCJ, Q4, MODE, PASS>(A, (int64_t)rec0 + i, slot, incv, nnz, ninc);
                 c0 = c1;
                 if (c + 1 == ncolors) cp_async_wait_all();
                 __syncthreads();
@@ -304,7 +308,7 @@ __global__ void __launch_bounds__(BT, MINB) k_tile(TileArgs A, int nblocks, int 
             }
         } else {
             for (int i = tid; i < nrec; i += BT)
-                tile_element<CALCJ, Q4, MODE>(A, (int64_t)rec0 + i, slot, incv, nnz, ninc);
+                tile_element<CALCJ, Q4, MODE, PASS>(A, (int64_t)rec0 + i, slot, incv, nnz, ninc);
             cp_async_wait_all();
             __syncthreads();
         }
@@ -370,10 +374,10 @@ __device__ __forceinline__ void tile_mass_element(const TileArgs &A, const doubl
                                                   double *__restrict__ slot, double2 *__restrict__ incv, int bnnz,
                                                   int binc, const double *__restrict__ sval) {
     const int64_t n = A.nrec;
-    const uint4 p2 = ld_record(A.recs + 2 * n + i);
+    const uint4 p2 = ld_record<>(A.recs + 2 * n + i);
     const double sigma = sigma_e ? __ldg(sigma_e + p2.z) : 1.0;
     if (!(fabs(sigma) > 1e-12)) return;
-    const uint4 p0 = ld_record(A.recs + i);
+    const uint4 p0 = ld_record<>(A.recs + i);
     const int4 tt = make_int4((int)p0.x, (int)p0.y, (int)p0.z, (int)p0.w);
     const unsigned sb = (p2.w >> 8) & 0x3Fu;
     double M[21];  // row by row from the diagonal
@@ -403,7 +407,7 @@ __device__ __forceinline__ void tile_mass_element(const TileArgs &A, const doubl
                 for (int j = l; j < 6; j++, k++) M[k] = M[k] + dot3(N[l], N[j]) * sigma * w;
         }
     }
-    const uint4 p3 = ld_record(A.recs + 3 * n + i), p4 = ld_record(A.recs + 4 * n + i), p5 = ld_record(A.recs + 5 * n + i);
+    const uint4 p3 = ld_record<>(A.recs + 3 * n + i), p4 = ld_record<>(A.recs + 4 * n + i), p5 = ld_record<>(A.recs + 5 * n + i);
     const unsigned pos[6] = {p3.x, p3.y, p3.z, p3.w, p4.x, p4.y};
     const unsigned sl[6] = {p4.z, p4.w, p5.x, p5.y, p5.z, p5.w};
 #pragma unroll
@@ -495,8 +499,8 @@ __global__ void __launch_bounds__(BT, MINB)
         const int c1 = Bp->col_end[c];
         for (int i = c0 + tid; i < c1; i += BT) {
             const int64_t r = (int64_t)rec0 + i;
-            const uint32_t e = c == 0 ? tile_element<true, Q4, kStiffness, true>(A, r, slot, incv, nnz, ninc)
-                                      : tile_element<true, Q4, kStiffness>(A, r, slot, incv, nnz, ninc);
+            const uint32_t e = c == 0 ? tile_element<true, Q4, kStiffness, true, true>(A, r, slot, incv, nnz, ninc)
+                                      : tile_element<true, Q4, kStiffness, true>(A, r, slot, incv, nnz, ninc);
             if (!conducting) conducting = fabs(I.sigma ? __ldg(I.sigma + e) : 1.0) > 1e-12;
         }
         c0 = c1;
@@ -688,9 +692,22 @@ int resident_ctas(const void *kern, int threads, size_t smem, int *out) {
     return MAG_OK;
 }
 
+// Whether the records pass L1 by: below these sizes loads that go through it are faster. Measured, us,
+// through L1 / by: Jacobian at 20^3 hexahedra (72,000 records) 14.8 / 14.9, shuffled 26^3 (163,000) 27.7 /
+// 29.7, 34^3 (354,000) 37.8 / 38.2, 36^3 (420,000) 47.6 / 45.0, 40^3 65.2 / 62.5, 60^3 191 / 190; residual
+// alone at 26^3 shuffled 17.8 / 18.4, 40^3 (576,000) 28.1 / 28.9, 44^3 (767,000) 38.6 / 37.8, 48^3 53.1 /
+// 47.2. CTAs of the small shape have few records and each SM three of them: Jacobian at 8^3 9.24 / 9.06,
+// residual at 17^3 7.2 / 6.8, always by.
+template <bool CALCJ>
+bool records_pass(const TilePlan &tp) {
+    return tp.nrec >= (CALCJ ? 380000 : 650000);
+}
+
 template <bool CALCJ, bool Q4, int MODE, int BT, int MINB>
 int launch_shape(const TileArgs &a, const TilePlan &tp, size_t smem, cudaStream_t s) {
-    auto kern = k_tile<BT, MINB, CALCJ, Q4, MODE>;
+    auto kern = k_tile<BT, MINB, CALCJ, Q4, MODE, true>;
+    if constexpr (BT != kSmallBT)
+        if (!records_pass<CALCJ>(tp)) kern = k_tile<BT, MINB, CALCJ, Q4, MODE, false>;
     int resident = 0;
     MAG_TRY(resident_ctas((const void *)kern, BT, smem, &resident));
     // (ahead >= nblocks: no CTA prefetches)
