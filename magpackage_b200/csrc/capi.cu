@@ -454,6 +454,17 @@ bool capturing(cudaStream_t s) {
     return true;
 }
 
+// M(sigma) by the tile blocks, or, on small meshes whose blocks are not small, by the element blocks and
+// the row sums: a block of several hundred elements takes 20 us whatever their number, and blocks of
+// strongly stretched meshes evaluate each element more than twice. Measured, us, tile blocks / two
+// passes (elements, evaluations an element): 60 x 6 x 6 hexahedra (12,960, 1.72) 19.3 / 14.3, two cubes
+// far apart (20,736, 1.78) 20.7 / 18.7, a centred grading (24,576, 1.51) 20.1 / 19.1, 22 x 18 x 19 (45,144,
+// 1.44) 19.4 / 24.9, 1 x 1 x 4000 (24,000, 1.02) 14.1 / 17.9, stretched by 1000 (86,400, 2.77) 43.1 / 42.1.
+bool mass_by_tiles(const mag_mesh *m) {
+    const double e = m->tile.evals_per_elem / 1.5;
+    return m->tile.small_blocks || (double)m->ne >= 26000.0 * e * e;
+}
+
 // enqueue() uses the handle's element scratch on stream s. Calls from different threads and on
 // different streams take turns at it: each waits for the event recorded after the last use, and the
 // mutex is held until it has recorded its own, so that no other thread's wait comes between.
@@ -849,7 +860,8 @@ int mag_assemble_mass(mag_mesh *m, const double *d_sigma, double *d_vals, void *
         return MAG_E_ARG;
     }
     cudaStream_t s = (cudaStream_t)stream;
-    if (m->schedule == MAG_SCHEDULE_TILE_BLOCKS && m->tile.ok) {
+    // (a captured call stays one launch that needs nothing of the handle's)
+    if (m->schedule == MAG_SCHEDULE_TILE_BLOCKS && m->tile.ok && (mass_by_tiles(m) || capturing(s))) {
         MAG_TRY(launch_tile_mass(m->tile, m->elems(), d_sigma, m->qp, d_vals, m->status, s));
         return finish(s);
     }
