@@ -173,13 +173,21 @@ __global__ void k_rows(const int32_t *__restrict__ dofs, const int32_t *__restri
 // Three launches: the rows' counts and their sums within a CTA, the sums of the CTAs, the entries
 // to their places. A warp takes kDropAhead rows at a time, a lane per entry (rows of a Nedelec
 // matrix have 13 to 19, so a row is one coalesced load and its rank one vote), steps such groups
-// one after another. One thread per row walking its entries took 6.3 us to count and 10.4 us to
-// copy at 28,000 rows (460,000 entries), with a device-wide scan of 7.7 us between them: 6.2, 7.6
-// and 5.6 us here. The call, with its copy back, at 60^3 hexahedra (25 M entries): 565 to 350 us.
+// one after another; CTAs of short rows take a thread per row. One thread per row walking its entries took
+// 6.3 us to count and 10.4 us to copy at 28,000 rows (460,000 entries), with a device-wide scan of 7.7 us
+// between them: 6.2, 7.6 and 5.6 us here. The call, with its copy back, at 60^3 hexahedra (25 M entries):
+// 565 to 350 us. Without the bound on its CTAs the copying kernel takes 68 registers, three CTAs an SM: 3
+// million rows of 18 entries 760 against 606 us.
 constexpr int kDropThreads = 256;
 constexpr int kDropAhead = 4;
 constexpr int kDropStep = kDropThreads / 32 * kDropAhead;  // rows of a CTA's step
 constexpr int kDropMaxSteps = kDropThreads / kDropStep;    // at most a row per thread
+// A CTA of kDropMaxSteps steps with at most this many entries a row takes a thread per row: most lanes of
+// a row's load would be idle. Measured, us, the call with a lane per entry / a thread per row, no zeros and
+// 30 %: 3 million rows of 5 entries 553, 546 / 236, 209; of 14 628, 616 / 632, 481; of 16 653, 640 / 838, 629;
+// 400,000 rows of 5 entries 89, 88 / 52, 47; of 14 111, 110 / 113, 89. (Before the lanes came, with its
+// device-wide scan, one thread per row took 241, 208; 804, 575; 103, 102; 167, 141.)
+constexpr int kDropShort = 14;
 // Many rows: more of them per CTA, so that the sums of the CTAs (one CTA adds them) stay few.
 inline int drop_steps(int64_t nrows) { return nrows < 200000 ? 1 : kDropMaxSteps; }
 
@@ -188,7 +196,7 @@ inline int drop_steps(int64_t nrows) { return nrows < 200000 ? 1 : kDropMaxSteps
 // COPY true: the start of the CTA's first row is final; the others' are added up, and the rows'
 // nonzeros go to their places.
 template <bool COPY>
-__global__ void __launch_bounds__(kDropThreads) k_drop(const int64_t *__restrict__ rp, const int32_t *__restrict__ ci,
+__global__ void __launch_bounds__(kDropThreads, COPY ? 4 : 6) k_drop(const int64_t *__restrict__ rp, const int32_t *__restrict__ ci,
                                                        const double *__restrict__ v, int64_t nrows, int steps,
                                                        int64_t *__restrict__ rp_out, int32_t *__restrict__ ci_out,
                                                        double *__restrict__ v_out) {
@@ -198,7 +206,27 @@ __global__ void __launch_bounds__(kDropThreads) k_drop(const int64_t *__restrict
     const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
     const int64_t r0 = blockIdx.x * (int64_t)steps * kDropStep;
     const int64_t off = COPY ? rp_out[r0] : 0;
-    for (int st = 0; st < steps; st++) {
+    const int64_t r1 = r0 + (int64_t)steps * kDropStep < nrows ? r0 + (int64_t)steps * kDropStep : nrows;
+    const bool short_rows = steps == kDropMaxSteps && rp[r1] - rp[r0] <= kDropShort * (r1 - r0);  // of the CTA
+    if (short_rows) {
+        const int64_t r = r0 + threadIdx.x, b = r < nrows ? rp[r + 1] : 0;
+        int64_t o = COPY && r < nrows ? (r == r0 ? 0 : rp_out[r]) + off : 0;
+        if (COPY && threadIdx.x > 0 && r < nrows) rp_out[r] = o;
+        int n = 0;
+        for (int64_t k = r < nrows ? rp[r] : 0; k < b; k++) {
+            const double x = v[k];
+            if (x != 0.0) {
+                if (COPY) {
+                    ci_out[o] = ci[k];
+                    v_out[o] = x;
+                    o++;
+                }
+                n++;
+            }
+        }
+        if (!COPY) cnt[threadIdx.x] = n;
+    }
+    for (int st = 0; st < steps && !short_rows; st++) {
         const int i0 = st * kDropStep + warp * kDropAhead;  // row of the CTA
         int64_t a[kDropAhead], b[kDropAhead], o[kDropAhead];
         double x[kDropAhead];

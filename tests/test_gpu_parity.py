@@ -1012,3 +1012,37 @@ def test_tiles_cut_at_the_block_limits(kind, most_blocks):
     plan.set_schedule(_lib.SCHEDULE_TWO_PASS)
     want = results()
     assert all(bits_equal(a.cpu().numpy(), b.cpu().numpy()) for a, b in zip(got + [captured], want + [want[-1]]))
+
+
+@pytest.mark.parametrize("kind", ["short", "empty", "mixed", "one long row", "fourteen", "fifteen"])
+def test_dropping_zeros_of_many_short_rows(kind):
+    """From 200,000 rows on the CTAs whose rows have at most 14 entries on average take a thread per row,
+    the others a lane per entry: both forms, and matrices that hold both, against numpy."""
+    n = 200000 + 37
+    rng = np.random.default_rng(3)
+    lens = {"short": rng.integers(0, 6, n), "empty": np.zeros(n, dtype=np.int64), "fourteen": np.full(n, 14),
+            "fifteen": np.full(n, 15), "mixed": np.where(np.arange(n) // 1000 % 2 == 0, 3, 40),
+            "one long row": np.where(np.arange(n) == n - 3, 3000, 2)}[kind]
+    rp = np.concatenate([[0], np.cumsum(lens)]).astype(np.int64)
+    nnz = int(rp[-1])
+    v, ci = rng.normal(size=nnz), rng.integers(0, n, nnz).astype(np.int32)
+    v[rng.random(nnz) < 0.3] = 0.0
+    v[rng.random(nnz) < 0.01] = np.nan
+    v[::97] = -0.0
+    keep = v != 0.0
+    want_rp = np.concatenate([[0], np.cumsum(keep)])[rp]
+    drp, dci, dv = (torch.as_tensor(a, device="cuda") for a in (rp, ci, v))
+    rp2, ci2, v2 = torch.full_like(drp, -1), torch.full((nnz + 1,), -1, dtype=torch.int32, device="cuda"), torch.zeros(
+        nnz + 1, dtype=torch.float64, device="cuda")
+    count = C.c_int64()
+    p = lambda t: C.c_void_p(t.data_ptr())
+    drop = lambda a, b, c: _lib.check(_lib.lib().mag_csr_drop_zeros(a, b, c, n, p(rp2), p(ci2), p(v2), C.byref(count),
+                                                                    _lib.stream_ptr()))
+    if nnz == 0:  # (an empty tensor has no address)
+        dci, dv = torch.zeros(1, dtype=torch.int32, device="cuda"), torch.zeros(1, dtype=torch.float64, device="cuda")
+    drop(p(drp), p(dci), p(dv))
+    k = int(count.value)
+    assert k == int(keep.sum()) and np.array_equal(rp2.cpu().numpy(), want_rp)
+    assert np.array_equal(ci2.cpu().numpy()[:k], ci[keep])
+    assert np.array_equal(v2.cpu().numpy()[:k].view(np.int64), v[keep].view(np.int64))
+    assert int(ci2[k]) == -1 if k < nnz else True
