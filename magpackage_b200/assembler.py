@@ -198,9 +198,12 @@ class Assembler:
     def _by_tag(self, values, width=()):
         """values[tag] of every element from a {tag: value} dict, 0 where a tag is not named: a small
         table is copied and indexed by the plan's tags (in 1..255, checked when it was made). None if
-        the mesh's tags are no longer the plan's or a key is no possible tag."""
+        the mesh's tags are no longer the plan's or a key is no possible tag, and on small meshes, where
+        the elements' own values are copied sooner than the table indexed (K from a map, us, table / values:
+        48 elements 37 / 28, 1,296 37 / 32, 3,072 37 / 42; a source 39 / 29, 39 / 36, 39 / 51)."""
         tags = self.plan.tags
-        if not all(0 <= k <= 255 for k in values) or not np.array_equal(self.Mesh.RegionTags, self._plan_tags):
+        if (self.Mesh.num_elements < 2000 or not all(0 <= k <= 255 for k in values)
+                or not np.array_equal(self.Mesh.RegionTags, self._plan_tags)):
             return None
         table = np.zeros((256,) + width)
         for k, v in values.items():
@@ -237,7 +240,10 @@ class Assembler:
         else:
             a = np.asarray(source_map, dtype=np.float64)
             if a.size == 3:
-                js = self._dev(a.ravel()).expand(n, 3).contiguous()
+                if n < 800:  # as for a map (384 elements 32.5 / 30.7 us, 1,296 32.6 / 36.9)
+                    js = self._dev(np.broadcast_to(a.ravel(), (n, 3)))
+                else:
+                    js = self._dev(a.ravel()).expand(n, 3).contiguous()
             elif a.shape == (n, 3):
                 js = self._dev(a)
             else:

@@ -1046,3 +1046,25 @@ def test_dropping_zeros_of_many_short_rows(kind):
     assert np.array_equal(ci2.cpu().numpy()[:k], ci[keep])
     assert np.array_equal(v2.cpu().numpy()[:k].view(np.int64), v[keep].view(np.int64))
     assert int(ci2[k]) == -1 if k < nnz else True
+
+
+@pytest.mark.parametrize("form", ["map", "unknown_tags", "float_keys", "outside_keys", "retagged", "nonscalar"])
+def test_assembler_maps_on_a_mesh_of_3024_elements(form, monkeypatch):
+    """As above where the maps are expanded on the device (2,000 elements and more)."""
+    box = synth.kuhn_box
+    monkeypatch.setattr(synth, "kuhn_box", lambda *a, **k: box(9, 8, 7, seed=9))
+    test_assembler_maps_equal_expanded_arrays(form)
+
+
+@pytest.mark.parametrize("n", [2, 6])
+def test_assembler_uniform_source_equals_the_array(n):
+    mesh = synth.kuhn_box(n, seed=9)
+    m = Mesh(mesh.P, mesh.T, synth.cube_layout(mesh))
+    dh = DofHandler(m)
+    dh.distribute_dofs()
+    asm = Assembler(m, dh, matlab_storage=False)
+    js = np.array([0.3, -2.0, 1.5])
+    want = host(asm.assemble_source(np.tile(js, (m.num_elements, 1))))
+    assert np.abs(want).max() > 0
+    for a in (js, js[None, :], list(js)):
+        assert bits_equal(host(asm.assemble_source(a)), want)
