@@ -1068,3 +1068,35 @@ def test_assembler_uniform_source_equals_the_array(n):
     assert np.abs(want).max() > 0
     for a in (js, js[None, :], list(js)):
         assert bits_equal(host(asm.assemble_source(a)), want)
+
+
+def test_batch_of_large_tiles_equals_single_meshes():
+    """Eight meshes of 16^3 hexahedra run on plans with large tiles made for the batch, one of them alone
+    on its own small tiles: the same values, by every tile variant."""
+    from magpackage_b200.plan import ComplexBatch
+
+    plans, nus, sigmas = [], [], []
+    for i in range(8):
+        mesh = synth.kuhn_box(16, seed=30 + i)
+        edges, t2e, sign = generate_edges(mesh.T)
+        tags = synth.cube_layout(mesh)
+        plans.append(AssemblyPlan(mesh.P, mesh.T, t2e, int(edges.shape[0]), tags, sign))
+        g = torch.Generator(device="cuda").manual_seed(i)
+        nus.append(torch.rand(mesh.num_elements, dtype=torch.float64, device="cuda", generator=g) + 1.0)
+        sigmas.append(dev(np.where(tags == synth.ALUMINIUM, 3.5e7, 0.0)))
+    omegas = [100.0 * (i + 1) for i in range(8)]
+    assert sum(p.num_elements for p in plans) >= 60000 > 2 * plans[0].num_elements
+    batch = ComplexBatch(plans, nus, sigmas, omegas)
+    for variant in (4, 5):
+        batch.select(variant)
+        for v in batch.values:
+            v.zero_()
+        got = [v.clone() for v in batch.assemble()]
+        for i in (0, 7):
+            one = ComplexBatch(plans[i:i + 1], nus[i:i + 1], sigmas[i:i + 1], omegas[i:i + 1])
+            one.select(variant)
+            want = one.assemble()[0]
+            assert float(want.real.abs().max()) > 0 and float(want.imag.abs().max()) > 0
+            assert torch.equal(torch.view_as_real(got[i]), torch.view_as_real(want))
+            one.close()
+    batch.close()
