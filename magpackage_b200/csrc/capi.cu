@@ -1071,10 +1071,11 @@ void destroy_batch(mag_batch *b) {
 // Small tiles pay where a mesh alone leaves SMs idle; the meshes of a large batch run together, so
 // those with small tiles get plans with large ones, owned by the batch: fewer evaluations and one
 // launch shape. A plan takes 0.5 to 0.9 ms, so batches that leave SMs idle themselves keep the meshes'
-// own (from where on the large ones are no slower). Measured, us a launch, own tiles / large tiles, and ms to create the batch: 16 meshes of 8^3
-// hexahedra (49,000 elements) 33.3 / 33.4, 2.4 / 10.8; 4 of 14^3 (66,000) 34.2 / 33.6, 2.1 / 6.7; 12 of 5^3 to 16^3 (110,000) 52.7 / 50.4, 2.9 / 11.7;
-// 16 of 12^3 (166,000) 78.5 / 69.6, 3.8 / 16.5; 12 of 5^3 to 20^3 (199,000) 93 / 69, 4.2 / 10.4; 64 of 10^3
-// (384,000) 200 / 134, 11 / 49.
+// own (from where on the large ones are no slower). Measured, us a launch, own tiles / large tiles,
+// and ms to create the batch: 16 meshes of 8^3 hexahedra (49,000 elements) 33.3 / 33.4, 2.4 / 10.8; 4 of
+// 14^3 (66,000) 34.2 / 33.6, 2.1 / 6.7; 12 of 5^3 to 16^3 (110,000) 52.7 / 50.4, 2.9 / 11.7; 16 of 12^3
+// (166,000) 78.5 / 69.6, 3.8 / 16.5; 12 of 5^3 to 20^3 (199,000) 93 / 69, 4.2 / 10.4; 64 of 10^3 (384,000)
+// 200 / 134, 11 / 49.
 constexpr int64_t kBatchLargeElems = 60000;
 
 int batch_large_tiles(mag_batch *b, mag_mesh *const *meshes, int n, cudaStream_t s) {
