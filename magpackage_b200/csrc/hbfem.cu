@@ -486,19 +486,34 @@ int launch_hb_std(const HbArgs &A, size_t smem, cudaStream_t s) {
 
 }  // namespace
 
-// With more samples than the register forms hold, k_hbfem_std<0> forms v(t) again for every group of
-// sums: for one or two harmonics the general kernel, compiled for the count, is then the faster one
-// once its one thread per element fills the GPU. Measured, us, constant-curl / general kernel: 1
+// Whether the general kernel, compiled for up to four harmonics, is the faster one although the
+// constant-curl kernel could serve. With more samples than the register forms hold, k_hbfem_std<0> forms
+// v(t) again for every group of sums: with one or two harmonics the general kernel then wins once its
+// one thread per element fills the GPU. Measured, us, constant-curl / general kernel, four points: 1
 // harmonic, 64 samples, residual and DC block at 29,478 elements 166 / 235, 48,000 252 / 252, 82,944
 // 401 / 346, 384,000 1825 / 1440, residual alone at 29,478 155 / 212, 48,000 239 / 225; 2 harmonics,
 // residual alone, 33 samples at 82,944 elements 252 / 287, 196,608 599 / 552, 663,552 2025 / 1751,
 // 160 samples there 7257 / 7159; with the DC block, 64 samples, 3428 / 3502.
+// A single point leaves no repeated work to merge: 64 samples at 48,000 and 384,000 elements, with the
+// DC block, 1 harmonic 127 / 100 and 775 / 535, 2 harmonics 145 / 123 and 1061 / 797, 3 harmonics 170 / 184
+// and 1224 / 1156; 3 harmonics, residual alone, 146 / 140 and 1160 / 869. Residuals alone with few samples
+// (the constant-curl kernel takes them 18 at a time): 1 harmonic at 384,000, 8 samples 188 / 137, 16
+// 186 / 168, 24 252 / 200, 32 260 / 238, but 196,608 elements 16 samples 89 / 109, 32 133 / 146; 2 harmonics,
+// 8 samples 256 / 227, 16 259 / 287.
+static bool hb_general_faster(int nq, int K, int N, int64_t ne, bool dc) {
+    if (nq == 1) {
+        if (ne < 45000) return false;
+        if (N > 32) return K <= 2 || (K == 3 && !dc && ne >= 150000);
+        return !dc && K <= 2 && (N <= 8 || (K == 1 && N > 16 && N <= 24));
+    }
+    if (N <= 32) return false;
+    return (K == 1 && ne >= (dc ? 60000 : 45000)) || (K == 2 && !dc && N <= 128 && ne >= 190000);
+}
+
 bool hbfem_constant_curls(const QuadParams &qp, int K, int N, int64_t ne, bool dc) {
     const int nt = N <= 16 ? 16 : N <= 24 ? 24 : N <= 32 ? 32 : 0;
-    if (!qp.standard_curl || !qp.uniform_w || hb_smem_bytes(K, N, nt) > (size_t)kMaxDynSmem) return false;
-    if (nt == 0 && K == 1 && ne >= (dc ? 60000 : 45000)) return false;
-    if (nt == 0 && K == 2 && !dc && N <= 128 && ne >= 190000) return false;
-    return true;
+    return qp.standard_curl && qp.uniform_w && hb_smem_bytes(K, N, nt) <= (size_t)kMaxDynSmem &&
+           !hb_general_faster(qp.nq, K, N, ne, dc);
 }
 
 namespace {

@@ -231,3 +231,26 @@ def test_hbfem_workspace_is_bounded_and_reported():
             assert need > base + (64 << 20)
         del R, sol
     plan.close()
+
+
+@pytest.mark.parametrize("harmonics,samples", [((1,), 33), ((1, 3), 40), ((1,), 7), ((1,), 20), ((0, 1), 8), ((1, 3), 16),
+                                               ((0, 1, 2), 33)])
+def test_hbfem_one_quadrature_point(oracle_port, harmonics, samples):
+    """One point on 47,880 elements, where either kernel may serve: with the DC block and alone."""
+    plan, m, pk, sol, E = _case(oracle_port, harmonics, n=(21, 20, 19), seed=7)
+    aft = AFT(harmonics, n_time_steps=samples)
+    assert aft.num_time_steps == samples
+    qw, val, curl = quadrature.reference_data(1)
+    plan.set_quadrature(qw, curl, val)
+    K = len(harmonics)
+    I, J, V, Rr, Rc, Rre, Rim = oracle_port.hbfem(m, sol, aft.D, aft.P, qw, curl, pk, True)
+    lin = Rr + (Rc - 1) * E
+    want_re = oracle_port.sparse_vec(lin, Rre, E * K).reshape(K, E)
+    want_im = oracle_port.sparse_vec(lin, Rim, E * K).reshape(K, E)
+    first = I <= E
+    _, _, rv = oracle_port.sparse_csr(I[first], J[first], V[first], E, drop_zeros=False)
+    for calc_j in (True, False):
+        R, vals = assemble_hbfem(plan, sol, aft, calc_j)
+        R = R.cpu().numpy()
+        assert bits_equal(np.real(R), want_re) and bits_equal(np.imag(R), want_im)
+        assert vals is None or bits_equal(vals.cpu().numpy(), rv)
