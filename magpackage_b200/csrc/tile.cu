@@ -697,7 +697,8 @@ int resident_ctas(const void *kern, int threads, size_t smem, int *out) {
 // 29.7, 34^3 (354,000) 37.8 / 38.2, 36^3 (420,000) 47.6 / 45.0, 40^3 65.2 / 62.5, 60^3 191 / 190; residual
 // alone at 26^3 shuffled 17.8 / 18.4, 40^3 (576,000) 28.1 / 28.9, 44^3 (767,000) 38.6 / 37.8, 48^3 53.1 /
 // 47.2. CTAs of the small shape have few records and each SM three of them: Jacobian at 8^3 9.24 / 9.06,
-// residual at 17^3 7.2 / 6.8, always by.
+// residual at 17^3 7.2 / 6.8, always by. So does the harmonic-balance DC block, which follows the
+// harmonic kernel's stores: the whole call at 24^3 with 4 harmonics, 64 samples 544 / 534.
 template <bool CALCJ>
 bool records_pass(const TilePlan &tp) {
     return tp.nrec >= (CALCJ ? 380000 : 650000);
@@ -706,7 +707,7 @@ bool records_pass(const TilePlan &tp) {
 template <bool CALCJ, bool Q4, int MODE, int BT, int MINB>
 int launch_shape(const TileArgs &a, const TilePlan &tp, size_t smem, cudaStream_t s) {
     auto kern = k_tile<BT, MINB, CALCJ, Q4, MODE, true>;
-    if constexpr (BT != kSmallBT)
+    if constexpr (BT != kSmallBT && MODE != kHarmonicDc)
         if (!records_pass<CALCJ>(tp)) kern = k_tile<BT, MINB, CALCJ, Q4, MODE, false>;
     int resident = 0;
     MAG_TRY(resident_ctas((const void *)kern, BT, smem, &resident));
