@@ -65,7 +65,7 @@ typedef struct {
 /* Jacobian assembly schedules; all give identical bits. */
 #define MAG_OPTION_SCHEDULE 1
 #define MAG_OPTION_TILE_VARIANT 2 /* launch shape of the tile schedule's Jacobian kernel: 0 = 320 threads x
-                                     2 CTAs/SM, on small meshes 160 x 3 (default),
+                                     2 CTAs/SM, on plans of small blocks 160 x 3 (default),
                                      1 = 288 x 2, 2 = 256 x 2, 3 = 512 x 1; same bits */
 #define MAG_OPTION_TILE_PREFETCH 3 /* staging depth of the tile schedule: how many waves of resident CTAs
                                       ahead a CTA prefetches its successor block's records into L2
